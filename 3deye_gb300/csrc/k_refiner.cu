@@ -6,14 +6,14 @@
 // "core matrix" rows the tensor core reads are 8 consecutive channels of one
 // pixel.
 //
-// Forward / input gradient (conv3x3_tc_kernel): M = 128 output pixels of one
-// image row, N = output channels, K = 9 taps x input channels.  The block
-// stages the 3 x 130-pixel input halo once, as planes of 8-channel chunks
-// (plane (row, chunk) holds the chunk of every halo pixel, 16 B apart).  In
-// that layout the A operand of tap (dy, dx) is the same planes started dx
-// pixels later, so each of the 9 taps is a descriptor offset -- no im2col
-// copy.  The input gradient is the same kernel run on the output gradient
-// with the transposed, tap-flipped weights.
+// Forward / input gradient (conv3x3_tc_kernel): M = 128 pixels of one image
+// row, K = input channels, N = the output channels of up to three output rows:
+// an input row is multiplied once per horizontal tap by the weights of all
+// three vertical taps side by side, which adds it to the three output rows it
+// belongs to.  Rows are staged as planes of 8-channel chunks whose pixels lie
+// so that a horizontal tap is an aligned descriptor offset -- no im2col copy.
+// The input gradient is the same kernel run on the output gradient with the
+// transposed, tap-flipped weights.
 //
 // Weight gradient (wgrad_tc_kernel): M = 128 rows of (tap row, input
 // channel), N = output channels, K = pixels, with MN-major operands read from
@@ -23,6 +23,7 @@
 // (deterministic).
 #include <cuda_bf16.h>
 
+#include <cstddef>
 #include <vector>
 
 #include "tde_common.cuh"
@@ -34,7 +35,13 @@ namespace refiner {
 namespace {
 
 constexpr int kTileM = 128;             // output pixels per MMA tile
-constexpr int kHaloW = kTileM + 2;      // halo pixels per row
+// A staged row of a 128-pixel tile and its two halo pixels: core matrix g (8
+// rows of 16 bytes, one channel chunk) holds the pixels g, g + 16, ..., g +
+// 112, so the tile is core matrices 0..15 and the tile one or two pixels on
+// is 1..16 or 2..17: each horizontal tap reads whole 128-byte lines of shared
+// memory, where with the pixels in order it would start 16 or 32 bytes into one.
+constexpr int kRowGroups = 18;
+constexpr int kPlaneBytes = kRowGroups * 128;  // one 8-channel chunk of a staged row
 constexpr int kWgK = 64;                // pixels per weight-gradient K step
 constexpr int kWgHalo = kWgK + 2;
 constexpr uint32_t kSmemPerSM = 228 * 1024;
@@ -102,36 +109,61 @@ __device__ __forceinline__ uint4 load_input_chunk(const Args &A, int img, int y,
 // A block owns strips of consecutive output rows of one 128-pixel column
 // tile.  Its warps have fixed roles, connected by mbarriers (no block-wide
 // barrier in the steady state):
-//   warps 4-7 (producers): input row j goes to warp 4 + (j & 3), which loads
+//   warps 0-3 (producers): input row j goes to warp j & 3, which loads
 //     the halo row (pixels x0-1 .. x0+128, every 8-channel chunk, as planes)
 //     into ring slot j % S once the tensor core has released that slot, and
 //     marks it full -- four rows in flight, one per warp;
-//   warp 8, one lane (MMA issuer): output row r waits for its three input
-//     rows and for a free accumulator (one of kConvAcc in tensor memory),
-//     issues 9 taps x CC/2 MMAs (M = 128 pixels, N = cout, K = 16), and
-//     commits them to the accumulator's "full" barrier and to the "empty"
-//     barrier of the input row no later output row reads;
-//   warps 0-3 (epilogue): TMEM lane quarter q of warp q, one pixel per
-//     thread -- wait for the accumulator, read it (tcgen05.ld), apply bias,
-//     ReLU, mask or the fused head, store bf16 NHWC, release the accumulator.
+//   warp 4 (MMA issuer): input row i of a strip belongs to output
+//     rows i - 2, i - 1 and i (vertical taps 2, 1, 0).  Their accumulators lie
+//     side by side in tensor memory and the three taps' weights side by side
+//     in shared memory, so each of the row's 3 x CC/2 MMAs (horizontal tap,
+//     K = 16 channels) has N = 3 cout: a third of the MMAs of one per tap to
+//     issue (some 70 cycles each, whatever they read, which was most of a row's
+//     time), and the pixels are read from shared memory once instead of three
+//     times.  An output row still sums its taps in the order (0,0), (0,1), ...
+//     (2,2), so its bits are those of one MMA per tap.  The accumulators form a ring of NA rows; the MMAs of
+//     a row whose outputs wrap around the ring are split there, and the first
+//     MMA of an output row, which overwrites its accumulator, is issued apart;
+//   warps 5-8, or 5-12 taking rows in turn (epilogue): a TMEM lane quarter
+//     each, one pixel per thread -- wait for the accumulator, read it
+//     (tcgen05.ld), release it, apply bias, ReLU, mask or the fused head, store
+//     bf16 NHWC.
 // Input rows are loaded once per strip; loads, MMAs and epilogues of
-// different rows overlap.  Every wait is bounded: on a timeout the block
+// different rows overlap.  At batch 16 of 640x480 the forward pass took 1138 us
+// with one MMA per tap, index arithmetic per copied piece and 16-byte stores a
+// pixel apart, and takes 792 us (batch 1: 156 and 135 us); what is left per row is
+// the issuer's chain of waits and issues (about 1000 cycles a row and block) and,
+// at the full resolution, memory (c2 moves 353 MB in 94 us).  Every wait is bounded: on a timeout the block
 // raises A.err, all roles leave their loops, the issuer waits (bounded) for
 // its MMAs in flight, and the tensor memory is freed.
 // ---------------------------------------------------------------------------
-constexpr int kConvEpiWarps = 4, kConvProdWarps = 4;
-constexpr int kConvThreads = 32 * (kConvEpiWarps + kConvProdWarps + 1);  // + the MMA warp
-constexpr int kConvMmaWarp = kConvEpiWarps + kConvProdWarps;
-constexpr int kConvAcc = 4;       // accumulators in tensor memory
+constexpr int kConvProdWarps = 4, kConvMmaWarp = kConvProdWarps;
+// Epilogue warps follow: one set of four where the output is pooled or the
+// input upsampled (the layer's other roles bound it; c4, c6 and c9 took 71, 64
+// and 86 us with two sets, 66, 57 and 59 with one, at batch 16 of 640x480), two
+// elsewhere (the input gradients of c2 and c10: 134 and 106 us with one, 106
+// and 82 with two).
+constexpr int conv_epi_sets(int mode, bool pool) { return mode == SRC_UP || pool ? 1 : 2; }
+__host__ __device__ constexpr int conv_threads(int sets) { return 32 * (kConvProdWarps + 1 + 4 * sets); }
+constexpr int kConvMaxPerSM = 2;  // resident blocks (three or four: the same times)
+constexpr int kConvMinAcc = 4;    // accumulator rows: three being summed, one being drained
+constexpr int kConvMaxAcc = 8;
 constexpr int kConvMaxSlots = 8;  // input-row ring
-constexpr int kConvMinSlots = 4;
+// No fewer slots than producer warps: a warp's row j - 4 was issued once row
+// j - 4 - S had been consumed, so the slot of row j is at most one phase behind
+// when it is waited for (a parity wait cannot tell more).
+constexpr int kConvMinSlots = kConvProdWarps;
+// Ring of the source rows that two input rows share (upsampled sources).
+__host__ __device__ constexpr int shared_slots(int slots) { return slots / 2 + 1; }
+constexpr int kConvMaxShared = shared_slots(kConvMaxSlots);
 constexpr int kStripRowsOneWave = 8;   // longest strip of a one-wave launch
 constexpr int kStripRowsBalanced = 16;  // strip length when the work is larger
 constexpr uint64_t kConvWaitNs = 2000000000ull;
 
 struct ConvPipe {
     uint64_t full[kConvMaxSlots], empty[kConvMaxSlots];
-    uint64_t acc_full[kConvAcc], acc_empty[kConvAcc];
+    uint64_t sfull[kConvMaxShared], sempty[kConvMaxShared];
+    uint64_t acc_full[kConvMaxAcc], acc_empty[kConvMaxAcc];
     uint64_t drain;
     uint32_t tmem;
     int abort;
@@ -189,131 +221,267 @@ __device__ __forceinline__ Strip strip_of(const ConvArgs &A, int item, int rows_
     return s;
 }
 
-// One warp starts the copies of input row y (halo pixels x0-1 .. x0+128) into
-// a slot as planes: CCA chunks of source A (read directly, or through the
-// nearest 2x upsample of an h/2 x w/2 tensor), then CCB chunks of source B;
-// 16-byte cp.async, zero outside the image; one commit group per row.
-// Consecutive lanes copy consecutive 16-byte pieces of a source row.
-template <int CP, bool UPS, int HALO = kHaloW>
-__device__ __forceinline__ void warp_copy_part(const bf16 *row, int px_elems, int w, int x_start, int plane0, bool row_in,
-                                               unsigned char *slot, const bf16 *dummy, int lane) {
-    for (int i = lane; i < HALO * CP; i += 32) {
-        const int px = i / CP, c = i - px * CP;
-        const int x = x_start + px;
-        const bool in = row_in && (unsigned)x < (unsigned)w;
-        const bf16 *src = in ? row + (size_t)(UPS ? (x >> 1) : x) * px_elems + 8 * c : dummy;
-        const uint32_t dst = tc::smem_u32(slot + ((size_t)(plane0 + c) * HALO + px) * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
-                     : "memory");
+// Copies of CP = 2 or 4 channel chunks (PXE channels a source pixel) of one
+// staged row into its planes, read directly or through the nearest 2x
+// upsample of a row half as wide; 16-byte cp.async, zeros past the row's ends.
+// Eight lanes write the eight pixels of a core matrix (one 128-byte line), the
+// four such sets of a warp two or four chunks of one or two pixels (whole
+// 32-byte sectors).  Unrolled, every address is a lane's base plus a constant:
+// a piece costs a compare, the copy and its zero store (predicated off), where
+// index arithmetic per piece made this the longest part of a row.
+template <int CP, bool UPS, int PXE>
+__device__ __forceinline__ void warp_copy_chunks(const bf16 *row, int x_start, int w, uint32_t dst, int lane) {
+    const int k = lane & 7, l3 = lane >> 3;
+    const int c = CP == 4 ? l3 : l3 & 1, gl = CP == 4 ? 0 : l3 >> 1;
+    const int x = x_start + gl + 16 * k;  // this lane's first pixel; x_start is one left of a multiple of 128
+    const int lim = w - x;
+    const bf16 *src = row + (UPS ? (x_start + 1) / 2 + 8 * k + ((gl - 1) >> 1) : x) * PXE + 8 * c;
+    dst += (uint32_t)(k * 16 + c * kPlaneBytes + gl * 128);
+#pragma unroll
+    for (int it = 0; it < kRowGroups * CP / 4; ++it) {
+        const int g = CP == 4 ? it : 2 * it;
+        const int off = UPS ? (CP == 4 ? (it + 1) >> 1 : it) : g;
+        if (g < lim && (it > 0 || x >= 0))
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + g * 128), "l"(src + off * PXE) : "memory");
+        else
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst + g * 128), "r"(0) : "memory");
     }
 }
-template <int MODE, int CCA, int CCB>
-__device__ __forceinline__ void warp_issue_row(const ConvArgs &A, unsigned char *slot, int img, int y, int x0, int lane) {
-    const bool row_in = y >= 0 && y < A.h;
-    const int yc = row_in ? y : 0;
-    if (MODE == SRC_UP) {
-        const bf16 *ra = A.a + (((size_t)img * (A.h >> 1) + (yc >> 1)) * (A.w >> 1)) * A.ca;
-        warp_copy_part<CCA, true>(ra, A.ca, A.w, x0 - 1, 0, row_in, slot, A.a, lane);
+template <int CC, bool UPS>
+__device__ __forceinline__ void warp_copy_source(const bf16 *row, int x_start, int w, uint32_t dst, int lane) {
+#pragma unroll
+    for (int c = 0; c + 4 <= CC; c += 4)
+        warp_copy_chunks<4, UPS, 8 * CC>(row + 8 * c, x_start, w, dst + c * kPlaneBytes, lane);
+    if constexpr (CC % 4 != 0)
+        warp_copy_chunks<2, UPS, 8 * CC>(row + 8 * (CC - 2), x_start, w, dst + (CC - 2) * kPlaneBytes, lane);
+}
+// One warp starts the copies of CC chunks of a row (halo pixels x0-1 .. x0+128)
+// into the planes at dst, or zeros when the row lies outside the image (null).
+template <int CC, bool UPS>
+__device__ __forceinline__ void warp_copy_row(const bf16 *row, int x0, int w, uint32_t dst, int lane) {
+    if (row) {
+        warp_copy_source<CC, UPS>(row, x0 - 1, w, dst, lane);
     } else {
-        const bf16 *ra = A.a + (((size_t)img * A.h + yc) * A.w) * A.ca;
-        warp_copy_part<CCA, false>(ra, A.ca, A.w, x0 - 1, 0, row_in, slot, A.a, lane);
+        for (int i = lane; i < CC * kPlaneBytes / 16; i += 32)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst + i * 16), "r"(0) : "memory");
     }
-    if (CCB > 0) {
-        const bf16 *rb = A.b + (((size_t)img * A.h + yc) * A.w) * A.cb;
-        warp_copy_part<CCB, false>(rb, A.cb, A.w, x0 - 1, CCA, row_in, slot, A.a, lane);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Epilogue of one output row for one pixel (TMEM lane quarter of this warp).
-// With a pooled output, `keep` holds the row's bf16 results when y is even;
-// at the odd row below it the 2x2 maximum (the row pair in registers, the
-// pixel pair across lanes x and x ^ 1) goes to pool_out -- the same bits as
-// a max pool of the stored rows.
-constexpr int kPoolMaxChunks = 8;  // pooled outputs have at most 64 channels
-__device__ __forceinline__ void conv_epilogue(const ConvArgs &A, uint32_t tacc, int quarter, int lane, int img, int y,
-                                              int x0, float depth_in, uint4 (&keep)[kPoolMaxChunks],
-                                              const float *s_bias, const float *s_head) {
-    const int m = quarter * 32 + lane;
-    const int x = x0 + m;
-    const bool valid = x < A.w;
-    const size_t pix = ((size_t)img * A.h + y) * A.w + (valid ? x : 0);
-    const bool pool_row = A.pool_out && (y & 1);
-    const size_t ppix = ((size_t)img * (A.h >> 1) + (y >> 1)) * (A.w >> 1) + (valid ? (x >> 1) : 0);
-    float r = 0.f;
-    for (int j = 0; j < A.cout; j += 16) {
-        float v[16];
-        tc::tmem_ld16(tacc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)j, v);
-        if (A.bias) {
+// Pixel of the tile that TMEM lane m holds: row m of a staged tile is element
+// m & 7 of core matrix m >> 3.
+__device__ __forceinline__ int tile_pixel(int m) { return (m >> 3) + 16 * (m & 7); }
+
+// Bias, ReLU and mask of 16 channels of one pixel, rounded to bf16.
+__device__ __forceinline__ void finish16(const ConvArgs &A, float (&v)[16], const float *bias, uint4 m0, uint4 m1, uint4 &q0,
+                                         uint4 &q1) {
+    if (A.bias) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] += s_bias[j + k];
+        for (int k = 0; k < 16; k += 4) {
+            const float4 b = *reinterpret_cast<const float4 *>(bias + k);
+            v[k] += b.x; v[k + 1] += b.y; v[k + 2] += b.z; v[k + 3] += b.w;
         }
-        if (A.relu) {
+    }
+    if (A.relu) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = v[k] > 0.f ? v[k] : 0.f;
-        }
-        if (A.mask) {
-            float mk[16];
-            unpack8(ldg16(A.mask + pix * A.cout + j), mk);
-            unpack8(ldg16(A.mask + pix * A.cout + j + 8), mk + 8);
+        for (int k = 0; k < 16; ++k) v[k] = v[k] > 0.f ? v[k] : 0.f;
+    }
+    if (A.mask) {
+        float mk[16];
+        unpack8(m0, mk);
+        unpack8(m1, mk + 8);
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = mk[k] > 0.f ? v[k] : 0.f;
+        for (int k = 0; k < 16; ++k) v[k] = mk[k] > 0.f ? v[k] : 0.f;
+    }
+    q0 = pack8(v);
+    q1 = pack8(v + 8);
+}
+__device__ __forceinline__ void store16(bf16 *o, uint4 q0, uint4 q1) {
+    reinterpret_cast<uint4 *>(o)[0] = q0;
+    reinterpret_cast<uint4 *>(o)[1] = q1;
+}
+__device__ __forceinline__ uint4 shfl_xor4(uint4 p, int m) {
+    return make_uint4(__shfl_xor_sync(0xffffffffu, p.x, m), __shfl_xor_sync(0xffffffffu, p.y, m),
+                      __shfl_xor_sync(0xffffffffu, p.z, m), __shfl_xor_sync(0xffffffffu, p.w, m));
+}
+
+// Ring position of an output row's accumulator.
+struct AccAt {
+    int a;
+    uint32_t phase;
+    __device__ __forceinline__ void next(int NA) {
+        if (++a == NA) {
+            a = 0;
+            phase ^= 1u;
         }
-        const uint4 q0 = pack8(v), q1 = pack8(v + 8);
-        if (valid) {
-            uint4 *o = reinterpret_cast<uint4 *>(A.out + pix * A.cout + j);
-            o[0] = q0;
-            o[1] = q1;
-        }
-        if (A.pool_out) {
-            const int c = j >> 3;
-            if (!pool_row) {
-                keep[c] = q0;
-                keep[c + 1] = q1;
-            } else {
-                uint4 p0 = bmax4(keep[c], q0), p1 = bmax4(keep[c + 1], q1);
-                uint4 n0, n1;
-                n0.x = __shfl_xor_sync(0xffffffffu, p0.x, 1); n0.y = __shfl_xor_sync(0xffffffffu, p0.y, 1);
-                n0.z = __shfl_xor_sync(0xffffffffu, p0.z, 1); n0.w = __shfl_xor_sync(0xffffffffu, p0.w, 1);
-                n1.x = __shfl_xor_sync(0xffffffffu, p1.x, 1); n1.y = __shfl_xor_sync(0xffffffffu, p1.y, 1);
-                n1.z = __shfl_xor_sync(0xffffffffu, p1.z, 1); n1.w = __shfl_xor_sync(0xffffffffu, p1.w, 1);
-                if (valid && !(x & 1)) {
-                    uint4 *o = reinterpret_cast<uint4 *>(A.pool_out + ppix * A.cout + j);
-                    o[0] = bmax4(p0, n0);
-                    o[1] = bmax4(p1, n1);
+    }
+};
+
+// The epilogue role of one warp: a TMEM lane quarter of every output row, or of every
+// other one -- with a pooled output every other pair of rows, whose 2x2
+// maximum (the row pair in registers, the pixel pair across lanes 8 apart) goes
+// to pool_out, the same bits as a max pool of the stored rows.  With two
+// sets of four warps one row's tensor-memory and global latencies overlap the
+// next one's.  What does not depend on the sums (the head's input depth, the
+// ReLU mask) is fetched before waiting for them, and the accumulator is released
+// as soon as it is in registers.
+//
+// A lane holds one pixel's channels, and its 16-byte stores would write a half
+// of a sector at a time, a pixel's stride apart.  The channels of four
+// neighbouring pixels are a run of 128 bytes or more: the warp collects its
+// eight runs in shared memory and stores them with consecutive lanes.  Of the
+// 16-byte units of a run (4 COUT / 8, a multiple of 8), unit u lies at u ^ k, k
+// the run, so that the eight lanes of one core matrix write to different banks.
+// Where a layer's shared memory has no room for it (conv_plan), each pixel is
+// stored directly.
+// Shared memory for it: 32 pixels of one row, or of two, per epilogue warp.
+__host__ __device__ constexpr size_t conv_stage_bytes(int cout, bool pool) {
+    return (size_t)32 * cout * 2 * (pool ? 2 : 1);
+}
+template <int COUT, bool POOL, int SETS>
+__device__ __forceinline__ void conv_epilogue(const ConvArgs &A, ConvPipe &pp, const float *s_bias, const float *s_head,
+                                           unsigned char *stage, int rows_per_item, int items, int NA, int warp, int lane) {
+    constexpr int ROWS = POOL ? 2 : 1;
+    const bool staged = stage != nullptr;
+    constexpr int UNITS = 4 * COUT / 8;  // 16-byte units of one run
+    const uint32_t sbase = tc::smem_u32(stage) + (uint32_t)((warp - kConvMmaWarp - 1) * ROWS * 32 * COUT * 2);
+    const int run = lane & 7, rpx = lane >> 3;
+    // a warp reads the tensor-memory lanes of its number modulo 4; any four
+    // consecutive warps cover a row
+    const uint32_t set = (uint32_t)(warp - kConvMmaWarp - 1) >> 2, quarter = (uint32_t)warp & 3u;
+    const uint32_t tmem = pp.tmem + (quarter << 21);  // lane 32 * quarter in bits 16..
+    const int px = tile_pixel(quarter * 32 + lane);
+    volatile int *abort = &pp.abort;
+    AccAt at{0, 0u};
+    uint32_t turn = 0;
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const Strip st = strip_of(A, item, rows_per_item);
+        const int x = st.x0 + px;
+        const bool valid = x < A.w;
+        for (int y = st.y0; y < st.y1; y += ROWS, ++turn) {
+            AccAt row[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                row[r] = at;
+                at.next(NA);
+            }
+            if (SETS > 1 && turn % SETS != set) continue;
+            const size_t pix = ((size_t)st.img * A.h + y) * A.w + (valid ? x : 0);
+            float din = 0.f;
+            if (COUT == 16 && !POOL && A.head_w && valid) din = __ldg(A.depth_in + pix);
+            uint4 m0[ROWS], m1[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                m0[r] = m1[r] = make_uint4(0u, 0u, 0u, 0u);
+                if (A.mask) {
+                    m0[r] = ldg16(A.mask + (pix + (size_t)r * A.w) * COUT);
+                    m1[r] = ldg16(A.mask + (pix + (size_t)r * A.w) * COUT + 8);
                 }
             }
-        }
-        if (A.head_w && valid) {
-            float f[16];
-            unpack8(q0, f);
-            unpack8(q1, f + 8);
 #pragma unroll
-            for (int k = 0; k < 16; ++k) r = fmaf(s_head[k], f[k], r);
-        }
-    }
-    if (valid && A.head_w) {
-        const float o = depth_in > 0.f ? depth_in + 0.01f * (r + s_head[16]) : 0.f;  // residual in cm
-        if (A.depth_out) A.depth_out[pix] = o;
-        if (A.depth_mm) {
-            const float mm = fminf(fmaxf(rintf(o * 1000.f), 0.f), (float)TDE_MAX_DEPTH_VALUE);
-            A.depth_mm[pix] = (uint16_t)mm;
+            for (int r = 0; r < ROWS; ++r)
+                if (!pipe_wait(&pp.acc_full[row[r].a], row[r].phase, abort, A.err)) return;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int j = 0; j < COUT; j += 16) {
+                float v[ROWS][16];
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) tc::tmem_ld16_nowait(tmem + (uint32_t)(row[r].a * COUT + j), v[r]);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) tc::tie16(v[r]);
+                if (j + 16 >= COUT) {
+                    tc::fence_before_sync();
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < ROWS; ++r)
+                        if (lane == 0) mbar_arrive(&pp.acc_empty[row[r].a]);
+                }
+                uint4 q0[ROWS], q1[ROWS];
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+                    const uint4 n0 = m0[r], n1 = m1[r];
+                    if (A.mask && j + 16 < COUT) {
+                        m0[r] = ldg16(A.mask + (pix + (size_t)r * A.w) * COUT + j + 16);
+                        m1[r] = ldg16(A.mask + (pix + (size_t)r * A.w) * COUT + j + 24);
+                    }
+                    finish16(A, v[r], s_bias + j, n0, n1, q0[r], q1[r]);
+                    if (staged) {
+                        const uint32_t at = sbase + (uint32_t)((r * 8 + run) * UNITS * 16);
+                        const int u = rpx * (COUT / 8) + j / 8;
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + ((u ^ run) * 16)), "r"(q0[r].x),
+                                     "r"(q0[r].y), "r"(q0[r].z), "r"(q0[r].w) : "memory");
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + (((u + 1) ^ run) * 16)),
+                                     "r"(q1[r].x), "r"(q1[r].y), "r"(q1[r].z), "r"(q1[r].w) : "memory");
+                    } else {
+                        if (valid) store16(A.out + (pix + (size_t)r * A.w) * COUT + j, q0[r], q1[r]);
+                    }
+                }
+                if constexpr (POOL) {
+                    const uint4 p0 = bmax4(q0[0], q0[1]), p1 = bmax4(q1[0], q1[1]);
+                    const uint4 n0 = shfl_xor4(p0, 8), n1 = shfl_xor4(p1, 8);
+                    if (valid && !(x & 1)) {
+                        const size_t ppix = ((size_t)st.img * (A.h >> 1) + (y >> 1)) * (A.w >> 1) + (x >> 1);
+                        store16(A.pool_out + ppix * COUT + j, bmax4(p0, n0), bmax4(p1, n1));
+                    }
+                }
+                if constexpr (COUT == 16 && !POOL) {
+                    if (A.head_w && valid) {
+                        float f[16], r = 0.f;
+                        unpack8(q0[0], f);
+                        unpack8(q1[0], f + 8);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) r = fmaf(s_head[k], f[k], r);
+                        const float o = din > 0.f ? din + 0.01f * (r + s_head[16]) : 0.f;  // residual in cm
+                        if (A.depth_out) A.depth_out[pix] = o;
+                        if (A.depth_mm) {
+                            const float mm = fminf(fmaxf(rintf(o * 1000.f), 0.f), (float)TDE_MAX_DEPTH_VALUE);
+                            A.depth_mm[pix] = (uint16_t)mm;
+                        }
+                    }
+                }
+            }
+            if (staged) {
+                __syncwarp();
+                // pixel 4 * quarter + 16 * k of the tile begins run k
+                bf16 *dst = A.out + (((size_t)st.img * A.h + y) * A.w + st.x0 + 4 * (int)quarter) * COUT;
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+                    for (int t = 0; t < UNITS / 4; ++t) {
+                        const int i = t * 32 + lane, k = i / UNITS, u = i - k * UNITS;
+                        const uint32_t at = sbase + (uint32_t)((r * 8 + k) * UNITS * 16);
+                        uint4 q;
+                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "r"(at + ((u ^ k) * 16)) : "memory");
+                        if (st.x0 + 4 * (int)quarter + 16 * k + u / (COUT / 8) < A.w)
+                            *reinterpret_cast<uint4 *>(dst + ((size_t)r * A.w + 16 * k) * COUT + u * 8) = q;
+                    }
+                }
+                __syncwarp();
+            }
         }
     }
 }
 
-template <int MODE, int CCA, int CCB>
-__global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs A, int rows_per_item, int S) {
+template <int MODE, int CCA, int CCB, int SETS>
+__global__ void __launch_bounds__(conv_threads(SETS), kConvMaxPerSM) conv3x3_tc_kernel(const __grid_constant__ ConvArgs A, int rows_per_item,
+                                                                        int S, int NA, int staged) {
     constexpr int CC = CCA + CCB;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ ConvPipe pp;
-    __shared__ float s_bias[128], s_head[17];  // bias; head weights and head bias
+    __shared__ __align__(16) float s_bias[128], s_head[17];  // bias; head weights and head bias
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr uint32_t slot_bytes = (uint32_t)CC * kHaloW * 16;
+    // A slot holds what only its input row has; an upsampled source's rows,
+    // each that of two input rows, lie in a ring of their own.
+    constexpr int CS = MODE == SRC_UP ? CCA : 0, CO = CC - CS;
+    constexpr uint32_t slot_bytes = (uint32_t)CO * kPlaneBytes, shared_bytes = (uint32_t)CS * kPlaneBytes;
+    const int SS = shared_slots(S);
     unsigned char *halo = smem;
-    unsigned char *wsm = smem + (size_t)S * slot_bytes;
-    const uint32_t ncols = tmem_cols(A.cout);
-    const uint32_t tcols = kConvAcc * ncols;
+    unsigned char *shared_rows = smem + (size_t)S * slot_bytes;
+    unsigned char *wsm = shared_rows + (CS ? (size_t)SS * shared_bytes : 0);
+    unsigned char *stage = staged ? wsm + (size_t)9 * CC * A.cout * 16 : nullptr;
+    const uint32_t ncols = (uint32_t)A.cout;  // tensor-memory columns of one output row
+    const uint32_t tcols = tmem_cols(NA * A.cout);
     volatile int *abort = &pp.abort;
 
     // the next layer may start its prologue; it waits for this grid before
@@ -325,23 +493,29 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
             tc::mbar_init(&pp.full[s], 1);
             tc::mbar_init(&pp.empty[s], 1);
         }
-        for (int a = 0; a < kConvAcc; ++a) {
+        for (int s = 0; s < kConvMaxShared; ++s) {
+            tc::mbar_init(&pp.sfull[s], 1);
+            tc::mbar_init(&pp.sempty[s], 1);
+        }
+        for (int a = 0; a < kConvMaxAcc; ++a) {
             tc::mbar_init(&pp.acc_full[a], 1);
-            tc::mbar_init(&pp.acc_empty[a], kConvEpiWarps);
+            tc::mbar_init(&pp.acc_empty[a], 4);  // the four warps that drain a row
         }
         tc::mbar_init(&pp.drain, 1);
         pp.abort = 0;
     }
     if (A.bias && tid < A.cout) s_bias[tid] = A.bias[tid];
     if (A.head_w && tid < 17) s_head[tid] = tid < 16 ? A.head_w[tid] : A.head_b[0];
-    // weights: global [co][t][ci] -> planes (t, chunk) of cout rows x 16 B.
+    // weights: global [co][t][ci] -> planes (dx, chunk) of 3 cout rows x 16 B:
+    // the rows of vertical taps 2, 1, 0 (output rows i - 2, i - 1, i of input row i).
     // No kernel launched right before a convolution writes weights, so they
     // are fetched before waiting for the previous grid.
     {
         const int nw = A.cout * 9 * CC;
-        for (int i = tid; i < nw; i += kConvThreads) {
+        for (int i = tid; i < nw; i += (int)blockDim.x) {
             const int c = i % CC, t = (i / CC) % 9, co = i / (9 * CC);
-            const uint32_t dst = tc::smem_u32(wsm + ((size_t)(t * CC + c) * A.cout + co) * 16);
+            const int dy = t / 3, dx = t - 3 * dy;
+            const uint32_t dst = tc::smem_u32(wsm + ((size_t)((dx * CC + c) * 3 + 2 - dy) * A.cout + co) * 16);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(A.wgt + (size_t)i * 8) : "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -355,12 +529,13 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
     const int tiles_x = (A.w + kTileM - 1) / kTileM;
     const int items = A.n * tiles_x * ((A.h + rows_per_item - 1) / rows_per_item);
 
-    if (warp >= kConvEpiWarps && warp < kConvMmaWarp) {
+    if (warp < kConvProdWarps) {
         // ---- producers: warp pw loads the input rows j = pw (mod 4), two in
-        // flight; a row is marked full once its copies have landed ----
-        const int pw = warp - kConvEpiWarps;
-        uint32_t j = 0;                  // this block's input-row sequence
-        int pending = -1;                // slot of the row issued before the current one
+        // flight; a row is marked full once its copies have landed, at the
+        // latest before this warp waits for anything ----
+        const int pw = warp;
+        uint32_t j = 0, js = 0;          // this block's input-row and shared-row sequences
+        int pending = -1, spending = -1; // slots of the row issued before the current one
         bool ok = true;
         auto publish = [&](int wait_groups) {
             if (pending < 0) return;
@@ -368,101 +543,194 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
             tc::fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&pp.full[pending]);
-            pending = -1;
+            if (lane == 0) {
+                mbar_arrive(&pp.full[pending]);
+                if (CS && spending >= 0) mbar_arrive(&pp.sfull[spending]);
+            }
+            pending = spending = -1;
+        };
+        auto wait_empty = [&](uint64_t *bar, uint32_t k) {
+            if (k == 0 || tc::mbar_test_wait(bar, (k - 1) & 1u)) return true;
+            publish(0);
+            return pipe_wait(bar, (k - 1) & 1u, abort, A.err);
         };
         for (int item = blockIdx.x; item < items && ok && !*abort; item += gridDim.x) {
             const Strip st = strip_of(A, item, rows_per_item);
             const int nin = st.y1 - st.y0 + 2;
             for (int i = 0; i < nin; ++i, ++j) {
-                if ((int)(j & 3u) != pw) continue;
-                const uint32_t s = j % (uint32_t)S, k = j / (uint32_t)S;
-                if (k > 0) {
-                    // the MMA that frees this slot reads input rows up to
-                    // j - S + 2; when that reaches this warp's previous row
-                    // (j - 4, S <= 6), publish it before waiting
-                    if (S <= 6) publish(0);
-                    if (!(ok = pipe_wait(&pp.empty[s], (k - 1) & 1u, abort, A.err))) break;
+                const int y = st.y0 - 1 + i;
+                const bool fresh = CS && (i == 0 || !(y & 1));  // the first input row of its shared row
+                if ((int)(j % (uint32_t)kConvProdWarps) != pw) {
+                    js += fresh;
+                    continue;
                 }
-                warp_issue_row<MODE, CCA, CCB>(A, halo + (size_t)s * slot_bytes, st.img, st.y0 - 1 + i, st.x0, lane);
+                const bool row_in = y >= 0 && y < A.h;
+                const uint32_t s = j % (uint32_t)S, ss = js % (uint32_t)SS;
+                if (!(ok = wait_empty(&pp.empty[s], j / (uint32_t)S))) break;
+                if (fresh && !(ok = wait_empty(&pp.sempty[ss], js / (uint32_t)SS))) break;
+                const uint32_t dst = tc::smem_u32(halo) + s * slot_bytes;
+                if constexpr (MODE == SRC_UP) {
+                    if (fresh)
+                        warp_copy_row<CCA, true>(
+                            row_in ? A.a + ((size_t)st.img * (A.h >> 1) + (y >> 1)) * (A.w >> 1) * (8 * CCA) : nullptr,
+                            st.x0, A.w, tc::smem_u32(shared_rows) + ss * shared_bytes, lane);
+                    warp_copy_row<CCB, false>(row_in ? A.b + ((size_t)st.img * A.h + y) * A.w * (8 * CCB) : nullptr, st.x0,
+                                              A.w, dst, lane);
+                } else {
+                    warp_copy_row<CCA, false>(row_in ? A.a + ((size_t)st.img * A.h + y) * A.w * (8 * CCA) : nullptr, st.x0,
+                                              A.w, dst, lane);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
                 publish(1);  // the previous row of this warp, while this one is in flight
                 pending = (int)s;
+                spending = fresh ? (int)ss : -1;
+                js += fresh;
             }
         }
         publish(0);
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == kConvMmaWarp) {
         // ---- MMA issuer ----
-        if (lane == 0) {
-            const uint32_t halo_s = tc::smem_u32(halo), w_s = tc::smem_u32(wsm);
-            const uint32_t idesc = tc::idesc_bf16(kTileM, A.cout);
-            // descriptor bases: A at a slot's first plane (LBO = plane stride),
-            // B at the first weight plane; an MMA adds its byte offset >> 4
-            const uint64_t a_desc0 = tc::desc(halo_s, kHaloW * 16, 128);
-            const uint64_t b_desc0 = tc::desc(w_s, A.cout * 16, 128);
-            const uint32_t b_plane = (uint32_t)A.cout * 16;
-            uint32_t jin = 0, waited = 0, q = 0;  // input rows of earlier strips, rows known full, output rows
-            bool ok = true;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-                const Strip st = strip_of(A, item, rows_per_item);
-                const int R = st.y1 - st.y0;
-                for (int o = 0; o < R && ok; ++o, ++q) {
-                    // its input rows jin + o .. jin + o + 2
-                    for (; waited <= jin + o + 2 && ok; ++waited)
-                        ok = pipe_wait(&pp.full[waited % (uint32_t)S], (waited / (uint32_t)S) & 1u, abort, A.err);
-                    const uint32_t a = q % kConvAcc, ka = q / kConvAcc;
-                    if (ok && ka > 0) ok = pipe_wait(&pp.acc_empty[a], (ka - 1) & 1u, abort, A.err);
-                    if (!ok) break;
-                    tc::fence_after_sync();
-                    const uint32_t dacc = tmem + a * ncols;
+        // The whole warp runs this loop (every value in it is the same in all
+        // lanes), one elected lane issues, without a branch of its own: a
+        // forward pass of batch 16 took 825 us with the MMAs in a branch that
+        // the elected lane took, and takes 800 us without.
+        const uint32_t halo_s = tc::smem_u32(halo), w_s = tc::smem_u32(wsm);
+        const uint32_t s_lo0 = (uint32_t)tc::desc(tc::smem_u32(shared_rows), kPlaneBytes, 128);
+        // descriptors: A at a slot's first plane (LBO = plane stride), B at the
+        // first weight plane; an MMA adds its byte offset >> 4 to the low word
+        const uint64_t a_desc0 = tc::desc(halo_s, kPlaneBytes, 128);
+        const uint64_t b_desc0 = tc::desc(w_s, 3 * A.cout * 16, 128);
+        const uint32_t a_lo0 = (uint32_t)a_desc0, a_hi = (uint32_t)(a_desc0 >> 32);
+        const uint32_t b_lo0 = (uint32_t)b_desc0, b_hi = (uint32_t)(b_desc0 >> 32);
+        const uint32_t b_row = (uint32_t)A.cout;                      // one tap's weight rows, 16-byte units
+        const int max_rows = 256 / A.cout >= 3 ? 3 : 256 / A.cout;    // output rows of one MMA (N <= 256)
+        const uint32_t id1 = tc::idesc_bf16(kTileM, A.cout);
+        const uint32_t id_row = tc::idesc_bf16(0, A.cout) - tc::idesc_bf16(0, 0);  // one more output row
+        const uint32_t lead = tc::elect_one(), bar0 = tc::smem_u32(&pp);
+        uint32_t slot = 0, sphase = 0;      // ring slot and phase of the next input row
+        uint32_t sslot = 0, ssphase = 0;    // and of the shared row of the current one
+        int acc = 0;                        // accumulator of the next output row to start
+        uint32_t aphase = 1;                // its phase: a fresh ring needs no wait (parity of the phase before)
+        bool ok = true;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const Strip st = strip_of(A, item, rows_per_item);
+            const int R = st.y1 - st.y0;
+            for (int i = 0; i < R + 2; ++i) {
+                const int y = st.y0 - 1 + i;
+                ok = pipe_wait(&pp.full[slot], sphase, abort, A.err);
+                if (CS && ok && (i == 0 || !(y & 1))) ok = pipe_wait(&pp.sfull[sslot], ssphase, abort, A.err);
+                // output rows lo .. hi of the strip; row i, if there is one, starts here
+                const int lo = i < 2 ? 0 : i - 2, hi = i < R ? i : R - 1;
+                if (ok && i < R) ok = pipe_wait(&pp.acc_empty[acc], aphase, abort, A.err);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc::fence_after_sync();
+                // accumulator of row lo: acc is that of row i, or of the one after hi
+                int alo = acc - ((i < R ? i : R) - lo);
+                if (alo < 0) alo += NA;
+                // their accumulators are adjacent but for the ring's end: one or two runs
+                const int n = hi - lo + 1;
+                const int n0 = min(min(n, NA - alo), max_rows);
+                const uint32_t b0 = (uint32_t)(lo - i + 2) * b_row;
+                const uint32_t d0 = tmem + (uint32_t)alo * ncols;
+                // chunk kc of horizontal tap dx: in the shared row, or in this row's slot
+                const uint32_t o_lo = a_lo0 + ((slot * slot_bytes) >> 4), s_lo = s_lo0 + ((sslot * shared_bytes) >> 4);
+                auto a_at = [&](int dx, int kc) {
+                    return (kc < CS ? s_lo + (uint32_t)((kc * kPlaneBytes + dx * 128) >> 4)
+                                    : o_lo + (uint32_t)(((kc - CS) * kPlaneBytes + dx * 128) >> 4));
+                };
+                const uint32_t a_lo = a_at(0, 0);
+                const uint32_t done = alo;   // row lo is complete after this input row when i >= 2
+                {
+                    if (n0 == n) {
+                        const uint32_t id = id1 + (uint32_t)(n - 1) * id_row;
+                        // a new output row overwrites its accumulator
+                        if (i < R) {
+                            tc::mma_bf16<false>(d0 + (uint32_t)(n - 1) * ncols, a_lo, a_hi, b_lo0 + 2 * b_row, b_hi, id1, lead);
+                            if (n > 1) tc::mma_bf16<true>(d0, a_lo, a_hi, b_lo0 + b0, b_hi, id - id_row, lead);
+                        } else {
+                            tc::mma_bf16<true>(d0, a_lo, a_hi, b_lo0 + b0, b_hi, id, lead);
+                        }
 #pragma unroll
-                    for (int t = 0; t < 9; ++t) {
-                        const int dy = t / 3, dx = t % 3;
-                        const uint32_t a_off = ((jin + o + dy) % (uint32_t)S) * slot_bytes + dx * 16;
+                        for (int m = 1; m < 3 * CC / 2; ++m) {
+                            const int dx = m / (CC / 2), kc = 2 * (m % (CC / 2));
+                            tc::mma_bf16<true>(d0, a_at(dx, kc), a_hi,
+                                               b_lo0 + b0 + (uint32_t)(dx * CC + kc) * 3u * b_row, b_hi, id, lead);
+                        }
+                    } else {
+                        const int n1 = n - n0;
+                        const uint32_t d1 = alo + n0 == NA ? tmem : d0 + (uint32_t)n0 * ncols;
+                        const uint32_t b1 = b0 + (uint32_t)n0 * b_row;
+                        const uint32_t i0 = id1 + (uint32_t)(n0 - 1) * id_row, i1 = id1 + (uint32_t)(n1 - 1) * id_row;
+                        tc::mma_bf16<true>(d0, a_lo, a_hi, b_lo0 + b0, b_hi, i0, lead);
+                        if (i < R) {
+                            if (n1 > 1) tc::mma_bf16<true>(d1, a_lo, a_hi, b_lo0 + b1, b_hi, id1, lead);
+                            tc::mma_bf16<false>(d1 + (uint32_t)(n1 - 1) * ncols, a_lo, a_hi, b_lo0 + 2 * b_row, b_hi, id1, lead);
+                        } else {
+                            tc::mma_bf16<true>(d1, a_lo, a_hi, b_lo0 + b1, b_hi, i1, lead);
+                        }
 #pragma unroll
-                        for (int kc = 0; kc < CC; kc += 2) {
-                            const uint64_t ad = a_desc0 + ((a_off + (uint32_t)kc * kHaloW * 16) >> 4);
-                            const uint64_t bd = b_desc0 + (((uint32_t)(t * CC + kc) * b_plane) >> 4);
-                            tc::mma_bf16(dacc, ad, bd, idesc, (t | kc) ? 1u : 0u);
+                        for (int m = 1; m < 3 * CC / 2; ++m) {
+                            const int dx = m / (CC / 2), kc = 2 * (m % (CC / 2));
+                            const uint32_t ad = a_at(dx, kc);
+                            const uint32_t bd = b_lo0 + (uint32_t)(dx * CC + kc) * 3u * b_row;
+                            tc::mma_bf16<true>(d0, ad, a_hi, bd + b0, b_hi, i0, lead);
+                            tc::mma_bf16<true>(d1, ad, a_hi, bd + b1, b_hi, i1, lead);
                         }
                     }
-                    tc::commit(&pp.acc_full[a]);
-                    // input row o is read by no later output row of the strip;
-                    // after the last output row, neither are the two below it
-                    tc::commit(&pp.empty[(jin + o) % (uint32_t)S]);
-                    if (o == R - 1) {
-                        tc::commit(&pp.empty[(jin + o + 1) % (uint32_t)S]);
-                        tc::commit(&pp.empty[(jin + o + 2) % (uint32_t)S]);
-                    }
+                    tc::commit_lead(bar0 + (uint32_t)offsetof(ConvPipe, empty) + 8u * slot, lead);  // this input row is read by no later MMA
+                    if (CS && ((y & 1) || i == R + 1)) tc::commit_lead(bar0 + (uint32_t)offsetof(ConvPipe, sempty) + 8u * sslot, lead);
+                    if (i >= 2) tc::commit_lead(bar0 + (uint32_t)offsetof(ConvPipe, acc_full) + 8u * done, lead);
                 }
-                jin += (uint32_t)(R + 2);
+                if (++slot == (uint32_t)S) {
+                    slot = 0;
+                    sphase ^= 1u;
+                }
+                if (CS && ((y & 1) || i == R + 1) && ++sslot == (uint32_t)SS) {
+                    sslot = 0;
+                    ssphase ^= 1u;
+                }
+                if (i < R && ++acc == NA) {
+                    acc = 0;
+                    aphase ^= 1u;
+                }
             }
-            // every MMA issued has finished before the tensor memory is freed
-            tc::commit(&pp.drain);
-            tc::mbar_wait(&pp.drain, 0u, kConvWaitNs);
         }
+        // every MMA issued has finished before the tensor memory is freed
+        tc::commit_lead(tc::smem_u32(&pp.drain), lead);
+        __syncwarp();
+        tc::mbar_wait(&pp.drain, 0u, kConvWaitNs);
         __syncwarp();
     } else {
-        // ---- epilogue: warp q drains TMEM lanes 32q .. 32q + 31 ----
-        uint32_t q = 0;
-        uint4 keep[kPoolMaxChunks];
-        for (int item = blockIdx.x; item < items && !*abort; item += gridDim.x) {
-            const Strip st = strip_of(A, item, rows_per_item);
-            bool ok = true;
-            for (int y = st.y0; y < st.y1; ++y, ++q) {
-                const int x = st.x0 + warp * 32 + lane;
-                float din = 0.f;  // the head's input depth, fetched before the wait
-                if (A.head_w && x < A.w) din = __ldg(A.depth_in + ((size_t)st.img * A.h + y) * A.w + x);
-                const uint32_t a = q % kConvAcc, ka = q / kConvAcc;
-                if (!(ok = pipe_wait(&pp.acc_full[a], ka & 1u, abort, A.err))) break;
-                tc::fence_after_sync();
-                conv_epilogue(A, tmem + a * ncols, warp, lane, st.img, y, st.x0, din, keep, s_bias, s_head);
-                tc::fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&pp.acc_empty[a]);
-            }
-            if (!ok) break;
+        // ---- epilogue ----
+        // (the output channels that the network's layers and their gradients
+        // have with this many input channels)
+#define TDE_EPILOGUE(N, P) \
+    conv_epilogue<N, P, SETS>(A, pp, s_bias, s_head, stage, rows_per_item, items, NA, warp, lane)
+        if constexpr (MODE == SRC_UP) {
+            TDE_EPILOGUE(8 * CCB, false);
+        } else if constexpr (SETS == 1) {
+            TDE_EPILOGUE(8 * CCA, true);
+        } else if constexpr (CCA == 2) {
+            if (A.cout == 16) TDE_EPILOGUE(16, false);
+            else if (A.cout == 32) TDE_EPILOGUE(32, false);
+            else TDE_EPILOGUE(48, false);
+        } else if constexpr (CCA == 4) {
+            if (A.cout == 16) TDE_EPILOGUE(16, false);
+            else if (A.cout == 32) TDE_EPILOGUE(32, false);
+            else if (A.cout == 48) TDE_EPILOGUE(48, false);
+            else TDE_EPILOGUE(80, false);
+        } else if constexpr (CCA == 6) {
+            if (A.cout == 32) TDE_EPILOGUE(32, false);
+            else if (A.cout == 48) TDE_EPILOGUE(48, false);
+            else if (A.cout == 64) TDE_EPILOGUE(64, false);
+            else TDE_EPILOGUE(112, false);
+        } else {
+            if (A.cout == 48) TDE_EPILOGUE(48, false);
+            else TDE_EPILOGUE(64, false);
         }
+#undef TDE_EPILOGUE
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -477,11 +745,16 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const ConvArgs
     X(SRC_DIRECT, 2, 0) X(SRC_DIRECT, 4, 0) X(SRC_DIRECT, 6, 0) X(SRC_DIRECT, 8, 0) \
     X(SRC_UP, 4, 2) X(SRC_UP, 6, 4) X(SRC_UP, 8, 6)
 
-// The kernel for a source mode and the input chunks of sources A and B.
-const void *conv_kernel_fn(int mode, int cca, int ccb) {
+// The kernel for a source mode, the input chunks of sources A and B, and
+// whether the output is pooled as well.
+const void *conv_kernel_fn(int mode, int cca, int ccb, bool pool) {
 #define TDE_CONV_FN(M, A, B) \
-    if (mode == M && cca == A && ccb == B) return (const void *)conv3x3_tc_kernel<M, A, B>;
+    if (mode == M && cca == A && ccb == B && !pool) return (const void *)conv3x3_tc_kernel<M, A, B, conv_epi_sets(M, false)>;
     TDE_CONV_VARIANTS(TDE_CONV_FN)
+#undef TDE_CONV_FN
+#define TDE_CONV_FN(A) \
+    if (mode == SRC_DIRECT && cca == A && ccb == 0 && pool) return (const void *)conv3x3_tc_kernel<SRC_DIRECT, A, 0, 1>;
+    TDE_CONV_FN(2) TDE_CONV_FN(4) TDE_CONV_FN(6)
 #undef TDE_CONV_FN
     return nullptr;
 }
@@ -543,6 +816,22 @@ struct WgPipe {
     uint32_t tmem;
     int abort;
 };
+
+// Pixels x_start .. x_start + kWgHalo - 1 of one row as planes of kWgHalo
+// pixels in order; consecutive lanes copy consecutive 16-byte pieces of the row.
+template <int CP, bool UPS>
+__device__ __forceinline__ void wg_copy_part(const bf16 *row, int px_elems, int w, int x_start, int plane0, bool row_in,
+                                             unsigned char *slot, const bf16 *dummy, int lane) {
+    for (int i = lane; i < kWgHalo * CP; i += 32) {
+        const int px = i / CP, c = i - px * CP;
+        const int x = x_start + px;
+        const bool in = row_in && (unsigned)x < (unsigned)w;
+        const bf16 *src = in ? row + (size_t)(UPS ? (x >> 1) : x) * px_elems + 8 * c : dummy;
+        const uint32_t dst = tc::smem_u32(slot + ((size_t)(plane0 + c) * kWgHalo + px) * 16);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
+                     : "memory");
+    }
+}
 
 template <int MODE, int CCA, int CCB>
 __global__ void __launch_bounds__(kWgThreadsP) wgrad_tc_kernel(const WgradArgs A, int S) {
@@ -606,14 +895,14 @@ __global__ void __launch_bounds__(kWgThreadsP) wgrad_tc_kernel(const WgradArgs A
                 const int yc = row_in ? yy : 0;
                 if (MODE == SRC_UP) {
                     const bf16 *ra = A.a + (((size_t)img * (A.h >> 1) + (yc >> 1)) * (A.w >> 1)) * A.ca;
-                    warp_copy_part<CCA, true, kWgHalo>(ra, A.ca, A.w, x0 - 1, dy * CC, row_in, xs, A.a, lane);
+                    wg_copy_part<CCA, true>(ra, A.ca, A.w, x0 - 1, dy * CC, row_in, xs, A.a, lane);
                 } else {
                     const bf16 *ra = A.a + (((size_t)img * A.h + yc) * A.w) * A.ca;
-                    warp_copy_part<CCA, false, kWgHalo>(ra, A.ca, A.w, x0 - 1, dy * CC, row_in, xs, A.a, lane);
+                    wg_copy_part<CCA, false>(ra, A.ca, A.w, x0 - 1, dy * CC, row_in, xs, A.a, lane);
                 }
                 if (CCB > 0) {
                     const bf16 *rb = A.b + (((size_t)img * A.h + yc) * A.w) * A.cb;
-                    warp_copy_part<CCB, false, kWgHalo>(rb, A.cb, A.w, x0 - 1, dy * CC + CCA, row_in, xs, A.a, lane);
+                    wg_copy_part<CCB, false>(rb, A.cb, A.w, x0 - 1, dy * CC + CCA, row_in, xs, A.a, lane);
                 }
             }
             // dZ: planes of 8 output channels over 64 pixels, zero past the row end
@@ -1060,10 +1349,11 @@ int prepare_kernels() {
     // launches (also inside stream capture) make no other runtime call
     std::vector<const void *> fns;
 #define TDE_CONV_FN(M, A, B) \
-    fns.push_back((const void *)conv3x3_tc_kernel<M, A, B>); \
+    fns.push_back(conv_kernel_fn(M, A, B, false)); \
     fns.push_back((const void *)wgrad_tc_kernel<M, A, B>);
     TDE_CONV_VARIANTS(TDE_CONV_FN)
 #undef TDE_CONV_FN
+    for (int cca = 2; cca <= 6; cca += 2) fns.push_back(conv_kernel_fn(SRC_DIRECT, cca, 0, true));
     for (const void *fn : fns) {
         cudaFuncAttributes fa;
         TDE_CUDA(cudaFuncGetAttributes(&fa, fn), "refiner: kernel attributes");
@@ -1074,44 +1364,71 @@ int prepare_kernels() {
     return TDE_OK;
 }
 
-int conv_plan(int mode, int ca, int cin, int cout, ConvPlan *out) {
+int conv_plan(int mode, int ca, int cin, int cout, bool pool, ConvPlan *out) {
     // Two resident blocks per SM when the tensor memory, the registers and the
     // shared memory allow them at least kConvMinSlots input rows each, else
     // one; the ring takes as many rows (up to kConvMaxSlots) as then fit.  The
     // shared memory is padded so that no further block becomes resident.
-    const void *fn = conv_kernel_fn(mode, ca / 8, (cin - ca) / 8);
+    const void *fn = conv_kernel_fn(mode, ca / 8, (cin - ca) / 8, pool);
     if (!fn) return set_error(TDE_ERR_UNSUPPORTED, "refiner conv: no kernel for mode %d with %d + %d input channels", mode,
                               ca, cin - ca);
     cudaFuncAttributes fa;
     TDE_CUDA(cudaFuncGetAttributes(&fa, fn), "refiner: kernel attributes");
-    const size_t slot = (size_t)(cin / 8) * kHaloW * 16, wb = (size_t)9 * (cin / 8) * cout * 16;
-    const int by_tmem = (int)(512u / (kConvAcc * tmem_cols(cout)));
-    const int by_regs = 65536 / (((fa.numRegs + 7) / 8) * 8 * kConvThreads);
+    const size_t shared = mode == SRC_UP ? (size_t)(ca / 8) * kPlaneBytes : 0;
+    const size_t slot = (size_t)(cin / 8) * kPlaneBytes - shared;
+    const int sets = conv_epi_sets(mode, pool), threads = conv_threads(sets);
+    const size_t weights = (size_t)9 * (cin / 8) * cout * 16, stage = 4 * sets * conv_stage_bytes(cout, pool);
+    size_t fixed = 0;
+    auto need = [&](size_t S) { return S * slot + (shared ? (size_t)shared_slots((int)S) * shared : 0) + fixed; };
+    const int by_tmem = (int)(512u / tmem_cols(kConvMinAcc * cout));
+    const int by_regs = 65536 / (((fa.numRegs + 7) / 8) * 8 * threads);
     int bps = by_tmem < by_regs ? by_tmem : by_regs;
-    bps = bps > 2 ? 2 : bps;
+    bps = bps > kConvMaxPerSM ? kConvMaxPerSM : bps;
     for (; bps >= 1; --bps) {
         const size_t budget = kSmemPerSM / bps - 1024 - fa.sharedSizeBytes;
-        if (budget < wb + kConvMinSlots * slot) continue;
-        size_t S = (budget - wb) / slot;
-        S = S > (size_t)kConvMaxSlots ? (size_t)kConvMaxSlots : S;
-        size_t smem = S * slot + wb;
+        fixed = weights + stage;
+        out->staged = budget >= need(kConvMinSlots);
+        if (!out->staged) fixed = weights;
+        if (budget < need(kConvMinSlots)) continue;
+        size_t S = kConvMinSlots;
+        while (S < (size_t)kConvMaxSlots && need(S + 1) <= budget) ++S;
+        size_t smem = need(S);
         const size_t floor = kSmemPerSM / (bps + 1) - 1024 - fa.sharedSizeBytes + 16;
         if (smem < floor) smem = floor;
         out->per_sm = bps;
+        out->threads = threads;
         out->slots = (int)S;
+        // as many accumulator rows as the block's share of tensor memory holds
+        int acc = kConvMaxAcc;
+        while (tmem_cols(acc * cout) * (uint32_t)bps > 512u) --acc;
+        out->acc = acc;
         out->smem = smem;
         return TDE_OK;
     }
     return set_error(TDE_ERR_UNSUPPORTED, "refiner conv: cin=%d cout=%d does not fit an SM", cin, cout);
 }
 
+// Whether conv3x3_tc_kernel has an epilogue for these channels.
+static bool epilogue_for(int mode, int cca, int ccb, int cout, bool pool) {
+    if (mode == SRC_UP) return cout == 8 * ccb && !pool;
+    if (pool) return cca < 8 && cout == 8 * cca;
+    switch (cca) {
+    case 2: return cout == 16 || cout == 32 || cout == 48;
+    case 4: return cout == 16 || cout == 32 || cout == 48 || cout == 80;
+    case 6: return cout == 32 || cout == 48 || cout == 64 || cout == 112;
+    default: return cca == 8 && (cout == 48 || cout == 64);
+    }
+}
+
 int launch_conv(const ConvArgs &a, const ConvPlan &plan, int num_sms, cudaStream_t s) {
     const int cin = a.ca + a.cb;
     if (cin % 16 || a.ca % 8 || a.cout % 16 || a.cout < 16 || a.cout > 128 || cin > 128 || a.w <= 0 || a.h <= 0 ||
         a.n <= 0 || (a.head_w && a.cout != 16) || (a.mode_a == SRC_UP && (a.h % 2 || a.w % 2)) ||
-        (a.pool_out && (a.h % 2 || a.w % 2 || a.cout > 8 * kPoolMaxChunks)))
+        (a.pool_out && (a.h % 2 || a.w % 2 || a.mask)) ||
+        !epilogue_for(a.mode_a, a.ca / 8, a.cb / 8, a.cout, a.pool_out != nullptr))
         return set_error(TDE_ERR_INVALID_ARG, "refiner conv: unsupported shape cin=%d cout=%d", cin, a.cout);
-    if (plan.slots < kConvMinSlots || plan.slots > kConvMaxSlots || plan.per_sm < 1 || plan.smem > 227 * 1024 - 256)
+    if (plan.slots < kConvMinSlots || plan.slots > kConvMaxSlots || plan.per_sm < 1 || plan.smem > 227 * 1024 - 256 ||
+        plan.acc < kConvMinAcc || plan.acc > kConvMaxAcc || tmem_cols(plan.acc * a.cout) * plan.per_sm > 512)
         return set_error(TDE_ERR_INVALID_ARG, "refiner conv: bad launch plan");
     // rows per block: as many as keep every resident block busy
     const int tiles_x = (a.w + kTileM - 1) / kTileM;
@@ -1128,7 +1445,7 @@ int launch_conv(const ConvArgs &a, const ConvPlan &plan, int num_sms, cudaStream
     const int grid = (int)(items < slots ? items : slots);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kConvThreads);
+    cfg.blockDim = dim3(plan.threads);
     cfg.dynamicSmemBytes = plan.smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -1136,11 +1453,11 @@ int launch_conv(const ConvArgs &a, const ConvPlan &plan, int num_sms, cudaStream
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const void *fn = conv_kernel_fn(a.mode_a, a.ca / 8, a.cb / 8);
+    const void *fn = conv_kernel_fn(a.mode_a, a.ca / 8, a.cb / 8, a.pool_out != nullptr);
     if (!fn) return set_error(TDE_ERR_UNSUPPORTED, "refiner conv: no kernel for mode %d with %d + %d input channels",
                               a.mode_a, a.ca, a.cb);
-    int S = plan.slots;
-    void *args[] = {(void *)&a, (void *)&rows, (void *)&S};
+    int S = plan.slots, NA = plan.acc, staged = plan.staged;
+    void *args[] = {(void *)&a, (void *)&rows, (void *)&S, (void *)&NA, (void *)&staged};
     cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "refiner conv: %s", cudaGetErrorString(e));
     return check_launch("refiner conv");

@@ -59,13 +59,16 @@ struct WgradArgs {
 // Once per process and device, before any launch: shared-memory limits.
 int prepare_kernels();
 // Launch geometry of one convolution shape, fixed once: resident blocks per
-// SM, input rows in each block's ring, dynamic shared memory per block.
+// SM, threads a block, input rows in each block's ring, output rows in its ring of accumulators,
+// dynamic shared memory per block.
 struct ConvPlan {
-    int per_sm, slots;
+    int per_sm, threads, slots, acc;
+    bool staged;  // results go to global memory through shared memory
     size_t smem;
 };
-// ca of the cin input channels come from source A (the rest from B).
-int conv_plan(int mode, int ca, int cin, int cout, ConvPlan *out);
+// ca of the cin input channels come from source A (the rest from B); pool: the
+// output is pooled too.
+int conv_plan(int mode, int ca, int cin, int cout, bool pool, ConvPlan *out);
 // One lane waits, with the kernels' bounded wait, for a barrier phase nothing
 // completes; out (device, 2 values): the raised flag and the nanoseconds waited.
 int launch_wait_selftest(uint64_t limit_ns, unsigned long long *out, cudaStream_t s);
