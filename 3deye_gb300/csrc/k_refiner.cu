@@ -15,12 +15,11 @@
 // The input gradient is the same kernel run on the output gradient with the
 // transposed, tap-flipped weights.
 //
-// Weight gradient (wgrad_tc_kernel): M = 128 rows of (tap row, input
-// channel), N = output channels, K = pixels, with MN-major operands read from
-// the staged NHWC data; an all-ones operand gives the bias gradient.  Each
-// block accumulates its share of the pixels in tensor memory and writes one
-// partial; a reduction kernel sums the partials in a fixed order
-// (deterministic).
+// Weight gradient (wgrad_tc_kernel): M = (horizontal tap, output channel), N =
+// (vertical tap, input channel), K = pixels, with MN-major operands read from
+// the staged NHWC data.  Each block accumulates its share of the pixels in
+// tensor memory and writes one partial; a reduction kernel sums the partials in
+// a fixed order (deterministic).
 #include <cuda_bf16.h>
 
 #include <cstddef>
@@ -42,11 +41,9 @@ constexpr int kTileM = 128;             // output pixels per MMA tile
 // memory, where with the pixels in order it would start 16 or 32 bytes into one.
 constexpr int kRowGroups = 18;
 constexpr int kPlaneBytes = kRowGroups * 128;  // one 8-channel chunk of a staged row
-constexpr int kWgK = 64;                // pixels per weight-gradient K step
-constexpr int kWgHalo = kWgK + 2;
 constexpr uint32_t kSmemPerSM = 228 * 1024;
 
-__host__ __device__ inline uint32_t tmem_cols(int n) {
+__host__ __device__ constexpr uint32_t tmem_cols(int n) {
     uint32_t c = 32;
     while (c < (uint32_t)n) c <<= 1;
     return c;
@@ -762,238 +759,357 @@ const void *conv_kernel_fn(int mode, int cca, int ccb, bool pool) {
 // ---------------------------------------------------------------------------
 // Weight gradient
 //
-// dW[co][t][ci] = sum_p dZ[p][co] X[p + s_t][ci] as D = A B with K = pixels,
-// both operands MN-major: the tensor core reads the staged NHWC data as it
-// lies.  X is staged per 64-pixel step as planes of 8-channel chunks (3 rows
-// x 66 halo pixels, 16 B per pixel); for horizontal tap offset dx, the rows
-// (dy, ci) of A are the planes in order (a uniform chunk stride) and the
-// pixel window starts dx pixels later (16 * dx bytes).  dZ is staged the same
-// way (planes of 8 output channels).  The bias gradient is the same MMA with
-// a constant all-ones A.  Without swizzling, a descriptor's LBO is the stride
-// between 8-element groups along K and its SBO the stride along M (or N), for
-// MN-major operands as for K-major ones.
+// dW[co][dy][dx][ci] = sum over output pixels of dZ[y][x][co] X[y+dy-1][x+dx-1][ci],
+// as D = A B with K = pixels, both operands MN-major: the tensor core reads the
+// staged NHWC data as it lies, as planes of 8 channels (16 bytes a pixel).  For
+// output row y and input pixels q of a column of KP = 128 pixels (64 in the
+// layers whose rings would not fit):
+//   A, M = (dx, co): three copies of dZ's row y, copy dx shifted so that pixel q
+//     holds dZ[y][q + 1 - dx];
+//   B, N = (dy, ci): X's rows y - 1, y, y + 1, neighbours in a ring of rows.
+// One MMA per 16 pixels then does all nine taps of a layer whose 3 cout fit in
+// M = 128 (two MMAs beyond; two more where the ring wraps), and each row of X is
+// staged once for the three output rows it belongs to.  Before, an MMA did one
+// horizontal tap and 128 rows (dy, ci) of X -- 28 MMAs where this takes 4, at some
+// 100 cycles of issue each -- and X was staged three times; wgrad of c11 and c2 at
+// batch 16 of 640x480: 811 and 576 us then, 238 and 156 us now, of all layers
+// together 2230 and 940 (about 1800 cycles a step of 128 pixels remain).
+// Rows of A past 3 cout read whatever follows in shared memory; their rows of D
+// are not used.  The bias gradient is summed on the CUDA cores from copy dx = 1.
+// Without swizzling, a descriptor's LBO is the stride between 8-element groups
+// along K and its SBO the stride along M (or N), for MN-major operands as for
+// K-major ones.
+//
+// A block takes a contiguous share of all (image, column, row) steps, rows
+// fastest; each stretch of one column is a run of n output rows and n + 2 rows
+// of X, staged as units: unit u holds X row u and dZ row u - 2 of the run.
+//   warps 0-3 (producers): unit j goes to warp j & 3, two in flight each;
+//   warp 4 (MMA issuer): at unit u >= 2 the MMAs of output row u - 2, committed to
+//     the dZ slot and to the slot of the X row no later step reads;
+//   warps 5-8: sum dZ for the bias; at the end drain the accumulators, which
+//     stay in tensor memory across all the block's steps, into its partial.
+// Bounded waits as in the convolution.
 // ---------------------------------------------------------------------------
-constexpr int kWgPlaneX = kWgHalo * 16;   // 1056 B: one 8-channel plane of X
-constexpr int kWgPlaneZ = kWgK * 16;      // 1024 B: one 8-channel plane of dZ
-
-struct WgLayout {
-    int cin, cc, mtiles, xplanes, zplanes;
-    uint32_t x_bytes, z_bytes, tcols;
-};
-__host__ __device__ inline WgLayout wg_layout(int cin, int cout) {
-    WgLayout L;
-    L.cin = cin;
-    L.cc = cin / 8;
-    L.mtiles = (3 * cin + 127) / 128;                 // rows (dy, ci) per horizontal offset
-    L.xplanes = max(3 * L.cc, 16 * L.mtiles);         // MMAs read whole 16-chunk row tiles
-    L.zplanes = cout / 8;
-    L.x_bytes = (uint32_t)(L.xplanes * kWgPlaneX);
-    L.z_bytes = (uint32_t)(L.zplanes * kWgPlaneZ);
-    L.tcols = (uint32_t)(3 * L.mtiles * cout + cout);  // 3 dx x row tiles, + bias
-    return L;
+constexpr int kWgProdWarps = 4, kWgMmaWarp = 4, kWgBiasWarps = 4;
+constexpr int kWgThreads = 32 * (kWgProdWarps + 1 + kWgBiasWarps);
+constexpr int kWgMaxFlight = 8;
+// Pixels of a step, and units in flight beside the step being multiplied, for
+// cc input and cz output chunks: what one block's shared memory holds.  The dZ
+// ring has no fewer slots than producer warps (as the convolution's ring).
+__host__ __device__ constexpr uint32_t wg_smem(int cc, int cz, int kp, int flight) {
+    return (uint32_t)(((flight + 1) * 3 * cz + (flight + 3) * cc) * kp * 16);
+}
+constexpr uint32_t kWgSmem = 224 * 1024;
+__host__ __device__ constexpr int wg_kp(int cc, int cz) { return wg_smem(cc, cz, 128, 3) <= kWgSmem ? 128 : 64; }
+__host__ __device__ constexpr int wg_flight(int cc, int cz) {
+    int f = 3;
+    while (f < kWgMaxFlight && wg_smem(cc, cz, wg_kp(cc, cz), f + 1) <= kWgSmem) ++f;
+    return f;
 }
 
 // MN-major kind::f16 instruction descriptor (bits 15, 16 = 1).
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
     return tc::idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
+__host__ __device__ constexpr int wg_mtiles(int cout) { return (3 * cout + 127) / 128; }
+// Floats of one block's partial: [3 cout][3 cin], then the bias.
+__host__ __device__ constexpr int wg_partial(int cin, int cout) { return 9 * cin * cout + cout; }
 
-// Pipelined form: a block owns K steps k = blockIdx.x, + gridDim.x, ... (one
-// 64-pixel segment of one row each).  Up to 8 producer warps stage step k --
-// X over 3 rows x 66 halo pixels and dZ over 64 pixels, as planes, with
-// cp.async -- into ring stage k % S once the tensor core has released it
-// (step k - S done), warp k % min(S, 8) taking step k; warp 8, one lane, issues each
-// step's MMAs into the block's accumulators (3 dx x row tiles + the bias
-// column block), which stay in tensor memory across all the block's steps,
-// and commits them to the stage's "empty" barrier.  At the end every warp
-// drains the accumulators into the block's partial.  Bounded waits as in the
-// convolution: a timeout raises A.err and the block leaves cleanly.
-constexpr int kWgProdWarps = 8;
-constexpr int kWgThreadsP = 32 * (kWgProdWarps + 1);
-constexpr int kWgMaxStages = 8;
 struct WgPipe {
-    uint64_t full[kWgMaxStages], empty[kWgMaxStages], drain;
+    uint64_t full[kWgMaxFlight + 3], empty[kWgMaxFlight + 3], zempty[kWgMaxFlight + 1], drain;
     uint32_t tmem;
     int abort;
 };
 
-// Pixels x_start .. x_start + kWgHalo - 1 of one row as planes of kWgHalo
-// pixels in order; consecutive lanes copy consecutive 16-byte pieces of the row.
-template <int CP, bool UPS>
-__device__ __forceinline__ void wg_copy_part(const bf16 *row, int px_elems, int w, int x_start, int plane0, bool row_in,
-                                             unsigned char *slot, const bf16 *dummy, int lane) {
-    for (int i = lane; i < kWgHalo * CP; i += 32) {
-        const int px = i / CP, c = i - px * CP;
-        const int x = x_start + px;
-        const bool in = row_in && (unsigned)x < (unsigned)w;
-        const bf16 *src = in ? row + (size_t)(UPS ? (x >> 1) : x) * px_elems + 8 * c : dummy;
-        const uint32_t dst = tc::smem_u32(slot + ((size_t)(plane0 + c) * kWgHalo + px) * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
-                     : "memory");
+// Copies of CP = 2 or 4 channel chunks of KP pixels of a row (PXE channels a
+// pixel) from pixel x_start on, read directly or through the nearest 2x
+// upsample (x_start even then), into planes; zeros past the row's ends.  Eight
+// lanes take eight neighbouring pixels of one chunk, the four such sets of a
+// warp the chunks of the same pixels.
+template <int KP, int CP, bool UPS, int PXE>
+__device__ __forceinline__ void wg_copy_chunks(const bf16 *row, int x_start, int w, uint32_t dst, int lane) {
+    const int k = lane & 7, l3 = lane >> 3;
+    const int c = CP == 4 ? l3 : l3 & 1, bl = CP == 4 ? 0 : l3 >> 1;
+    const int x = x_start + 8 * bl + k, lim = w - x;
+    const bf16 *src = row + (UPS ? (x_start >> 1) + 4 * bl + (k >> 1) : x) * PXE + 8 * c;
+    dst += (uint32_t)(c * KP * 16 + (8 * bl + k) * 16);
+#pragma unroll
+    for (int it = 0; it < KP * CP / 32; ++it) {
+        const int px = (CP == 4 ? 8 : 16) * it;
+        if (px < lim && (it > 0 || x >= 0))
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + px * 16), "l"(src + (UPS ? px / 2 : px) * PXE)
+                         : "memory");
+        else
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst + px * 16), "r"(0) : "memory");
+    }
+}
+template <int KP, int CC, bool UPS>
+__device__ __forceinline__ void wg_copy_row(const bf16 *row, int x_start, int w, uint32_t dst, int lane) {
+    if (row) {
+#pragma unroll
+        for (int c = 0; c + 4 <= CC; c += 4)
+            wg_copy_chunks<KP, 4, UPS, 8 * CC>(row + 8 * c, x_start, w, dst + c * KP * 16, lane);
+        if constexpr (CC % 4 != 0)
+            wg_copy_chunks<KP, 2, UPS, 8 * CC>(row + 8 * (CC - 2), x_start, w, dst + (CC - 2) * KP * 16, lane);
+    } else {
+        for (int i = lane; i < CC * KP; i += 32)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst + i * 16), "r"(0) : "memory");
     }
 }
 
-template <int MODE, int CCA, int CCB>
-__global__ void __launch_bounds__(kWgThreadsP) wgrad_tc_kernel(const WgradArgs A, int S) {
-    constexpr int CC = CCA + CCB;
+// A stretch of one column: image, first pixel, output rows [y0, y1).
+struct WgRun { int img, x0, y0, y1; };
+template <int KP> __device__ __forceinline__ WgRun wg_run(const WgradArgs &A, int step, int last) {
+    const int tiles_x = (A.w + KP - 1) / KP;
+    const int col = step / A.h;
+    WgRun r;
+    r.img = col / tiles_x;
+    r.x0 = (col - r.img * tiles_x) * KP;
+    r.y0 = step - col * A.h;
+    r.y1 = min(A.h, r.y0 + last - step);
+    return r;
+}
+
+template <int MODE, int CCA, int CCB, int CZ>
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const WgradArgs A) {
+    constexpr int CC = CCA + CCB, CIN = 8 * CC, COUT = 8 * CZ, MT = wg_mtiles(COUT), N = 3 * CIN;
+    constexpr int KP = wg_kp(CC, CZ), kRowSlots = wg_flight(CC, CZ) + 3, kDzSlots = wg_flight(CC, CZ) + 1;
+    constexpr int kPlane = KP * 16;  // one 8-channel plane of a row
+    constexpr uint32_t xbytes = CC * kPlane, zbytes = 3 * CZ * kPlane;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ WgPipe pp;
-    const int cin = A.ca + A.cb, cout = A.cout;
-    const WgLayout L = wg_layout(cin, cout);
-    const int zc = cout / 8;
+    __shared__ float s_bias[kWgBiasWarps][COUT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t ncols = tmem_cols((int)L.tcols);
-    const uint32_t stage_bytes = L.x_bytes + L.z_bytes;
-    unsigned char *ones = smem + (size_t)S * stage_bytes;
+    constexpr uint32_t tcols = tmem_cols(MT * N);
+    // dZ ring first: the rows of A that a tile of 128 reads past it are X's
+    unsigned char *zring = smem, *xring = smem + kDzSlots * zbytes;
     volatile int *abort = &pp.abort;
-
-    if (warp == kWgProdWarps) tc::tmem_alloc(&pp.tmem, ncols);
+    if (warp == kWgMmaWarp) tc::tmem_alloc(&pp.tmem, tcols);
     if (tid == 0) {
-        for (int s = 0; s < kWgMaxStages; ++s) {
+        for (int s = 0; s < kRowSlots; ++s) {
             tc::mbar_init(&pp.full[s], 1);
             tc::mbar_init(&pp.empty[s], 1);
         }
+        for (int s = 0; s < kDzSlots; ++s) tc::mbar_init(&pp.zempty[s], 1 + kWgBiasWarps);
         tc::mbar_init(&pp.drain, 1);
         pp.abort = 0;
     }
-    {
-        const uint4 one8 = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);  // eight bf16 1.0
-        for (int i = tid; i < 256; i += kWgThreadsP) *reinterpret_cast<uint4 *>(ones + (size_t)i * 16) = one8;
-    }
-    tc::fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = pp.tmem;
-    const int tiles_x = (A.w + kWgK - 1) / kWgK;
-    const int ntiles = A.n * A.h * tiles_x;
-    // this block's steps: k-th step is tile blockIdx.x + k * gridDim.x
-    const int nsteps = blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const long steps = (long)A.n * A.h * ((A.w + KP - 1) / KP);
+    const int s0 = (int)(steps * blockIdx.x / gridDim.x), s1 = (int)(steps * (blockIdx.x + 1) / gridDim.x);
 
-    // Producer warps: no more than the ring has stages, so that the stage a
-    // warp waits for was released one phase ago at most (a parity wait cannot
-    // tell phase f - 1 from f - 3): steps are released in order, and a warp's
-    // previous wait already covered step k - np - S >= k - 2S.
-    const int np = S < kWgProdWarps ? S : kWgProdWarps;
-    if (warp < np) {
+    if (warp < kWgProdWarps) {
         // ---- producers ----
-        for (int k = warp; k < nsteps && !*abort; k += np) {
-            const uint32_t s = (uint32_t)k % (uint32_t)S, f = (uint32_t)k / (uint32_t)S;
-            if (f > 0 && !pipe_wait(&pp.empty[s], (f - 1) & 1u, abort, A.err)) break;
-            const int tile = blockIdx.x + k * gridDim.x;
-            const int xt = tile % tiles_x, rowi = tile / tiles_x;
-            const int y = rowi % A.h, img = rowi / A.h;
-            const int x0 = xt * kWgK;
-            unsigned char *xs = smem + (size_t)s * stage_bytes;
-            unsigned char *zs = xs + L.x_bytes;
-            // X: planes (dy, c) of 66 halo pixels; consecutive lanes take
-            // consecutive 16-byte pieces of a source pixel row
-#pragma unroll 1
-            for (int dy = 0; dy < 3; ++dy) {
-                const int yy = y + dy - 1;
-                const bool row_in = yy >= 0 && yy < A.h;
-                const int yc = row_in ? yy : 0;
-                if (MODE == SRC_UP) {
-                    const bf16 *ra = A.a + (((size_t)img * (A.h >> 1) + (yc >> 1)) * (A.w >> 1)) * A.ca;
-                    wg_copy_part<CCA, true>(ra, A.ca, A.w, x0 - 1, dy * CC, row_in, xs, A.a, lane);
-                } else {
-                    const bf16 *ra = A.a + (((size_t)img * A.h + yc) * A.w) * A.ca;
-                    wg_copy_part<CCA, false>(ra, A.ca, A.w, x0 - 1, dy * CC, row_in, xs, A.a, lane);
-                }
-                if (CCB > 0) {
-                    const bf16 *rb = A.b + (((size_t)img * A.h + yc) * A.w) * A.cb;
-                    wg_copy_part<CCB, false>(rb, A.cb, A.w, x0 - 1, dy * CC + CCA, row_in, xs, A.a, lane);
-                }
-            }
-            // dZ: planes of 8 output channels over 64 pixels, zero past the row end
-            for (int i = lane; i < kWgK * zc; i += 32) {
-                const int c = i % zc, px = i / zc;
-                const bool in = x0 + px < A.w;
-                const bf16 *src = in ? A.dz + (((size_t)img * A.h + y) * A.w + x0 + px) * cout + 8 * c : A.dz;
-                const uint32_t dst = tc::smem_u32(zs + (size_t)c * kWgPlaneZ + px * 16);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
-                             : "memory");
-            }
-            asm volatile("cp.async.wait_all;" ::: "memory");
+        uint32_t j = 0, jz = 0;  // units and dZ rows of this block so far
+        int pending = -1;
+        bool ok = true;
+        auto publish = [&](int wait_groups) {
+            if (pending < 0) return;
+            if (wait_groups) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
             tc::fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&pp.full[s]);
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (warp == kWgProdWarps && lane == 0) {
-        // ---- MMA issuer ----
-        const uint32_t s0 = tc::smem_u32(smem), ones_s = tc::smem_u32(ones);
-        const uint32_t idesc = idesc_bf16_mn(128, cout);
-        for (int k = 0; k < nsteps; ++k) {
-            const uint32_t s = (uint32_t)k % (uint32_t)S;
-            if (!pipe_wait(&pp.full[s], ((uint32_t)k / (uint32_t)S) & 1u, abort, A.err)) break;
-            tc::fence_after_sync();
-            const uint32_t xb = s0 + s * stage_bytes, zb = xb + L.x_bytes;
-            for (int kk = 0; kk < kWgK / 16; ++kk) {
-                const uint32_t acc = (k == 0 && kk == 0) ? 0u : 1u;
-                const uint64_t bd = tc::desc(zb + (uint32_t)(kk * 16 * 16), 128, kWgPlaneZ);
-                for (int dx = 0; dx < 3; ++dx)
-                    for (int mt = 0; mt < L.mtiles; ++mt) {
-                        const uint64_t ad =
-                            tc::desc(xb + (uint32_t)(16 * mt * kWgPlaneX + (kk * 16 + dx) * 16), 128, kWgPlaneX);
-                        tc::mma_bf16(tmem + (uint32_t)((dx * L.mtiles + mt) * cout), ad, bd, idesc, acc);
-                    }
-                const uint64_t od = tc::desc(ones_s, 128, 256);
-                tc::mma_bf16(tmem + (uint32_t)(3 * L.mtiles * cout), od, bd, idesc, acc);
+            if (lane == 0) mbar_arrive(&pp.full[pending]);
+            pending = -1;
+        };
+        auto wait_empty = [&](uint64_t *bar, uint32_t k) {
+            if (k == 0 || tc::mbar_test_wait(bar, (k - 1) & 1u)) return true;
+            publish(0);
+            return pipe_wait(bar, (k - 1) & 1u, abort, A.err);
+        };
+        for (int step = s0; step < s1 && ok && !*abort;) {
+            const WgRun run = wg_run<KP>(A, step, s1);
+            const int n = run.y1 - run.y0;
+            for (int u = 0; u < n + 2; ++u, ++j) {
+                const bool has_z = u >= 2;
+                if ((int)(j % (uint32_t)kWgProdWarps) != warp) {
+                    jz += has_z;
+                    continue;
+                }
+                const uint32_t s = j % (uint32_t)kRowSlots, sz = jz % (uint32_t)kDzSlots;
+                if (!(ok = wait_empty(&pp.empty[s], j / (uint32_t)kRowSlots))) break;
+                if (has_z && !(ok = wait_empty(&pp.zempty[sz], jz / (uint32_t)kDzSlots))) break;
+                const int y = run.y0 - 1 + u;
+                const bool row_in = y >= 0 && y < A.h;
+                const uint32_t xd = tc::smem_u32(xring) + s * xbytes;
+                if constexpr (MODE == SRC_UP)
+                    wg_copy_row<KP, CCA, true>(
+                        row_in ? A.a + ((size_t)run.img * (A.h >> 1) + (y >> 1)) * (A.w >> 1) * (8 * CCA) : nullptr, run.x0,
+                        A.w, xd, lane);
+                else
+                    wg_copy_row<KP, CCA, false>(row_in ? A.a + ((size_t)run.img * A.h + y) * A.w * (8 * CCA) : nullptr, run.x0,
+                                            A.w, xd, lane);
+                if constexpr (CCB > 0)
+                    wg_copy_row<KP, CCB, false>(row_in ? A.b + ((size_t)run.img * A.h + y) * A.w * (8 * CCB) : nullptr, run.x0,
+                                            A.w, xd + CCA * kPlane, lane);
+                if (has_z) {
+                    const bf16 *zrow = A.dz + ((size_t)run.img * A.h + y - 1) * A.w * COUT;
+                    const uint32_t zd = tc::smem_u32(zring) + sz * zbytes;
+#pragma unroll 1
+                    for (int dx = 0; dx < 3; ++dx)
+                        wg_copy_row<KP, CZ, false>(zrow, run.x0 + 1 - dx, A.w, zd + (uint32_t)(dx * CZ * kPlane), lane);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                publish(1);
+                pending = (int)s;
+                jz += has_z;
             }
-            tc::commit(&pp.empty[s]);
+            step += n;
+        }
+        publish(0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == kWgMmaWarp) {
+        // ---- MMA issuer (the whole warp runs the loop, one lane issues) ----
+        const uint64_t z0 = tc::desc(tc::smem_u32(zring), 128, kPlane), x0 = tc::desc(tc::smem_u32(xring), 128, kPlane);
+        const uint32_t z_lo = (uint32_t)z0, z_hi = (uint32_t)(z0 >> 32), x_lo = (uint32_t)x0, x_hi = (uint32_t)(x0 >> 32);
+        const uint32_t id1 = idesc_bf16_mn(128, CIN), id_row = tc::idesc_bf16(0, CIN) - tc::idesc_bf16(0, 0);
+        const uint32_t lead = tc::elect_one(), bar0 = tc::smem_u32(&pp);
+        const uint32_t empty0 = bar0 + (uint32_t)offsetof(WgPipe, empty), zempty0 = bar0 + (uint32_t)offsetof(WgPipe, zempty);
+        uint32_t slot = 0, sphase = 0, zslot = 0, acc = 0;
+        bool ok = true;
+        for (int step = s0; step < s1 && ok;) {
+            const WgRun run = wg_run<KP>(A, step, s1);
+            const int n = run.y1 - run.y0;
+            const int nk = (min(KP, A.w - run.x0) + 15) / 16;  // K steps with pixels of the image
+            for (int u = 0; u < n + 2; ++u) {
+                ok = __all_sync(0xffffffffu, pipe_wait(&pp.full[slot], sphase, abort, A.err));
+                if (!ok) break;
+                if (u >= 2) {
+                    tc::fence_after_sync();
+                    // X rows u - 2 .. u: one run of the ring, or two
+                    const uint32_t first = slot >= 2 ? slot - 2 : slot + kRowSlots - 2;
+                    const uint32_t r0 = min(3u, (uint32_t)kRowSlots - first);
+                    const uint32_t al = z_lo + ((zslot * zbytes) >> 4), b0 = x_lo + ((first * xbytes) >> 4);
+                    const uint32_t i0 = id1 + (r0 - 1) * id_row, i1 = id1 + (2 - r0) * id_row;
+                    for (int kk = 0; kk < nk; ++kk) {
+                        const uint32_t ko = (uint32_t)(kk * 16);  // 16 pixels, in 16-byte units
+#pragma unroll
+                        for (int mt = 0; mt < MT; ++mt) {
+                            const uint32_t a = al + ko + (uint32_t)(mt * 16 * kPlane >> 4), d = tmem + (uint32_t)(mt * N);
+                            tc::mma_bf16(d, a, z_hi, b0 + ko, x_hi, i0, acc, lead);
+                            if (r0 < 3) tc::mma_bf16(d + r0 * CIN, a, z_hi, x_lo + ko, x_hi, i1, acc, lead);
+                        }
+                        acc = 1;
+                    }
+                    tc::commit_lead(zempty0 + 8u * zslot, lead);
+                    tc::commit_lead(empty0 + 8u * first, lead);
+                    if (++zslot == (uint32_t)kDzSlots) zslot = 0;
+                    if (u == n + 1) {  // the run's last two rows are read by no later step either
+                        tc::commit_lead(empty0 + 8u * (slot >= 1 ? slot - 1 : (uint32_t)kRowSlots - 1), lead);
+                        tc::commit_lead(empty0 + 8u * slot, lead);
+                    }
+                }
+                if (++slot == (uint32_t)kRowSlots) {
+                    slot = 0;
+                    sphase ^= 1u;
+                }
+            }
+            step += n;
         }
         // every MMA issued has finished before the accumulators are read
-        tc::commit(&pp.drain);
-        if (!tc::mbar_wait(&pp.drain, 0u, kConvWaitNs)) {
+        tc::commit_lead(tc::smem_u32(&pp.drain), lead);
+        __syncwarp();
+        if (!tc::mbar_wait(&pp.drain, 0u, kConvWaitNs) && lane == 0) {
             *abort = 1;
             atomicExch(A.err, 1);
         }
+        __syncwarp();
+    } else {
+        // ---- bias: thread t sums pixel t % KP of chunks t / KP, + 128 / KP, ... ----
+        constexpr int GR = 128 / KP, CT = CZ / GR;
+        const int t = tid - 32 * (kWgMmaWarp + 1), px = t % KP, c0 = t / KP;
+        float sum[CT][8];
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum[c][e] = 0.f;
+        uint32_t slot = 0, sphase = 0, zslot = 0;
+        bool ok = true;
+        for (int step = s0; step < s1 && ok;) {
+            const WgRun run = wg_run<KP>(A, step, s1);
+            const int n = run.y1 - run.y0;
+            for (int u = 0; u < n + 2; ++u) {
+                if (!(ok = pipe_wait(&pp.full[slot], sphase, abort, A.err))) break;
+                if (u >= 2) {
+                    const unsigned char *z = zring + zslot * zbytes + CZ * kPlane + px * 16;  // copy dx = 1
+#pragma unroll
+                    for (int c = 0; c < CT; ++c) {
+                        float f[8];
+                        unpack8(*reinterpret_cast<const uint4 *>(z + (c0 + GR * c) * kPlane), f);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) sum[c][e] += f[e];
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&pp.zempty[zslot]);
+                    if (++zslot == (uint32_t)kDzSlots) zslot = 0;
+                }
+                if (++slot == (uint32_t)kRowSlots) {
+                    slot = 0;
+                    sphase ^= 1u;
+                }
+            }
+            step += n;
+        }
+        // over the warp's 32 pixels (the warps of a chunk are added below)
+        const int wb = warp - kWgMmaWarp - 1;
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float v = sum[c][e];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) s_bias[wb][8 * (c0 + GR * c) + e] = v;
+            }
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (!*abort && warp < kWgProdWarps) {
-        // rows R = dx * mtiles * 128 + (dy * cin + ci), bias row R = 3 * mtiles * 128;
-        // warps w and w + 4 share TMEM lane quarter w % 4 and split the tiles
-        const int q = warp & 3;
-        const size_t rows_pad = (size_t)3 * L.mtiles * 128 + 1;
-        float *dst = A.partial + (size_t)blockIdx.x * rows_pad * cout;
-        const int ntile = 3 * L.mtiles + 1;
-        for (int tl = 0; tl < ntile; ++tl) {
-            if ((tl & 1) != (warp >> 2)) continue;
-            for (int j = 0; j < cout; j += 16) {
+    if (!*abort && warp > kWgMmaWarp) {
+        // D row m = (dx, co), column n = (dy, ci)
+        float *dst = A.partial + (size_t)blockIdx.x * wg_partial(CIN, COUT);
+        const int q = warp & 3;  // a warp reads the tensor-memory lanes of its number modulo 4
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            const int m = mt * 128 + q * 32 + lane;
+            for (int j = 0; j < N; j += 16) {
                 float v[16];
-                tc::tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(tl * cout + j), v);
-                if (nsteps == 0) {
+                tc::tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * N + j), v);
+                if (m >= 3 * COUT) continue;
+                float4 *o = reinterpret_cast<float4 *>(dst + (size_t)m * N + j);
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) v[e] = 0.f;
-                }
-                const int rr = q * 32 + lane;
-                if (tl < 3 * L.mtiles) {
-                    const size_t r = (size_t)tl * 128 + rr;
-                    float4 *o = reinterpret_cast<float4 *>(dst + r * cout + j);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) o[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-                } else if (rr == 0) {
-                    float4 *o = reinterpret_cast<float4 *>(dst + (rows_pad - 1) * cout + j);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) o[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-                }
+                for (int e = 0; e < 4; ++e)
+                    o[e] = s0 < s1 ? make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3])
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
             }
+        }
+        const int t = tid - 32 * (kWgMmaWarp + 1);
+        if (t < COUT) {  // chunk t / 8 was summed by KP / 32 warps
+            const int wb = ((t >> 3) % (128 / KP)) * (KP / 32);
+            float v = s_bias[wb][t];
+#pragma unroll
+            for (int k = 1; k < KP / 32; ++k) v += s_bias[wb + k][t];
+            dst[3 * COUT * N + t] = v;
         }
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == kWgProdWarps) tc::tmem_dealloc(tmem, ncols);
+    if (warp == kWgMmaWarp) tc::tmem_dealloc(tmem, tcols);
 }
 
-// The weight-gradient kernel for a source mode and the input chunks of
-// sources A and B (the convolutions' own variants).
-const void *wgrad_kernel_fn(int mode, int cca, int ccb) {
-#define TDE_WG_FN(M, A, B) \
-    if (mode == M && cca == A && ccb == B) return (const void *)wgrad_tc_kernel<M, A, B>;
-    TDE_CONV_VARIANTS(TDE_WG_FN)
+// The weight-gradient kernel for a source mode, the input chunks of sources A
+// and B and the output chunks: c2 .. c8, c10, c11, and c9 as two (its 112 input
+// channels' accumulators exceed the tensor memory).
+#define TDE_WG_VARIANTS(X) \
+    X(SRC_DIRECT, 2, 0, 2) X(SRC_DIRECT, 2, 0, 4) X(SRC_DIRECT, 4, 0, 4) X(SRC_DIRECT, 4, 0, 6) X(SRC_DIRECT, 6, 0, 6) \
+    X(SRC_DIRECT, 6, 0, 8) X(SRC_DIRECT, 8, 0, 8) X(SRC_UP, 8, 0, 6) X(SRC_UP, 6, 4, 4) X(SRC_UP, 4, 2, 2)
+const void *wgrad_kernel_fn(int mode, int cca, int ccb, int cz) {
+#define TDE_WG_FN(M, A, B, Z) \
+    if (mode == M && cca == A && ccb == B && cz == Z) return (const void *)wgrad_tc_kernel<M, A, B, Z>;
+    TDE_WG_VARIANTS(TDE_WG_FN)
 #undef TDE_WG_FN
     return nullptr;
 }
@@ -1029,25 +1145,22 @@ __device__ __forceinline__ bool sum_partials(const float *__restrict__ partial, 
     return true;
 }
 
-// Weight gradients from the per-block partials [blocks][rows_pad][cout]: row
-// r = dx * mtiles * 128 + dy * cin + ci (rows past 3 cin of a dx are padding),
-// the last row the bias; dw[(co * 9 + 3 dy + dx) * cin + ci].
+// Weight gradients from the per-block partials [blocks][(dx, co)][(dy, ci)] and
+// their bias; this part's cin channels lie at ci0 of the layer's cin_all:
+// dw[(co * 9 + 3 dy + dx) * cin_all + ci0 + ci].
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restrict__ partial, int blocks, int cin,
-                                                           int cout, int mtiles, float *__restrict__ dw,
+                                                           int cin_all, int ci0, int cout, float *__restrict__ dw,
                                                            float *__restrict__ db) {
-    const int rows_pad = 3 * mtiles * 128 + 1;
     int e;
     float t;
-    if (!sum_partials(partial, blocks, rows_pad * cout, e, t)) return;
-    const int r = e / cout, co = e % cout;
-    if (r == rows_pad - 1) {
-        db[co] = t;
+    if (!sum_partials(partial, blocks, wg_partial(cin, cout), e, t)) return;
+    const int m = e / (3 * cin), n = e - m * (3 * cin);
+    if (m >= 3 * cout) {  // (the bias is shorter than a row of D)
+        if (db) db[n] = t;
         return;
     }
-    const int dx = r / (mtiles * 128), rem = r % (mtiles * 128);
-    if (rem >= 3 * cin) return;
-    const int dy = rem / cin, ci = rem % cin;
-    dw[((size_t)co * 9 + 3 * dy + dx) * cin + ci] = t;
+    const int dx = m / cout, co = m - dx * cout, dy = n / cin, ci = n - dy * cin;
+    dw[((size_t)co * 9 + 3 * dy + dx) * cin_all + ci0 + ci] = t;
 }
 
 // ---------------------------------------------------------------------------
@@ -1349,10 +1462,12 @@ int prepare_kernels() {
     // launches (also inside stream capture) make no other runtime call
     std::vector<const void *> fns;
 #define TDE_CONV_FN(M, A, B) \
-    fns.push_back(conv_kernel_fn(M, A, B, false)); \
-    fns.push_back((const void *)wgrad_tc_kernel<M, A, B>);
+    fns.push_back(conv_kernel_fn(M, A, B, false));
     TDE_CONV_VARIANTS(TDE_CONV_FN)
 #undef TDE_CONV_FN
+#define TDE_WG_FN(M, A, B, Z) fns.push_back((const void *)wgrad_tc_kernel<M, A, B, Z>);
+    TDE_WG_VARIANTS(TDE_WG_FN)
+#undef TDE_WG_FN
     for (int cca = 2; cca <= 6; cca += 2) fns.push_back(conv_kernel_fn(SRC_DIRECT, cca, 0, true));
     for (const void *fn : fns) {
         cudaFuncAttributes fa;
@@ -1463,37 +1578,29 @@ int launch_conv(const ConvArgs &a, const ConvPlan &plan, int num_sms, cudaStream
     return check_launch("refiner conv");
 }
 
-int wgrad_blocks(int num_sms, int cin, int cout) {
-    (void)cin;
-    (void)cout;
-    return num_sms;
-}
+// One block per SM.  Two blocks of 64-pixel steps took as long (912 against
+// 940 us for all layers at batch 16 of 640x480) with half as many additions into
+// each accumulator; the sums then differ by 3e-5 of a gradient's norm from those
+// of one block, which differ by 3e-6 from the per-tap form's.
+int wgrad_blocks(int num_sms) { return num_sms; }
 
-size_t wgrad_partial_floats(int blocks, int cin, int cout) {
-    const WgLayout L = wg_layout(cin, cout);
-    return (size_t)blocks * ((size_t)3 * L.mtiles * 128 + 1) * cout;
-}
+size_t wgrad_partial_floats(int blocks, int cin, int cout) { return (size_t)blocks * wg_partial(cin, cout); }
 
 int launch_wgrad(const WgradArgs &a, int blocks, cudaStream_t s) {
     const int cin = a.ca + a.cb;
-    const WgLayout L = wg_layout(cin, a.cout);
-    if (cin % 8 || a.cout % 16 || a.cout < 16 || L.tcols > 512 || a.mode_a == SRC_POOL)
-        return set_error(TDE_ERR_INVALID_ARG, "refiner wgrad: unsupported shape cin=%d cout=%d", cin, a.cout);
-    // as many ring stages as one block per SM holds (the ones tile after them)
-    const size_t stage = (size_t)L.x_bytes + L.z_bytes, ones = 16u * 256u;
-    const size_t budget = 227 * 1024 - 512 - ones;
-    int S = (int)(budget / stage);
-    S = S > kWgMaxStages ? kWgMaxStages : S;
-    if (S < 2) return set_error(TDE_ERR_UNSUPPORTED, "refiner wgrad: cin=%d cout=%d does not fit an SM", cin, a.cout);
-    size_t smem = (size_t)S * stage + ones;
-    const size_t fl = smem_floor_for_tmem(tmem_cols((int)L.tcols));
-    if (smem < fl) smem = fl;
-    const void *fn = wgrad_kernel_fn(a.mode_a, a.ca / 8, a.cb / 8);
-    if (!fn) return set_error(TDE_ERR_UNSUPPORTED, "refiner wgrad: no kernel for mode %d with %d + %d input channels",
-                              a.mode_a, a.ca, a.cb);
+    const void *fn = wgrad_kernel_fn(a.mode_a, a.ca / 8, a.cb / 8, a.cout / 8);
+    if (!fn) return set_error(TDE_ERR_UNSUPPORTED, "refiner wgrad: no kernel for mode %d with %d + %d input, %d output channels",
+                              a.mode_a, a.ca, a.cb, a.cout);
+    const int kp = wg_kp(cin / 8, a.cout / 8);
+    if ((long)a.n * a.h * ((a.w + kp - 1) / kp) > 0x7fffffffL)
+        return set_error(TDE_ERR_UNSUPPORTED, "refiner wgrad: %d images of %dx%d are too many", a.n, a.w, a.h);
     WgradArgs args = a;
-    void *kargs[] = {(void *)&args, (void *)&S};
-    cudaError_t e = cudaLaunchKernel(fn, dim3(blocks), dim3(kWgThreadsP), kargs, smem, s);
+    void *kargs[] = {(void *)&args};
+    // never more blocks than fit in tensor memory: pad the shared memory
+    size_t smem = wg_smem(cin / 8, a.cout / 8, kp, wg_flight(cin / 8, a.cout / 8));
+    const size_t fl = smem_floor_for_tmem(tmem_cols(wg_mtiles(a.cout) * 3 * cin));
+    if (smem < fl) smem = fl;
+    cudaError_t e = cudaLaunchKernel(fn, dim3(blocks), dim3(kWgThreads), kargs, smem, s);
     if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "refiner wgrad: %s", cudaGetErrorString(e));
     return check_launch("refiner wgrad");
 }
@@ -1503,10 +1610,9 @@ int launch_wait_selftest(uint64_t limit_ns, unsigned long long *out, cudaStream_
     return check_launch("wait selftest");
 }
 
-int launch_wgrad_reduce(const float *partial, int blocks, int cin, int cout, float *dw, float *db, cudaStream_t s) {
-    const WgLayout L = wg_layout(cin, cout);
-    const int n = (3 * L.mtiles * 128 + 1) * cout;
-    wgrad_reduce_kernel<<<div_up(n, 32), 256, 0, s>>>(partial, blocks, cin, cout, L.mtiles, dw, db);
+int launch_wgrad_reduce(const float *partial, int blocks, int cin, int cin_all, int ci0, int cout, float *dw, float *db,
+                        cudaStream_t s) {
+    wgrad_reduce_kernel<<<div_up(wg_partial(cin, cout), 32), 256, 0, s>>>(partial, blocks, cin, cin_all, ci0, cout, dw, db);
     return check_launch("refiner wgrad reduce");
 }
 

@@ -121,7 +121,6 @@ struct tde_refiner {
     bf16 *pooled[kPools] = {};  // 2x2 max pools of e0, e1, e2 (levels 1, 2, 3)
     bf16 *gr[GRAD_COUNT] = {};
     float *wpartial = nullptr;
-    int wg_blocks = 0;
     ConvPlan fwd_plan[kConvs] = {}, bwd_plan[kConvs] = {};  // launch geometry per convolution
     float *in_partial = nullptr;
     float *loss_partial = nullptr;
@@ -142,6 +141,10 @@ template <class T> int dalloc(tde_refiner *r, T **p, size_t count) {
     *p = static_cast<T *>(q);
     return TDE_OK;
 }
+
+// Launches of one layer's weight gradient: 3 cin columns of at most two row
+// tiles fit the 512 columns of tensor memory, or each source takes one.
+int wgrad_parts(int cin, int cout) { return (3 * cout + 127) / 128 * 3 * cin <= 512 && 3 * cin <= 256 ? 1 : 2; }
 
 size_t pixels(const tde_refiner *r, int batch, int level) {
     return (size_t)batch * (r->rows >> level) * (r->cols >> level);
@@ -203,8 +206,20 @@ int loss_grad(tde_refiner *r, const uint16_t *raw, const uint16_t *target, int n
         wa.dz = r->gr[k.dz]; wa.cout = c.cout;
         wa.n = n; wa.h = h; wa.w = w;
         wa.partial = r->wpartial; wa.err = r->err;
-        TDE_TRY(launch_wgrad(wa, r->wg_blocks, s));
-        TDE_TRY(launch_wgrad_reduce(r->wpartial, r->wg_blocks, cin, c.cout, r->grad + kL.w[i], r->grad + kL.b[i], s));
+        // c9's two sources one after the other: together their accumulators
+        // exceed the tensor memory
+        const int parts = wgrad_parts(cin, c.cout);
+        for (int k2 = 0; k2 < parts; ++k2) {
+            WgradArgs wp = wa;
+            if (parts == 2) {
+                if (k2 == 1) { wp.a = wa.b; wp.ca = wa.cb; wp.mode_a = SRC_DIRECT; }
+                wp.b = nullptr; wp.cb = 0;
+            }
+            const int ci = wp.ca + wp.cb, blocks = wgrad_blocks(r->num_sms);
+            TDE_TRY(launch_wgrad(wp, blocks, s));
+            TDE_TRY(launch_wgrad_reduce(r->wpartial, blocks, ci, cin, k2 ? c.ca : 0, c.cout, r->grad + kL.w[i],
+                                        k2 ? nullptr : r->grad + kL.b[i], s));
+        }
         // input gradient: the same convolution on dz with the flipped, transposed weights
         ConvArgs a;
         std::memset(&a, 0, sizeof(a));
@@ -245,7 +260,6 @@ int tde_refiner_create(int max_batch, int rows, int cols, uint64_t seed, tde_ref
         delete r;
         return set_error(TDE_ERR_CUDA, "refiner_create: no CUDA device");
     }
-    r->wg_blocks = wgrad_blocks(r->num_sms, 0, 0);
     st = prepare_kernels();
     for (int i = 0; i < kConvs && !st; ++i) {
         const int cin = kConv[i].ca + kConv[i].cb;
@@ -259,8 +273,12 @@ int tde_refiner_create(int max_batch, int rows, int cols, uint64_t seed, tde_ref
     }
     size_t wpart = 0;
     for (int i = 0; i < kConvs; ++i) {
-        const size_t f = wgrad_partial_floats(r->wg_blocks, kConv[i].ca + kConv[i].cb, kConv[i].cout);
-        if (f > wpart) wpart = f;
+        const int cin = kConv[i].ca + kConv[i].cb, parts = wgrad_parts(cin, kConv[i].cout);
+        for (int k2 = 0; k2 < parts; ++k2) {
+            const int ci = parts == 1 ? cin : k2 ? kConv[i].cb : kConv[i].ca;
+            const size_t f = wgrad_partial_floats(wgrad_blocks(r->num_sms), ci, kConv[i].cout);
+            if (f > wpart) wpart = f;
+        }
     }
     const size_t P = kL.total;
     do {

@@ -41,9 +41,9 @@ struct ConvArgs {
     bf16 *pool_out;
 };
 
-// Weight gradient of the same convolution: partial[blk][r][co] with rows
-// r = t * cin + ci (r = 9 * cin: bias), summed over the pixels block blk
-// visits; reduced by launch_wgrad_reduce.
+// Weight gradient of the same convolution, or of its channels from one source
+// alone (a null b): per block partial sums over the pixels it visits, reduced by
+// launch_wgrad_reduce.
 struct WgradArgs {
     const bf16 *a;
     int ca, mode_a;
@@ -74,11 +74,13 @@ int conv_plan(int mode, int ca, int cin, int cout, bool pool, ConvPlan *out);
 int launch_wait_selftest(uint64_t limit_ns, unsigned long long *out, cudaStream_t s);
 // Launches only (no other runtime call), so it may be stream-captured.
 int launch_conv(const ConvArgs &a, const ConvPlan &plan, int num_sms, cudaStream_t s);
-int wgrad_blocks(int num_sms, int cin, int cout);
+int wgrad_blocks(int num_sms);
 size_t wgrad_partial_floats(int blocks, int cin, int cout);
 int launch_wgrad(const WgradArgs &a, int blocks, cudaStream_t s);
-// dw[co][t][ci] and db[co] from the partials of `blocks` blocks
-int launch_wgrad_reduce(const float *partial, int blocks, int cin, int cout, float *dw, float *db, cudaStream_t s);
+// dw[co][t][ci0 + ci] (of cin_all input channels) and, unless null, db[co] from
+// the partials of `blocks` blocks
+int launch_wgrad_reduce(const float *partial, int blocks, int cin, int cin_all, int ci0, int cout, float *dw, float *db,
+                        cudaStream_t s);
 
 // Input preparation and the first convolution (3 features per tap -> 16
 // channels, FP32 on the CUDA cores): depth_m = raw * 0.001 (0 when raw == 0),

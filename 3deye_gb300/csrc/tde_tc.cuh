@@ -40,17 +40,8 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
            (static_cast<uint32_t>(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-
-// The same with the descriptors as 32-bit halves (an offset only moves the low
-// one) and the accumulation fixed, executed by the lane with `lead` set: for
+// D[tmem] (+)= A[smem] * B[smem]^T, executed by the lane with `lead` set; the
+// descriptors as 32-bit halves (an offset only moves the low one): for
 // loops that a whole warp runs with the same values.  Without a branch around
 // the issuing lane those values stay in uniform registers, which is where the
 // instruction takes its operands from.
@@ -65,6 +56,18 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_
         "setp.ne.b32 q, %7, 0;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
         ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC ? 1 : 0), "r"(lead));
+}
+// With the accumulation as an argument.
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                         uint32_t idesc, uint32_t accumulate, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %2};\n\t"
+        "mov.b64 b, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead));
 }
 // commit() by the lane with `lead` set; mbar: shared-memory address.
 __device__ __forceinline__ void commit_lead(uint32_t mbar, uint32_t lead) {
