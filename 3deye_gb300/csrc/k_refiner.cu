@@ -1171,96 +1171,205 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restri
 // invalid).  Differences in centimetres keep millimetre noise representable
 // once the first layer's output is stored as bf16.
 constexpr int kInCh = 3, kInK = 9 * kInCh;
-__device__ __forceinline__ void input_features(const float (&d)[9], float (&in)[kInK]) {
-    const float dc = d[4];
-#pragma unroll
-    for (int t = 0; t < 9; ++t) {
-        const bool vt = d[t] > 0.f;
-        in[3 * t] = (vt && dc > 0.f) ? (d[t] - dc) * 100.f : 0.f;
-        in[3 * t + 1] = vt ? 1.f : 0.f;
-        in[3 * t + 2] = d[t];
-    }
+// Two FP32 values in one 64-bit register and their fused multiply-adds (each
+// rounded as fmaf): half the instructions of the two scalar ones.
+__device__ __forceinline__ uint64_t f2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unf2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-__global__ void __launch_bounds__(256) conv_in_kernel(const uint16_t *__restrict__ raw, float *__restrict__ depth_m,
+// The three features of one tap, for the pixel with depth dc.
+__device__ __forceinline__ void tap_features(float d, float dc, float (&f)[kInCh]) {
+    const bool v = d > 0.f;
+    f[0] = (v && dc > 0.f) ? (d - dc) * 100.f : 0.f;
+    f[1] = v ? 1.f : 0.f;
+    f[2] = d;
+}
+
+// A thread makes kInRows pixels of one column, so that a weight read from shared
+// memory serves four fused multiply-adds (one pixel a thread waited for those
+// reads: 193 us at batch 16 of 640x480, 115 us now; the arithmetic alone is
+// 57 us).  Each output channel's sum runs over the features in order.
+constexpr int kInRows = 4;
+__global__ void __launch_bounds__(128) conv_in_kernel(const uint16_t *__restrict__ raw, float *__restrict__ depth_m,
                                                       const float *__restrict__ w1, const float *__restrict__ b1,
                                                       bf16 *__restrict__ e0a, int n, int h, int w) {
-    __shared__ float sw[16 * kInK + 16];
-    for (int i = threadIdx.x; i < 16 * kInK; i += blockDim.x) sw[i] = w1[i];
-    if (threadIdx.x < 16) sw[16 * kInK + threadIdx.x] = b1[threadIdx.x];
+    __shared__ __align__(16) float sw[kInK + 1][16];  // by feature, then the bias
+    for (int i = threadIdx.x; i < 16 * kInK; i += blockDim.x) sw[i % kInK][i / kInK] = w1[i];
+    if (threadIdx.x < 16) sw[kInK][threadIdx.x] = b1[threadIdx.x];
     __syncthreads();
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= (size_t)n * h * w) return;
-    const int x = (int)(p % w), y = (int)((p / w) % h), img = (int)(p / ((size_t)w * h));
-    float d[9];
+    // rows are multiples of kInRows; lanes run over w, a multiple of 8
+    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned x = p % (unsigned)w, strip = p / (unsigned)w, strips = (unsigned)h / kInRows;
+    const bool live = strip < (unsigned)n * strips;
+    const int img = live ? (int)(strip / strips) : 0, y0 = live ? (int)(strip % strips) * kInRows : 0;
+    float d[kInRows + 2][3];
+#pragma unroll
+    for (int r = 0; r < kInRows + 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int yy = y0 + r - 1, xx = (int)x + c - 1;
+            d[r][c] = 0.f;
+            if (yy >= 0 && yy < h && xx >= 0 && xx < w) d[r][c] = (float)__ldg(raw + ((size_t)img * h + yy) * w + xx) * 0.001f;
+        }
+    uint64_t o2[kInRows][8];  // channel pairs
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int r = 0; r < kInRows; ++r) o2[r][c] = f2(sw[kInK][2 * c], sw[kInK][2 * c + 1]);
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
-        const int yy = y + t / 3 - 1, xx = x + t % 3 - 1;
-        d[t] = 0.f;
-        if (yy >= 0 && yy < h && xx >= 0 && xx < w) d[t] = (float)raw[((size_t)img * h + yy) * w + xx] * 0.001f;
-    }
-    float in[kInK];
-    input_features(d, in);
-    depth_m[p] = d[4];
-    float o[16];
+        float f[kInRows][kInCh];
 #pragma unroll
-    for (int co = 0; co < 16; ++co) {
-        float s = sw[16 * kInK + co];
+        for (int r = 0; r < kInRows; ++r) tap_features(d[r + t / 3][t % 3], d[r + 1][1], f[r]);
 #pragma unroll
-        for (int k = 0; k < kInK; ++k) s = fmaf(sw[co * kInK + k], in[k], s);
-        o[co] = s > 0.f ? s : 0.f;
+        for (int k = 0; k < kInCh; ++k) {
+            uint64_t ff[kInRows];
+#pragma unroll
+            for (int r = 0; r < kInRows; ++r) ff[r] = f2(f[r][k], f[r][k]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 wv = *reinterpret_cast<const float4 *>(&sw[kInCh * t + k][4 * q]);
+                const uint64_t wa = f2(wv.x, wv.y), wb = f2(wv.z, wv.w);
+#pragma unroll
+                for (int r = 0; r < kInRows; ++r) {
+                    o2[r][2 * q] = fma2(wa, ff[r], o2[r][2 * q]);
+                    o2[r][2 * q + 1] = fma2(wb, ff[r], o2[r][2 * q + 1]);
+                }
+            }
+        }
     }
-    uint4 *dst = reinterpret_cast<uint4 *>(e0a + p * 16);
-    dst[0] = pack8(o);
-    dst[1] = pack8(o + 8);
+    // Stores in whole sectors: an even lane and the odd one after it (the next
+    // pixel of the row: w is even) swap halves, so that a store's neighbouring
+    // lanes write the two halves of one pixel.
+    const bool odd = threadIdx.x & 1;
+#pragma unroll
+    for (int r = 0; r < kInRows; ++r) {
+        float o[16];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float2 v = unf2(o2[r][c]);
+            o[2 * c] = v.x > 0.f ? v.x : 0.f;
+            o[2 * c + 1] = v.y > 0.f ? v.y : 0.f;
+        }
+        const size_t pix = ((size_t)img * h + y0 + r) * w + x;
+        const uint4 q0 = pack8(o), q1 = pack8(o + 8);
+        const uint4 give = odd ? q0 : q1, got = shfl_xor4(give, 1);
+        if (live) {
+            depth_m[pix] = d[r + 1][1];
+            uint4 *dst = reinterpret_cast<uint4 *>(e0a + (pix - odd) * 16);  // the even pixel
+            dst[odd] = odd ? got : q0;
+            dst[2 + odd] = odd ? q1 : got;
+        }
+    }
 }
 
-// Block = 16 output channels x 16 pixel lanes; each block covers whole image
-// rows and writes 16 x 28 partial sums (27 weights + bias per channel).
-constexpr int kInRowsPerBlock = 4;
+// Gradient of the first convolution: C[16 channels][28 features] += G F over the
+// pixels (the 28th feature is 1: the bias).  A block stages 64 pixels of a row at
+// a time as feature and gradient rows in shared memory; thread (kg, cq, fq) takes
+// the pixels 4 kg .. 4 kg + 3, the channels cq + 4 i and the features 7 fq + j: 11
+// 16-byte reads for 112 multiply-adds.  (One channel a thread, each forming the
+// pixel's features again: 413 us at batch 16 of 640x480; 212 us now.)
+// Row strides of 72 words put a warp's eight distinct reads into different banks.
 constexpr int kInPartial = 16 * (kInK + 1);
-__global__ void __launch_bounds__(256) conv_in_wgrad_kernel(const float *__restrict__ depth_m,
+constexpr int kInTile = 64, kInStride = 72, kInMaxBlocks = 608;  // four blocks for each of 152 SMs
+__global__ void __launch_bounds__(256, 4) conv_in_wgrad_kernel(const float *__restrict__ depth_m,
                                                             const bf16 *__restrict__ dz1, int n, int h, int w,
                                                             float *__restrict__ partial) {
-    extern __shared__ float rows3[];  // depth rows y-1, y, y+1 with a zero column either side: 3 x (w + 2)
-    __shared__ float red[16][16][kInK + 1];
-    const int co = threadIdx.x & 15, pl = threadIdx.x >> 4;
-    const int W2 = w + 2;
-    float s[kInK + 1];
+    __shared__ __align__(16) float F[kInK + 1][kInStride], G[16][kInStride];
+    __shared__ float red[8][kInPartial];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int kg = tid >> 4, cq = (tid >> 2) & 3, fq = tid & 3;
+    float s[4][7];
 #pragma unroll
-    for (int k = 0; k <= kInK; ++k) s[k] = 0.f;
-    const int row0 = blockIdx.x * kInRowsPerBlock;
-    for (int rr = 0; rr < kInRowsPerBlock; ++rr) {
-        const int rowi = row0 + rr;
-        if (rowi >= n * h) break;
-        const int y = rowi % h, img = rowi / h;
-        __syncthreads();
-        for (int i = threadIdx.x; i < 3 * W2; i += blockDim.x) {
-            const int r = i / W2, x = i % W2 - 1, yy = y + r - 1;
-            rows3[i] = (x >= 0 && x < w && yy >= 0 && yy < h) ? depth_m[((size_t)img * h + yy) * w + x] : 0.f;
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 7; ++j) s[i][j] = 0.f;
+    if (tid < kInTile) F[kInK][tid] = 1.f;
+    const int tiles_x = (w + kInTile - 1) / kInTile;
+    const long tiles = (long)n * h * tiles_x;
+    const int px = tid & 63, part = tid >> 6;
+    // taps 3 part .. 3 part + 2 (one kernel row) by the first 192 threads, the
+    // gradients by the last 64; a tile is fetched while the one before is summed
+    float d[3], dc = 0.f;
+    uint4 gv[2];
+    auto fetch = [&](long tile) {
+        const long rowi = tile / tiles_x;
+        const int y = (int)(rowi % h), x = (int)(tile - rowi * tiles_x) * kInTile + px;
+        const bool in = tile < tiles && x < w;
+        if (part < 3) {
+            const float *row = depth_m + rowi * w;
+            const int yy = y + part - 1;
+            dc = in ? __ldg(row + x) : 0.f;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int xx = x + c - 1;
+                d[c] = in && yy >= 0 && yy < h && xx >= 0 && xx < w ? __ldg(row + (part - 1) * w + xx) : 0.f;
+            }
+        } else {
+            gv[0] = in ? ldg16(dz1 + (rowi * w + x) * 16) : make_uint4(0u, 0u, 0u, 0u);
+            gv[1] = in ? ldg16(dz1 + (rowi * w + x) * 16 + 8) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    fetch(blockIdx.x);
+    for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        __syncthreads();  // the previous tile has been read
+        if (part < 3) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                float f[kInCh];
+                tap_features(d[c], dc, f);
+#pragma unroll
+                for (int k = 0; k < kInCh; ++k) F[kInCh * (3 * part + c) + k][px] = f[k];
+            }
+        } else {
+            float f[16];
+            unpack8(gv[0], f);
+            unpack8(gv[1], f + 8);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) G[c][px] = f[c];
         }
         __syncthreads();
-        for (int x = pl; x < w; x += 16) {
-            const size_t p = ((size_t)img * h + y) * w + x;
-            const float g = __bfloat162float(dz1[p * 16 + co]);
-            if (g == 0.f) continue;
-            float d[9];
+        fetch(tile + gridDim.x);
+        float4 g[4];
 #pragma unroll
-            for (int t = 0; t < 9; ++t) d[t] = rows3[(t / 3) * W2 + x + t % 3];
-            float in[kInK];
-            input_features(d, in);
+        for (int i = 0; i < 4; ++i) g[i] = *reinterpret_cast<const float4 *>(&G[cq + 4 * i][4 * kg]);
 #pragma unroll
-            for (int k = 0; k < kInK; ++k) s[k] = fmaf(g, in[k], s[k]);
-            s[kInK] += g;
+        for (int j = 0; j < 7; ++j) {
+            const float4 f = *reinterpret_cast<const float4 *>(&F[7 * fq + j][4 * kg]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s[i][j] = fmaf(g[i].x, f.x, s[i][j]);
+                s[i][j] = fmaf(g[i].y, f.y, s[i][j]);
+                s[i][j] = fmaf(g[i].z, f.z, s[i][j]);
+                s[i][j] = fmaf(g[i].w, f.w, s[i][j]);
+            }
         }
     }
+    // the warp's two pixel groups, then the warps in order
 #pragma unroll
-    for (int k = 0; k <= kInK; ++k) red[pl][co][k] = s[k];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            const float v = s[i][j] + __shfl_xor_sync(0xffffffffu, s[i][j], 16);
+            if (lane < 16) red[warp][(cq + 4 * i) * (kInK + 1) + 7 * fq + j] = v;
+        }
     __syncthreads();
-    for (int i = threadIdx.x; i < kInPartial; i += blockDim.x) {
-        const int c = i / (kInK + 1), k = i % (kInK + 1);
-        float t = 0.f;
-        for (int l = 0; l < 16; ++l) t += red[l][c][k];
+    for (int i = tid; i < kInPartial; i += blockDim.x) {
+        float t = red[0][i];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) t += red[k][i];
         partial[(size_t)blockIdx.x * kInPartial + i] = t;
     }
 }
@@ -1618,19 +1727,21 @@ int launch_wgrad_reduce(const float *partial, int blocks, int cin, int cin_all, 
 
 int launch_conv_in(const uint16_t *raw, float *depth_m, const float *w1, const float *b1, bf16 *e0a, int n, int h,
                    int w, cudaStream_t s) {
-    const size_t np = (size_t)n * h * w;
-    conv_in_kernel<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(raw, depth_m, w1, b1, e0a, n, h, w);
+    if (h % kInRows || w % 2) return set_error(TDE_ERR_INVALID_ARG, "refiner conv_in: %dx%d", w, h);
+    const size_t items = (size_t)n * (h / kInRows) * w;
+    if (items > 0x7fffff00u) return set_error(TDE_ERR_UNSUPPORTED, "refiner conv_in: %d images of %dx%d are too many", n, w, h);
+    conv_in_kernel<<<(unsigned)((items + 127) / 128), 128, 0, s>>>(raw, depth_m, w1, b1, e0a, n, h, w);
     return check_launch("refiner conv_in");
 }
 
-int conv_in_wgrad_blocks(int n, int h) { return div_up(n * h, kInRowsPerBlock); }
+int conv_in_wgrad_blocks(int n, int h, int w) {
+    const size_t tiles = (size_t)n * h * ((w + kInTile - 1) / kInTile);
+    return (int)(tiles < (size_t)kInMaxBlocks ? tiles : (size_t)kInMaxBlocks);
+}
 
 int launch_conv_in_wgrad(const float *depth_m, const bf16 *dz1, int n, int h, int w, float *partial, int blocks,
                          float *dw1, float *db1, cudaStream_t s) {
-    const size_t rows_bytes = (size_t)3 * (w + 2) * sizeof(float);
-    if (rows_bytes + sizeof(float) * 16 * 16 * (kInK + 1) > 48 * 1024)
-        return set_error(TDE_ERR_UNSUPPORTED, "refiner: %d columns exceed the input-layer gradient kernel", w);
-    conv_in_wgrad_kernel<<<blocks, 256, rows_bytes, s>>>(depth_m, dz1, n, h, w, partial);
+    conv_in_wgrad_kernel<<<blocks, 256, 0, s>>>(depth_m, dz1, n, h, w, partial);
     TDE_TRY(check_launch("refiner conv_in wgrad"));
     conv_in_wgrad_reduce_kernel<<<div_up(kInPartial, 32), 256, 0, s>>>(partial, blocks, dw1, db1);
     return check_launch("refiner conv_in wgrad reduce");
