@@ -182,25 +182,17 @@ int tde_estimate_combined(const float *vmap_cur, const float *nmap_cur, const fl
     uintptr_t sp = reinterpret_cast<uintptr_t>(gbuf + part);
     sp = (sp + 255) & ~uintptr_t(255);
     IcpState *st = reinterpret_cast<IcpState *>(sp);
-    IcpState h;
-    std::memset(&h, 0, sizeof(h));
+    IcpPose pose;
     const float *Rc = &R_cur->row[0].x, *Rp = &R_prev_inv->row[0].x;
-    for (int k = 0; k < 9; ++k) { h.pose.R_cur[k] = Rc[k]; h.pose.R_prev_inv[k] = Rp[k]; h.R[k] = Rc[k]; }
-    h.pose.t_cur[0] = t_cur->x; h.pose.t_cur[1] = t_cur->y; h.pose.t_cur[2] = t_cur->z;
-    h.pose.t_prev[0] = t_prev->x; h.pose.t_prev[1] = t_prev->y; h.pose.t_prev[2] = t_prev->z;
-    cudaError_t e = cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "estimate_combined: %s", cudaGetErrorString(e));
+    for (int k = 0; k < 9; ++k) { pose.R_cur[k] = Rc[k]; pose.R_prev_inv[k] = Rp[k]; }
+    pose.t_cur[0] = t_cur->x; pose.t_cur[1] = t_cur->y; pose.t_cur[2] = t_cur->z;
+    pose.t_prev[0] = t_prev->x; pose.t_prev[1] = t_prev->y; pose.t_prev[2] = t_prev->z;
     IcpArgs a;
     a.vcur = vmap_cur; a.ncur = nmap_cur; a.vprev = vmap_prev_g; a.nprev = nmap_prev_g;
     a.W = intr->cols; a.H = intr->rows;
     a.fx = intr->fx; a.fy = intr->fy; a.cx = intr->cx; a.cy = intr->cy;
     icp_set_thresholds(a, dist_thresh, angle_thresh);
-    int st_code = launch_icp(a, st, mbuf, s);
-    if (st_code) return st_code;
-    // the host copy of h must outlive the async copy above
-    e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "estimate_combined: %s", cudaGetErrorString(e));
-    return TDE_OK;
+    return launch_icp(a, pose, st, mbuf, s);
 }
 
 int tde_transform_estimation(const float *gbuf, float *out, int buf_length, int group_stride, void *stream) {

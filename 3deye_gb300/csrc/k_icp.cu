@@ -259,34 +259,36 @@ __device__ __forceinline__ void load_current(const IcpArgs &a, float3 (&nc)[PIX]
     }
 }
 
-// One-shot sums for the pose in st->pose (the Estimate_Combined drop-in):
-// the last block writes the exact totals to st->sums / mbuf and resets the
-// accumulators.
-__global__ void __launch_bounds__(kThreads) icp_sums_kernel(const IcpArgs a, IcpState *__restrict__ st,
-                                                            float *__restrict__ mbuf) {
-    __shared__ IcpPose P;
+// One-shot sums (the Estimate_Combined drop-in) for a pose given by value: the
+// caller's scratch needs no upload and the call no wait (a 6 KB state copied from
+// pageable memory and the stream synchronised after it made the call 26 us at
+// 640x480, of which the kernel was 9).  The accumulators of the scratch start
+// undefined: clear_sums_kernel zeroes them while this grid, launched with
+// programmatic serialisation, loads its maps.  The last block writes the exact
+// totals to st->sums / mbuf.
+__global__ void clear_sums_kernel(IcpState *__restrict__ st) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    unsigned long long *z = &st->acc[0][0][0][0];
+    for (int i = threadIdx.x; i < kIcpAccCopies * kIcpTerms * 3; i += blockDim.x) z[i] = 0ull;
+    if (threadIdx.x == 0) st->counter = 0u;
+}
+__global__ void __launch_bounds__(kThreads) icp_sums_kernel(const IcpArgs a, const __grid_constant__ IcpPose P,
+                                                            IcpState *__restrict__ st, float *__restrict__ mbuf) {
     __shared__ float red[kThreads / 32][32];
     __shared__ unsigned ticket;
     const int tid = threadIdx.x;
     float3 nc[kPixPerThread], vc[kPixPerThread];
     load_current<kPixPerThread, kThreads>(a, nc, vc);
-    if (tid < (int)(sizeof(IcpPose) / sizeof(float)))
-        reinterpret_cast<float *>(&P)[tid] = reinterpret_cast<const float *>(&st->pose)[tid];
-    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     accumulate_block<kPixPerThread, kThreads>(a, P, nc, vc, red, &st->acc[0]);
     if (!last_block(st, &ticket)) return;
     if (tid < kIcpTerms) {
         long long whole;
         const double d = read_total(&st->acc[0], tid, &whole);
-        #pragma unroll
-        for (int c = 0; c < kIcpAccCopies; ++c)
-            #pragma unroll
-            for (int l = 0; l < 3; ++l) st->acc[0][c][tid][l] = 0ull;
         st->sums[tid] = d;
         if (tid < 27) mbuf[tid] = (float)d;
         if (tid == 27) st->inliers = (int)whole;
     }
-    if (tid == 0) st->counter = 0u;
 }
 
 // Pipeline form, launch `iter` of the frame (see the file comment).
@@ -487,9 +489,20 @@ size_t icp_gbuf_floats(int W, int H) {
     return 64;
 }
 
-int launch_icp(const IcpArgs &a, IcpState *st, float *mbuf, cudaStream_t stream) {
-    const unsigned nb = div_up((unsigned)(a.W * a.H), (unsigned)(kThreads * kPixPerThread));
-    icp_sums_kernel<<<nb, kThreads, 0, stream>>>(a, st, mbuf);
+int launch_icp(const IcpArgs &a, const IcpPose &pose, IcpState *st, float *mbuf, cudaStream_t stream) {
+    clear_sums_kernel<<<1, kThreads, 0, stream>>>(st);
+    TDE_TRY(check_launch("estimate_combined"));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(div_up((unsigned)(a.W * a.H), (unsigned)(kThreads * kPixPerThread)));
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, icp_sums_kernel, a, pose, st, mbuf);
+    if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "estimate_combined: %s", cudaGetErrorString(e));
     return check_launch("estimate_combined");
 }
 

@@ -94,9 +94,9 @@ __host__ __device__ inline void so3_exp(const double *x, double *R) {
 
 size_t icp_gbuf_floats(int W, int H);
 
-// One-shot form: the 27 sums (and the inlier count) for the pose in
-// st->pose, exact totals to mbuf[0..26]; no solve.
-int launch_icp(const IcpArgs &a, IcpState *st, float *mbuf, cudaStream_t stream);
+// One-shot form: the 27 sums (and the inlier count) for `pose`, exact totals to
+// mbuf[0..26]; no solve.  st: scratch, its contents undefined before.
+int launch_icp(const IcpArgs &a, const IcpPose &pose, IcpState *st, float *mbuf, cudaStream_t stream);
 // Pipeline form: launch `iter` of a frame's ICP (iterations of all levels
 // counted together), with a programmatic dependency on the previous kernel in
 // the stream.  Launch 0 starts from st->R / st->t (and records it as the
