@@ -49,3 +49,54 @@ def test_estimate_combined_takes_undefined_scratch_on_any_stream(cuda, tde, cols
     mag = np.array([S[i, k] for i in range(6) for k in range(i, 7)])
     # per-thread, warp and block sums of 1024 pixels in float, a cross product and a product each rounded thrice
     assert np.all(np.abs(out[0] - ref) <= 32 * 2.0 ** -24 * mag + 1e-30)
+
+
+def _volume_of(fmt, f, w):
+    """Packed records of float values and weights (logical order, origin 0)."""
+    if fmt == 2:
+        return np.concatenate([f.astype(np.float32).view(np.uint8), w.astype(np.uint16).view(np.uint8)])
+    v = f.astype(np.float16).view(np.uint16) if fmt == 1 else np.trunc(f * 32767).astype(np.int16).view(np.uint16)
+    return np.stack([v, w.astype(np.uint16)], -1).reshape(-1).view(np.uint8)
+
+
+@pytest.mark.parametrize("fmt", [0, 1, 2])
+@pytest.mark.parametrize("dims,origin", [((32, 40, 128), (0, 0, 0)), ((64, 300, 128), (21, 299, 5)),
+                                         ((260, 33, 128), (259, 7, 127)), ((37, 31, 128), (3, 30, 64))])
+@pytest.mark.parametrize("density", ["none", "one", "sparse", "every"])
+def test_volume_export_of_empty_sparse_and_full_tiles(cuda, tde, orc, fmt, dims, origin, density):
+    """Extract_Tsdf_Volume equals the oracle, points, weights and order, where no
+    voxel, one voxel, a few and every voxel of a tile emits (alternating signs:
+    three points a voxel, more than the scatter lists at once), for rows of whole
+    and of odd groups, tiles of one row to 256 and shifted origins."""
+    import torch
+    nx, ny, nz = dims
+    n = nx * ny * nz
+    rng = np.random.default_rng(n + fmt)
+    w = rng.integers(1, 100, n)
+    f = np.full(n, 1.0)
+    if density == "one":
+        f[rng.integers(0, n)] = -0.5
+    elif density == "sparse":
+        f[rng.random(n) < 0.002] = -0.25
+        f[rng.random(n) < 0.01] = 0.5
+    elif density == "every":
+        z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+        f = np.where((x + y + z).ravel() % 2 == 0, 0.5, -0.5)
+    if density == "none":
+        w[:] = 0
+    if density == "one":  # its neighbours emit, being neither 1 nor unseen
+        f[f == 1.0] = 0.75
+    vol = _volume_of(fmt, f, w)
+    ob = orc.make_rb(dims, (1.0, 1.0, 1.0))
+    ob.origin_GRID[:] = origin
+    cell = np.array([1.0 / nx, 1.0 / ny, 1.0 / nz], np.float32)
+    po, wo, no = orc.extract_tsdf_volume(vol, fmt, ob, cell, weights=True)
+    assert (no == 0) == (density == "none")
+    rb = tde.round_buffer(dims, (1.0, 1.0, 1.0), origin)
+    dv = torch.from_numpy(vol.copy()).cuda()
+    for cap in (max(no, 1), max(no // 2, 1)):
+        pts, wts, k = tde.extract_tsdf_volume(dv, fmt, rb, tuple(cell), capacity=cap, weights=True)
+        assert k == no
+        m = min(cap, no)
+        assert np.array_equal(pts.cpu().numpy()[:m].view(np.uint32), po[:m].view(np.uint32))
+        assert np.array_equal(wts.cpu().numpy()[:m], wo[:m])
