@@ -162,18 +162,18 @@ int record_segment(tde_pipeline *p, Segment seg, int set, cudaStream_t s) {
             // learned refinement replaces the bilateral filter; ICP and
             // integration both use the refined depth
             TDE_TRY(tde_refiner_forward(p->refiner, raw, 1, depth[0], nullptr, s));
-            TDE_TRY(launch_vertex_map(depth[0], vcur[0], p->intr[0], s));
+            TDE_TRY(launch_vertex_map(depth[0], vcur[0], p->intr[0], s, false));
         } else {
             TDE_TRY(launch_bilateral(raw, depth[0], W, H, c.sigma_space, c.sigma_color, c.max_depth_mm, vcur[0],
-                                     &p->intr[0], s));
+                                     &p->intr[0], s, false));
         }
         for (int l = 1; l < p->levels; ++l)
             TDE_TRY(launch_pyramid(depth[l - 1], depth[l], p->intr[l - 1].cols, p->intr[l - 1].rows, c.sigma_color,
-                                   vcur[l], &p->intr[l], s));
+                                   vcur[l], &p->intr[l], s, false));
         for (int l = 0; l < p->levels; ++l)
-            TDE_TRY(launch_normal_map(vcur[l], ncur[l], p->intr[l].cols, p->intr[l].rows, s));
+            TDE_TRY(launch_normal_map(vcur[l], ncur[l], p->intr[l].cols, p->intr[l].rows, s, false));
         // integration inputs: depth along the ray, and its per-tile maxima
-        TDE_TRY(launch_scale_depth(p->refiner ? depth[0] : raw, p->scaled[set], p->intr[0], s));
+        TDE_TRY(launch_scale_depth(p->refiner ? depth[0] : raw, p->scaled[set], p->intr[0], s, false));
         return launch_depth_max(p->scaled[set], W, H, static_cast<float *>(p->iscratch[set]), s);
     }
     case SEG_ICP: {

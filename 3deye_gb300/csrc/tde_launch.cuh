@@ -5,13 +5,17 @@
 
 namespace tde {
 
+// The preprocessing launches; chained: each comes up while the kernel before it on
+// the stream finishes (see k_depth.cu for where that does not pay).
 int launch_bilateral(const uint16_t *src, uint16_t *dst, int W, int H, float ss, float sc, uint32_t max_mm,
-                     float *vmap, const tde_intrinsics *intr, cudaStream_t stream);
+                     float *vmap, const tde_intrinsics *intr, cudaStream_t stream, bool chained = true);
 int launch_pyramid(const uint16_t *src, uint16_t *dst, int sW, int sH, float sigma_color, float *vmap,
-                   const tde_intrinsics *intr_dst, cudaStream_t stream);
-int launch_scale_depth(const uint16_t *depth, float *scaled, const tde_intrinsics &intr, cudaStream_t stream);
-int launch_vertex_map(const uint16_t *depth, float *vmap, const tde_intrinsics &intr, cudaStream_t stream);
-int launch_normal_map(const float *vmap, float *nmap, int W, int H, cudaStream_t stream);
+                   const tde_intrinsics *intr_dst, cudaStream_t stream, bool chained = true);
+int launch_scale_depth(const uint16_t *depth, float *scaled, const tde_intrinsics &intr, cudaStream_t stream,
+                       bool chained = true);
+int launch_vertex_map(const uint16_t *depth, float *vmap, const tde_intrinsics &intr, cudaStream_t stream,
+                      bool chained = true);
+int launch_normal_map(const float *vmap, float *nmap, int W, int H, cudaStream_t stream, bool chained = true);
 
 int launch_raycast(const void *volume, int format, float *vmap, float *nmap, const tde_point3f &t,
                    const tde_matrix3f &R, float trunc, const tde_intrinsics &intr, const tde_round_buffer &rb,

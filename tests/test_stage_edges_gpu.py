@@ -100,3 +100,23 @@ def test_volume_export_of_empty_sparse_and_full_tiles(cuda, tde, orc, fmt, dims,
         m = min(cap, no)
         assert np.array_equal(pts.cpu().numpy()[:m].view(np.uint32), po[:m].view(np.uint32))
         assert np.array_equal(wts.cpu().numpy()[:m], wo[:m])
+
+
+@pytest.mark.parametrize("cols,rows", [(2, 2), (13, 14), (33, 9), (44, 20), (45, 21), (46, 45), (97, 37)])
+def test_bilateral_and_pyramid_at_window_edges(cuda, tde, orc, cols, rows):
+    """Images below, at and above the size from which a block's windows stay
+    inside: the filter within its rounding of the oracle's weighted mean, the
+    pyramid level equal."""
+    import torch
+    rng = np.random.default_rng(cols * 100 + rows)
+    d = (1500 + 40 * rng.random((rows, cols)) + np.arange(cols) * 2).astype(np.uint16)
+    d[rng.random((rows, cols)) < 0.05] = 0
+    src = torch.from_numpy(d.view(np.int16)).to("cuda").view(torch.uint16)
+    out = tde.bilateral_filter(src, None, 4.5, 30.0, 32767).cpu().numpy().astype(np.float64)
+    _, ratio = orc.bilateral(d, 4.5, 30.0, 32767, want_ratio=True)
+    ratio = np.nan_to_num(ratio)  # a hole in the last row or column: nothing in its window counts
+    # 169 additions and products a sum, weights off by up to 2 + 1.2 |x| units (|x| < 20 where they count), two sums
+    tol = 2 * (2 * 169 + 26) * 2.0 ** -24
+    assert np.all(np.abs(out - ratio) <= 0.5 + tol * ratio)
+    lvl = tde.depth_pyramid_level(src, 30.0).cpu().numpy()
+    assert np.array_equal(lvl, orc.pyramid(d, 30.0))
