@@ -380,7 +380,7 @@ int tde_raycast_ex(const void *volume, int format, float *vmap, float *nmap, con
     TDE_REQUIRE(valid_round_buffer(rb), "raycast: bad round_buffer");
     TDE_REQUIRE(trunc > 0.f && std::isfinite(trunc), "raycast: bad truncation distance");
     TDE_REQUIRE(cell->x > 0.f && cell->y > 0.f && cell->z > 0.f, "raycast: bad cell size");
-    return launch_raycast(volume, format, vmap, nmap, *t, *R, trunc, *intr, *rb, *cell, nullptr, brick_flags,
+    return launch_raycast(volume, format, vmap, nmap, *t, *R, trunc, *intr, *rb, *cell, nullptr, brick_flags, nullptr,
                           as_stream(stream));
 }
 

@@ -24,6 +24,7 @@ struct RayParams {
     const CamPose *dpose;   // when set, t and R are read from here
     const uint8_t *neg_flags;  // per physical 8^3 brick: 0 = holds no negative value
     const uint8_t *super_flags;  // per physical 32^3 super-brick (null: no sample skipping)
+    const unsigned long long *neg_masks;  // the brick flags as one word per super-brick (FLAG_MASKS)
     float inv_cell[3];
     unsigned *touched;      // measurement runs: one bit per voxel record read
 };
@@ -71,20 +72,21 @@ __device__ __forceinline__ float read_tsdf(const void *vol, const RayParams &p, 
 // hit share two of their three axes with the refined point, so those are
 // formed once.
 struct Axis {
-    size_t i0, i1;
+    unsigned i0, i1;  // a volume has fewer than 2^31 voxels
     float w;
 };
 
-__device__ __forceinline__ bool tri_axis(float pt, float q, float cell, int N, int origin, size_t stride, Axis &ax) {
+__device__ __forceinline__ bool tri_axis(float pt, float q, float cell, int N, int origin, unsigned stride, Axis &ax) {
     int g = floor_sat(q);
     if (g <= 0 || g >= N - 1) return false;
     const float v = ((float)g + 0.5f) * cell;
     g = (pt < v) ? g - 1 : g;
     float a = q - ((float)g + 0.5f);
     if (a < 0) { g--; a += 1.0f; }
-    // the two corners g, g + 1 are inside [0, N) here
-    ax.i0 = (size_t)wrap_mod(g + origin, N) * stride;
-    ax.i1 = (size_t)wrap_mod(g + 1 + origin, N) * stride;
+    // the two corners g, g + 1 are inside [0, N) here, and so is the origin
+    const int w0 = g + origin, w1 = w0 + 1;
+    ax.i0 = (unsigned)(w0 - (w0 >= N ? N : 0)) * stride;
+    ax.i1 = (unsigned)(w1 - (w1 >= N ? N : 0)) * stride;
     ax.w = a;
     return true;
 }
@@ -92,7 +94,7 @@ __device__ __forceinline__ bool tri_axis(float pt, float q, float cell, int N, i
 template <int FMT, bool STATS>
 __device__ __forceinline__ float tri_corners(const void *vol, const RayParams &p, const Axis &X, const Axis &Y,
                                              const Axis &Z) {
-    const size_t r00 = Y.i0 + Z.i0, r01 = Y.i0 + Z.i1, r10 = Y.i1 + Z.i0, r11 = Y.i1 + Z.i1;
+    const unsigned r00 = Y.i0 + Z.i0, r01 = Y.i0 + Z.i1, r10 = Y.i1 + Z.i0, r11 = Y.i1 + Z.i1;
     float v000 = load_rec<FMT, STATS>(vol, p, X.i0 + r00), v001 = load_rec<FMT, STATS>(vol, p, X.i0 + r01);
     float v010 = load_rec<FMT, STATS>(vol, p, X.i0 + r10), v011 = load_rec<FMT, STATS>(vol, p, X.i0 + r11);
     float v100 = load_rec<FMT, STATS>(vol, p, X.i1 + r00), v101 = load_rec<FMT, STATS>(vol, p, X.i1 + r01);
@@ -108,11 +110,11 @@ __device__ __forceinline__ bool axis_x(const RayParams &p, float pt, float q, Ax
     return tri_axis(pt, q, p.cell.x, p.rb.voxels_size.x, p.rb.origin_GRID.x, 1, ax);
 }
 __device__ __forceinline__ bool axis_y(const RayParams &p, float pt, float q, Axis &ax) {
-    return tri_axis(pt, q, p.cell.y, p.rb.voxels_size.y, p.rb.origin_GRID.y, (size_t)p.rb.voxels_size.x, ax);
+    return tri_axis(pt, q, p.cell.y, p.rb.voxels_size.y, p.rb.origin_GRID.y, (unsigned)p.rb.voxels_size.x, ax);
 }
 __device__ __forceinline__ bool axis_z(const RayParams &p, float pt, float q, Axis &ax) {
     return tri_axis(pt, q, p.cell.z, p.rb.voxels_size.z, p.rb.origin_GRID.z,
-                    (size_t)p.rb.voxels_size.x * (size_t)p.rb.voxels_size.y, ax);
+                    (unsigned)p.rb.voxels_size.x * (unsigned)p.rb.voxels_size.y, ax);
 }
 
 template <int FMT, bool STATS>
@@ -169,15 +171,20 @@ __device__ __noinline__ void refine_surface(const void *vol, const RayParams &p,
 }
 
 // Voxel of the sample at time ct: floor(pos / cell) with pos = t + dir * ct
-// evaluated exactly as the reference does whenever it matters.  The fast
-// estimate o/c + (d/c) ct is within ~4e-4 voxel of the exact quotient, so a
-// fractional part clear of 4e-3 from an integer settles the floor; otherwise
-// the position and the IEEE quotient are computed.
+// evaluated exactly as the reference does whenever it matters.  With u = 2^-24
+// and M = |o/c| + |d/c| ct, the estimate o/c + (d/c) ct is within 6 u M of the
+// reference's quotient (two roundings each of o/c and d/c and one of the sum; the
+// reference's product, sum and quotient), so an estimate further than 8 u M from
+// the nearest integer settles the floor; otherwise the position and the IEEE
+// quotient are computed.  The margin is formed once a ray, for the time at which
+// it leaves the volume: near 5e-4 voxel in 512^3, where one warp in ten needs the
+// exact form for some lane (a fixed 4e-3: every second one).
 constexpr float kSkipMargin = 1e-2f;  // voxels
 
 struct RayFast {
     float o[3], d[3];  // t / cell, dir / cell
     float inv_d[3];    // 1 / d
+    float margin;      // voxels
 };
 
 // Time at which the ray (fast coordinates) leaves the box [lo, lo + size)^3
@@ -191,32 +198,68 @@ __device__ __forceinline__ float box_exit(const RayFast &rf, float lox, float lo
     return fminf(fminf(ex, ey), ez);
 }
 
-__device__ __forceinline__ int axis_floor(float q, float o, float d, float cell, float ct) {
-    const float fr = q - floorf(q);
-    if (fabsf(q) < 2048.f && fr > 4e-3f && fr < 1.f - 4e-3f) return __float2int_rd(q);
+// Out of line: the march loop has to stay within the instruction cache.
+__device__ __noinline__ int axis_exact(float o, float d, float cell, float ct) {
     return floor_sat((o + d * ct) / cell);
+}
+
+// Nearest integer of q (|q| < 2^22) and q's distance from it; the floor follows.
+__device__ __forceinline__ int axis_floor(float q, float &dist) {
+    const float magic = 12582912.f;  // 1.5 * 2^23
+    const float t = q + magic;
+    dist = q - (t - magic);
+    return __float_as_int(t) - __float_as_int(magic) - (dist < 0.f ? 1 : 0);
 }
 
 __device__ __forceinline__ void sample_voxel(const RayParams &p, const f3 &org, const f3 &dir, const RayFast &rf,
                                              float ct, int &sx, int &sy, int &sz) {
-    sx = axis_floor(fmaf(rf.d[0], ct, rf.o[0]), org.x, dir.x, p.cell.x, ct);
-    sy = axis_floor(fmaf(rf.d[1], ct, rf.o[1]), org.y, dir.y, p.cell.y, ct);
-    sz = axis_floor(fmaf(rf.d[2], ct, rf.o[2]), org.z, dir.z, p.cell.z, ct);
+    float dx, dy, dz;
+    sx = axis_floor(fmaf(rf.d[0], ct, rf.o[0]), dx);
+    sy = axis_floor(fmaf(rf.d[1], ct, rf.o[1]), dy);
+    sz = axis_floor(fmaf(rf.d[2], ct, rf.o[2]), dz);
+    if (!(fabsf(dx) > rf.margin && fabsf(dy) > rf.margin && fabsf(dz) > rf.margin)) {
+        if (!(fabsf(dx) > rf.margin)) sx = axis_exact(org.x, dir.x, p.cell.x, ct);
+        if (!(fabsf(dy) > rf.margin)) sy = axis_exact(org.y, dir.y, p.cell.y, ct);
+        if (!(fabsf(dz) > rf.margin)) sz = axis_exact(org.z, dir.z, p.cell.z, ct);
+    }
 }
 
-// A block takes 16 x kRayBlockRows pixels, a warp an 8 x 4 tile.
-constexpr int kRayBlockRows = 16;
-constexpr int kRayThreads = 16 * kRayBlockRows;
+// The last of the sample times tn, tn + step, ... (each a rounded addition) before
+// `lim` that a march from tn reaches before max_time; four additions a round.
+__device__ __forceinline__ float advance(float tn, float step, float lim, float max_time) {
+    for (;;) {
+        const float a = tn + step, b = a + step, c = b + step, d = c + step;
+        if (d < lim && c < max_time) { tn = d; continue; }
+        // the times grow: each condition holds only where the one before does
+        return (c < lim && b < max_time) ? c : (b < lim && a < max_time) ? b : (a < lim && tn < max_time) ? a : tn;
+    }
+}
 
-template <int FMT, bool SKIP, bool STATS>
+// A block is a row of kRayWarps warps, a warp an 8 x 4 tile of pixels, so its rays
+// start close together and sample neighbouring voxels.  What bounds the kernel
+// at 640x480 / 512^3: its instructions (4000 a warp, 1600 of them the refinement's;
+// 66 % of the issue slots while an SM is busy) and the longest rays' chain of
+// loads (an SM is busy for 100 to 140 thousand cycles; blocks of 1 to 8 warps end
+// within 5 % of each other).  The pipeline's cast: 97 us with byte flags read
+// sample by sample, 67 us with a word of flags a super-brick, rarer exact places
+// and four additions a round of `advance`.
+constexpr int kRayWarps = 4;
+constexpr int kRayThreads = 32 * kRayWarps;
+constexpr int kRayBlockCols = 8 * kRayWarps, kRayBlockRows = 4;
+
+// What the march knows of empty bricks: nothing, a byte each (the flags a caller
+// keeps), or a word of 64 bits per 32^3 super-brick (the pipeline's): one load where
+// a ray enters the super-brick in place of two dependent ones and one for each of
+// its bricks.
+enum FlagKind { FLAG_NONE, FLAG_BYTES, FLAG_MASKS };
+
+template <int FMT, FlagKind FLAGS, bool STATS>
 __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__restrict__ vol, float *__restrict__ vmap,
                                                      float *__restrict__ nmap, const __grid_constant__ RayParams p) {
-    // each warp takes an 8x4 tile so its rays start close together and
-    // sample neighbouring voxels
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    const int y = blockIdx.y * kRayBlockRows + (warp >> 1) * 4 + (lane >> 3);
+    const int x = blockIdx.x * kRayBlockCols + warp * 8 + (lane & 7);
+    const int y = blockIdx.y * kRayBlockRows + (lane >> 3);
     const int W = p.intr.cols, H = p.intr.rows;
     // the pose: from the parameters, or read on the device
     tde_matrix3f R = p.R;
@@ -274,6 +317,12 @@ __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__rest
         rf.o[0] = org.x * p.inv_cell[0]; rf.o[1] = org.y * p.inv_cell[1]; rf.o[2] = org.z * p.inv_cell[2];
         rf.d[0] = dir.x * p.inv_cell[0]; rf.d[1] = dir.y * p.inv_cell[1]; rf.d[2] = dir.z * p.inv_cell[2];
         rf.inv_d[0] = 1.f / rf.d[0]; rf.inv_d[1] = 1.f / rf.d[1]; rf.inv_d[2] = 1.f / rf.d[2];
+        // samples up to one step past the exit are placed; none of an estimate too large for axis_floor
+        const float t_far = t_exit + 2.f * step;
+        const float far = fmaxf(fmaxf(fmaf(fabsf(rf.d[0]), t_far, fabsf(rf.o[0])),
+                                      fmaf(fabsf(rf.d[1]), t_far, fabsf(rf.o[1]))),
+                                fmaf(fabsf(rf.d[2]), t_far, fabsf(rf.o[2])));
+        rf.margin = far < 4194304.f ? far * 4.76837158e-7f : 1.f;  // 8 * 2^-24
         // previous sample: its value when `known`, else only "non-negative";
         // its time lets the value be fetched when it turns out to matter
         float tsdf = read_tsdf<FMT, STATS>(vol, p, gx, gy, gz);
@@ -283,8 +332,51 @@ __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__rest
         const int nsx = (N.x + 31) >> 5, nsy = (N.y + 31) >> 5;
         int last_super = -1;
 
-        // raycast.cl:254-404, one sample per iteration
-        while (time_curr < p.max_time) {
+        // raycast.cl:254-404
+        if (FLAGS == FLAG_NONE) {
+            // kAhead samples a round: their records are read together (the next
+            // sample's place does not depend on them), then tested in order: 88 us
+            // at 640x480 / 512^3 for 107 one by one (3: 89, 6: 90, 8: 91)
+            constexpr int kAhead = STATS ? 1 : 4;
+            bool more = true;
+            while (more) {
+                float at[kAhead + 1], v[kAhead];
+                bool alive[kAhead];
+                at[0] = time_curr;
+                #pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
+                    at[k + 1] = at[k] + step;
+                    int sx, sy, sz;
+                    sample_voxel(p, org, dir, rf, at[k + 1], sx, sy, sz);
+                    alive[k] = (k == 0 || alive[k > 0 ? k - 1 : 0]) && at[k] < p.max_time &&
+                               (unsigned)sx < (unsigned)N.x && (unsigned)sy < (unsigned)N.y &&
+                               (unsigned)sz < (unsigned)N.z;
+                    v[k] = 0.f;
+                    if (alive[k]) {
+                        int px = sx + p.rb.origin_GRID.x; px -= px >= N.x ? N.x : 0;
+                        int py = sy + p.rb.origin_GRID.y; py -= py >= N.y ? N.y : 0;
+                        int pz = sz + p.rb.origin_GRID.z; pz -= pz >= N.z ? N.z : 0;
+                        v[k] = load_rec<FMT, STATS>(
+                            vol, p, (unsigned)px + (unsigned)N.x * ((unsigned)py + (unsigned)N.y * (unsigned)pz));
+                    }
+                }
+                #pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
+                    more = more && alive[k];
+                    if (more && tsdf > 0.f && v[k] < 0.f) { hit = true; hit_time = at[k]; more = false; }
+                    if (tsdf < 0.f && v[k] > 0.f) more = false;
+                    tsdf = v[k];
+                }
+                time_curr = at[kAhead];
+            }
+        }
+        // with flags, one sample per iteration; a sample in a super-brick (or else
+        // in a brick) without negative values, after a non-negative one, lets
+        // time advance by the same additions, without evaluating samples, until
+        // the next one nears the exit: no test can fire in between
+        unsigned long long mask = 0;
+        bool empty_super = false;
+        while (FLAGS != FLAG_NONE && time_curr < p.max_time) {
             const float ct = time_curr + step;
             int sx, sy, sz;
             sample_voxel(p, org, dir, rf, ct, sx, sy, sz);
@@ -292,52 +384,31 @@ __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__rest
             int px = sx + p.rb.origin_GRID.x; px -= px >= N.x ? N.x : 0;
             int py = sy + p.rb.origin_GRID.y; py -= py >= N.y ? N.y : 0;
             int pz = sz + p.rb.origin_GRID.z; pz -= pz >= N.z ? N.z : 0;
-            bool have = true;
-            if (SKIP) {
-                if (p.super_flags && !(known && tsdf < 0.f)) {
-                    const int sid = (px >> 5) + nsx * ((py >> 5) + nsy * (pz >> 5));
-                    if (sid != last_super) {
-                        last_super = sid;
-                        if (!__ldg(p.super_flags + sid)) {
-                            // A 32^3 super-brick with no negative value entered after a
-                            // non-negative sample: no test can fire inside it, so time
-                            // advances by the same additions without evaluating samples
-                            // until the next one nears the exit.
-                            const float lim = box_exit(rf, (float)(sx - (px & 31)), (float)(sy - (py & 31)),
-                                                       (float)(sz - (pz & 31)), 32.f);
-                            float tn = time_curr;
-                            int m = 0;
-                            while (tn < p.max_time && tn + step < lim) { tn = tn + step; ++m; }
-                            if (m > 0) {
-                                time_curr = tn;
-                                known = false;
-                                prev_ct = tn;
-                                continue;
-                            }
-                        }
-                    }
+            const int sid = (px >> 5) + nsx * ((py >> 5) + nsy * (pz >> 5));
+            bool have;
+            if (FLAGS == FLAG_MASKS) {
+                if (sid != last_super) {
+                    mask = __ldg(p.neg_masks + sid);
+                    empty_super = mask == 0 && p.super_flags;
                 }
-                have = __ldg(p.neg_flags + ((px >> 3) + nbx * ((py >> 3) + nby * (pz >> 3)))) != 0;
+                have = (mask >> (((px >> 3) & 3) | ((py >> 1) & 12) | ((pz << 1) & 48))) & 1;
+            } else {
+                if (sid != last_super) empty_super = p.super_flags && !__ldg(p.super_flags + sid);
+                have = !empty_super && __ldg(p.neg_flags + ((px >> 3) + nbx * ((py >> 3) + nby * (pz >> 3)))) != 0;
             }
-            const size_t addr = (size_t)px + (size_t)N.x * ((size_t)py + (size_t)N.y * (size_t)pz);
-            float cur = 0.f;
-            if (SKIP && !have) {
-                if (!(known && tsdf < 0.f)) {
-                    // a non-negative sample after a non-negative one: no test can
-                    // fire, nor at the following samples inside this 8^3 brick,
-                    // which advance by the same additions
-                    const float lim = box_exit(rf, (float)(sx - (px & 7)), (float)(sy - (py & 7)),
-                                               (float)(sz - (pz & 7)), 8.f);
-                    float tn = ct;
-                    while (tn < p.max_time && tn + step < lim) tn = tn + step;
-                    known = false;
-                    prev_ct = tn;
-                    time_curr = tn;
-                    continue;
-                }
+            last_super = sid;
+            if (!have && !(known && tsdf < 0.f)) {
+                const int edge = empty_super ? 31 : 7;
+                const float lim = box_exit(rf, (float)(sx - (px & edge)), (float)(sy - (py & edge)),
+                                           (float)(sz - (pz & edge)), (float)(edge + 1));
+                time_curr = advance(ct, step, lim, p.max_time);
+                known = false;
+                prev_ct = time_curr;
+                continue;
             }
-            cur = load_rec<FMT, STATS>(vol, p, addr);
-            if (SKIP && !known) {
+            const unsigned addr = (unsigned)px + (unsigned)N.x * ((unsigned)py + (unsigned)N.y * (unsigned)pz);
+            const float cur = load_rec<FMT, STATS>(vol, p, addr);
+            if (!known) {
                 if (!(cur < 0.f)) {  // prev >= 0 and cur >= 0
                     tsdf = cur;
                     known = true;
@@ -507,8 +578,8 @@ __global__ void transform_maps_kernel(const float *__restrict__ vs, const float 
 
 int launch_raycast(const void *volume, int format, float *vmap, float *nmap, const tde_point3f &t,
                    const tde_matrix3f &R, float trunc, const tde_intrinsics &intr, const tde_round_buffer &rb,
-                   const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags, cudaStream_t stream,
-                   unsigned *touched) {
+                   const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags, const unsigned long long *neg_masks,
+                   cudaStream_t stream, unsigned *touched) {
     RayParams p;
     p.dpose = dpose;
     p.neg_flags = neg_flags;
@@ -519,19 +590,21 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
     p.inv_cell[0] = 1.f / cell.x; p.inv_cell[1] = 1.f / cell.y; p.inv_cell[2] = 1.f / cell.z;
     // super-brick sample skipping needs whole 32^3 super-bricks on every axis
     const bool whole = rb.voxels_size.x % 32 == 0 && rb.voxels_size.y % 32 == 0 && rb.voxels_size.z % 32 == 0;
+    // (with masks only asked whether it is null)
     p.super_flags = (neg_flags && whole) ? neg_flags + brick_count(rb) : nullptr;
+    p.neg_masks = neg_masks;
     p.touched = touched;
     dim3 block(kRayThreads);
-    dim3 grid(div_up(intr.cols, 16), div_up(intr.rows, kRayBlockRows));
+    dim3 grid(div_up(intr.cols, kRayBlockCols), div_up(intr.rows, kRayBlockRows));
     return dispatch_format(format, [&](auto F) {
         constexpr int FM = decltype(F)::value;
-        if (touched) {
-            if (neg_flags) raycast_kernel<FM, true, true><<<grid, block, 0, stream>>>(volume, vmap, nmap, p);
-            else raycast_kernel<FM, false, true><<<grid, block, 0, stream>>>(volume, vmap, nmap, p);
-        } else {
-            if (neg_flags) raycast_kernel<FM, true, false><<<grid, block, 0, stream>>>(volume, vmap, nmap, p);
-            else raycast_kernel<FM, false, false><<<grid, block, 0, stream>>>(volume, vmap, nmap, p);
-        }
+        const auto kernel = [&](auto stats) {
+            constexpr bool ST = decltype(stats)::value;
+            return neg_masks ? raycast_kernel<FM, FLAG_MASKS, ST>
+                             : neg_flags ? raycast_kernel<FM, FLAG_BYTES, ST> : raycast_kernel<FM, FLAG_NONE, ST>;
+        };
+        const auto k = touched ? kernel(std::true_type{}) : kernel(std::false_type{});
+        k<<<grid, block, 0, stream>>>(volume, vmap, nmap, p);
         return check_launch("raycast");
     });
 }

@@ -103,6 +103,7 @@ struct tde_pipeline {
     FrameOut *out = nullptr;
     unsigned long long *stats = nullptr;
     uint8_t *negflags = nullptr;  // per physical brick: may hold a negative value
+    unsigned long long *negmasks = nullptr;  // the same flags, a word per 32^3 super-brick
     uint8_t *satflags = nullptr;  // per logical brick: every voxel at f = 1, maximum weight
     // colour volume (tde_pipeline_enable_color): RGB frames per input set, and
     // per set the level-0 model vertex map and camera pose the update reads
@@ -147,7 +148,7 @@ int cast_model(tde_pipeline *p, cudaStream_t s) {
     tde_point3f t0{0, 0, 0};
     tde_matrix3f R0{};
     return launch_raycast(p->volume, c.tsdf_format, p->vmod[0], p->nmod[0], t0, R0, c.trunc, p->intr[0], p->rb, p->cell,
-                          p->cam, p->negflags, s);
+                          p->cam, p->negflags, p->negmasks, s);
 }
 
 // Records one segment for input set `set` onto stream s.
@@ -207,7 +208,7 @@ int record_segment(tde_pipeline *p, Segment seg, int set, cudaStream_t s) {
         P.trunc = c.trunc; P.max_weight = c.max_weight; P.intr = p->intr[0]; P.rb = p->rb; P.cell = p->cell;
         P.n = voxel_count(p->rb); P.dpose = p->cam;
         return launch_integrate(p->scaled[set], p->volume, c.tsdf_format, P, p->iscratch[set], p->negflags, p->stats, s,
-                                p->satflags);
+                                p->satflags, p->negmasks);
     }
     case SEG_RAYCAST: {
         TDE_TRY(cast_model(p, s));
@@ -372,7 +373,8 @@ void release(tde_pipeline *p) {
     }
     for (int l = 0; l < 3; ++l) { cudaFree(p->vmod[l]); cudaFree(p->nmod[l]); }
     cudaFree(p->st); cudaFree(p->cam); cudaFree(p->out);
-    cudaFree(p->stats); cudaFree(p->volume); cudaFree(p->negflags); cudaFree(p->satflags);
+    cudaFree(p->stats); cudaFree(p->volume); cudaFree(p->negflags); cudaFree(p->negmasks);
+    cudaFree(p->satflags);
     cudaFree(p->slab_scratch); cudaFree(p->slab_points); cudaFree(p->slab_weights); cudaFree(p->slab_count);
     cudaFree(p->slab_colors); cudaFree(p->colvol); cudaFree(p->rgb[0]); cudaFree(p->rgb[1]); cudaFree(p->cscratch);
     if (p->pre_stream) cudaStreamDestroy(p->pre_stream);
@@ -572,12 +574,15 @@ int tde_pipeline_create(const tde_pipeline_config *cfg, const double *pose12, td
     if ((st = dalloc(&p->st, 1, "icp state")) || (st = dalloc(&p->cam, 1, "camera pose")) ||
         (st = dalloc(&p->out, 1, "frame out")) || (st = dalloc(&p->stats, 3, "stats")) ||
         (st = dalloc(&p->negflags, brick_flags_bytes(p->rb), "brick flags")) ||
+        (st = dalloc(&p->negmasks, superbrick_count(p->rb), "brick masks")) ||
         (st = dalloc(&p->satflags, brick_count(p->rb), "saturation flags")))
         return fail(st);
     e = cudaMemsetAsync(p->satflags, 0, brick_count(p->rb), p->stream);
     if (e != cudaSuccess) return fail(cuda_fail(e, "saturation flags"));
     e = cudaMemsetAsync(p->negflags, 0, brick_flags_bytes(p->rb), p->stream);
     if (e != cudaSuccess) return fail(cuda_fail(e, "brick flags"));
+    e = cudaMemsetAsync(p->negmasks, 0, superbrick_count(p->rb) * sizeof(unsigned long long), p->stream);
+    if (e != cudaSuccess) return fail(cuda_fail(e, "brick masks"));
     e = cudaMemsetAsync(p->stats, 0, 3 * sizeof(unsigned long long), p->stream);
     if (e != cudaSuccess) return fail(cuda_fail(e, "stats"));
     if (!c.integrate_stats) { cudaFree(p->stats); p->stats = nullptr; }
@@ -873,7 +878,8 @@ int tde_pipeline_raycast_records(tde_pipeline *p, int skip_empty, uint64_t *reco
         tde_point3f t0{0, 0, 0};
         tde_matrix3f R0{};
         st = launch_raycast(p->volume, p->cfg.tsdf_format, vm, nm, t0, R0, p->cfg.trunc, p->intr[0], p->rb, p->cell,
-                            p->cam, skip_empty ? p->negflags : nullptr, p->stream, bits);
+                            p->cam, skip_empty ? p->negflags : nullptr, skip_empty ? p->negmasks : nullptr, p->stream,
+                            bits);
         if (st == TDE_OK) {
             popcount_kernel<<<1024, 256, 0, p->stream>>>(bits, words, cnt);
             unsigned long long h = 0;
@@ -1090,6 +1096,7 @@ int tde_pipeline_restore(tde_pipeline *p, const void *buffer, size_t bytes) {
     // the model maps the next frame tracks against: cast from the restored
     // volume and pose, as the checkpointed frame cast them
     cudaStream_t s = p->stream;
+    TDE_TRY(launch_brick_masks(p->negflags, p->rb, p->negmasks, s));
     TDE_TRY(upload_camera(p, h.pose12, s));
     TDE_TRY(cast_model(p, s));
     TDE_TRY(record_segment(p, SEG_RESIZE, 0, s));

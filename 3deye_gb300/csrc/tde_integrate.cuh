@@ -73,8 +73,15 @@ size_t integrate_scratch_bytes(int W, int H, const tde_round_buffer &rb);
 // Such a brick lying entirely more than the truncation distance in front of
 // every observed depth it projects to would be left unchanged voxel by voxel,
 // so it is not swept.
+// neg_masks (may be null; neg_flags is set too then): per physical super-brick
+// (superbrick_count words) the flags of its bricks, bit x + 4 y + 16 z of the
+// brick's place in it.
 int launch_integrate(const float *depth_scaled, void *volume, int format, const IntegrateParams &P, void *scratch,
-                     uint8_t *neg_flags, unsigned long long *stats, cudaStream_t stream, uint8_t *sat_flags = nullptr);
+                     uint8_t *neg_flags, unsigned long long *stats, cudaStream_t stream, uint8_t *sat_flags = nullptr,
+                     unsigned long long *neg_masks = nullptr);
+// neg_masks from neg_flags.
+int launch_brick_masks(const uint8_t *neg_flags, const tde_round_buffer &rb, unsigned long long *neg_masks,
+                       cudaStream_t stream);
 // Colour integration (Integrate_Colors): scratch of integrate_colors_scratch_bytes (256-byte aligned);
 // `updated` (may be null) accumulates the count of voxels updated.
 size_t integrate_colors_scratch_bytes(int W, int H, const tde_round_buffer &rb);

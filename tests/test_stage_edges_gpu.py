@@ -120,3 +120,53 @@ def test_bilateral_and_pyramid_at_window_edges(cuda, tde, orc, cols, rows):
     assert np.all(np.abs(out - ratio) <= 0.5 + tol * ratio)
     lvl = tde.depth_pyramid_level(src, 30.0).cpu().numpy()
     assert np.array_equal(lvl, orc.pyramid(d, 30.0))
+
+
+@pytest.mark.parametrize("voxels,fmt", [(96, 2), (96, 1), (40, 1), (52, 0)])
+def test_empty_bricks_are_skipped_exactly(cuda, tde, orc, voxels, fmt):
+    """The pipeline's model maps (cast with the empty bricks' masks) equal a cast
+    of the same volume that skips nothing, bit for bit: while frames arrive,
+    after a shift that leaves bricks across the origin, and after a restore.
+    Volumes of whole super-bricks, of whole bricks, and of neither."""
+    syn = importlib.import_module("3deye_gb300.synth")
+    pl = importlib.import_module("3deye_gb300.pipeline")
+    cfg = syn.small_config("c1", frames=8, cols=97, rows=61, voxels=voxels, fmt=fmt)
+    scene, traj = syn.make_scene(cfg, 1000), syn.make_trajectory(cfg, 2000)
+    intr = orc.Intr(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cfg.cols, cfg.rows)
+    depths = [orc.apply_noise(orc.render_depth(scene, traj[i], intr), 3000, i) for i in range(cfg.frames)]
+    it = tde.Intrinsics(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cfg.cols, cfg.rows)
+    tde.lib.tde_memcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+
+    def check(p):
+        import torch
+        vol, rb = p.volume()
+        cell = [np.float32(rb.volume_size.x) / np.float32(voxels)] * 3
+        got = []
+        for ptr in p.model_maps(0):
+            a = np.zeros((cfg.rows, cfg.cols, 3), np.float32)
+            tde.check(tde.lib.tde_memcpy(a.ctypes.data_as(C.c_void_p), C.c_void_p(ptr), a.nbytes, 1))
+            got.append(a)
+        pose = p.pose().astype(np.float32)
+        ref = [torch.empty((cfg.rows, cfg.cols, 3), dtype=torch.float32, device=cuda) for _ in range(2)]
+        R, t, cs = tde.mat3(pose[:9].reshape(3, 3)), tde.vec3(pose[9:]), tde.vec3(cell)
+        tde.check(tde.lib.tde_raycast(vol, fmt, ref[0].data_ptr(), ref[1].data_ptr(), C.byref(t), C.byref(R),
+                                      cfg.trunc_m, C.byref(it), C.byref(rb), C.byref(cs), None))
+        torch.cuda.synchronize()
+        assert np.isfinite(got[0]).any()
+        for a, b in zip(got, ref):
+            assert np.array_equal(a.view(np.uint32), b.cpu().numpy().view(np.uint32))
+
+    p = pl.Pipeline(cfg, traj[0])
+    for d in depths[:3]:
+        p.process(d)
+        check(p)
+    p.shift((3, -2, 5))
+    assert p.volume()[1].origin_GRID.x % 8 and p.volume()[1].origin_GRID.z % 8
+    for d in depths[3:6]:
+        p.process(d)
+        check(p)
+    q = pl.Pipeline(cfg, traj[0])
+    q.restore(p.checkpoint())
+    check(q)
+    q.process(depths[6])
+    check(q)
