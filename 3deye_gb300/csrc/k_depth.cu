@@ -2,10 +2,7 @@
 // depth, vertex maps and PCA normal maps.
 //
 // These kernels follow one another on a stream and take a few microseconds
-// each, so a caller's launches are chained by programmatic serialisation: a
-// kernel's blocks come up while the one before finishes and wait there before
-// they touch memory.  Every block waits, and none reads through the read-only path
-// (a load that the compiler may move over the wait).  A 640x480 frame's nine
+// each, so a caller's launches are chained (tde_common.cuh).  A 640x480 frame's nine
 // launches (filter, two pyramid levels, three vertex and three normal maps) took
 // 92 us with plain launches and loops that kept to the image, 60 us now.  The
 // pipeline's preprocessing runs beside the tracking and is not what a frame waits
@@ -13,13 +10,8 @@
 // tracker's want (a frame of the learned pipeline 370 us, 377 chained).
 #include "tde_common.cuh"
 
-#include <utility>
-
 namespace tde {
 namespace {
-
-__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 constexpr int kBR = 6;   // bilateral radius, compute_bilateral_filtering.cl:19
 constexpr int kBX = 32, kBY = 8;
@@ -277,20 +269,12 @@ __global__ void __launch_bounds__(kBX *kBY) normal_map_kernel(const float *vmap,
 
 namespace {
 
+// A grid of kBX x kBY threads over a cols x rows image.
 template <typename... KArgs, typename... Args>
-int launch(const char *what, bool chained, void (*kernel)(KArgs...), int cols, int rows, int block_rows,
-           cudaStream_t stream, Args &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(div_up(cols, kBX), div_up(rows, block_rows));
-    cfg.blockDim = dim3(kBX, kBY);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    TDE_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...), what);
-    return check_launch(what);
+int launch(const char *what, bool chained, void (*kernel)(KArgs...), int cols, int rows, cudaStream_t stream,
+           Args &&...args) {
+    return launch_chained(what, chained, kernel, dim3(div_up(cols, kBX), div_up(rows, kBY)), dim3(kBX, kBY), stream,
+                          std::forward<Args>(args)...);
 }
 
 }  // namespace
@@ -300,7 +284,7 @@ int launch_bilateral(const uint16_t *src, uint16_t *dst, int W, int H, float ss,
     const float inv_ss = 0.5f / (ss * ss), inv_sc = 0.5f / (sc * sc);
     const float fx = intr ? intr->fx : 1.f, fy = intr ? intr->fy : 1.f, cx = intr ? intr->cx : 0.f,
                 cy = intr ? intr->cy : 0.f;
-    return launch("bilateral", chained, bilateral_kernel, W, H, kBY, stream, src, dst, W, H, inv_ss, inv_sc, max_mm, vmap,
+    return launch("bilateral", chained, bilateral_kernel, W, H, stream, src, dst, W, H, inv_ss, inv_sc, max_mm, vmap,
                   fx, fy, cx, cy);
 }
 
@@ -309,22 +293,22 @@ int launch_pyramid(const uint16_t *src, uint16_t *dst, int sW, int sH, float sig
     const int thresh = (int)(3.f * sigma_color);
     const float fx = intr_dst ? intr_dst->fx : 1.f, fy = intr_dst ? intr_dst->fy : 1.f;
     const float cx = intr_dst ? intr_dst->cx : 0.f, cy = intr_dst ? intr_dst->cy : 0.f;
-    return launch("depth_pyramid", chained, pyramid_kernel, sW >> 1, sH >> 1, kBY, stream, src, dst, sW, sH, thresh, vmap,
+    return launch("depth_pyramid", chained, pyramid_kernel, sW >> 1, sH >> 1, stream, src, dst, sW, sH, thresh, vmap,
                   fx, fy, cx, cy);
 }
 
 int launch_scale_depth(const uint16_t *depth, float *scaled, const tde_intrinsics &intr, cudaStream_t stream,
                        bool chained) {
-    return launch("scale_depth", chained, scale_depth_kernel, intr.cols, intr.rows, kBY, stream, depth, scaled, intr);
+    return launch("scale_depth", chained, scale_depth_kernel, intr.cols, intr.rows, stream, depth, scaled, intr);
 }
 
 int launch_vertex_map(const uint16_t *depth, float *vmap, const tde_intrinsics &intr, cudaStream_t stream,
                       bool chained) {
-    return launch("vertex_map", chained, vertex_map_kernel, intr.cols, intr.rows, kBY, stream, depth, vmap, intr);
+    return launch("vertex_map", chained, vertex_map_kernel, intr.cols, intr.rows, stream, depth, vmap, intr);
 }
 
 int launch_normal_map(const float *vmap, float *nmap, int W, int H, cudaStream_t stream, bool chained) {
-    return launch("normal_map", chained, normal_map_kernel, W, H, kBY, stream, vmap, nmap, W, H);
+    return launch("normal_map", chained, normal_map_kernel, W, H, stream, vmap, nmap, W, H);
 }
 
 }  // namespace tde

@@ -21,6 +21,12 @@
 // distance in front of the smallest depth it projects to, is not swept either:
 // each of its voxels would get tsdf = 1 and keep f = 1, w = max, bit for bit.
 //
+// A caller's launches (depth tiles, cull, sweep) are chained and start from one
+// memset (three before): a 611x457 frame into 384^3, 16-bit, 58 -> 49 us a call.
+// The pipeline's stay plain (640x480 frames into 512^3: 262 us a frame, 294
+// chained, since waiting blocks keep the next frame's preprocessing out), but
+// its frames no longer start the sweep with a memset of their own.
+//
 // Built with -fmad=false (no contraction beyond the explicit __fmaf_rn) so every
 // voxel decision and value equals the oracle's.
 #include "tde_common.cuh"
@@ -36,7 +42,10 @@ constexpr float kNoDepth = 3.3961514e38f;  // bytes 0x7f7f7f7f: "no non-zero dep
 
 // ---------------------------------------------------------------------------
 // Max scaled depth per 16x16 tile (level 0) and per 32..256 tiles (levels 1-4,
-// by atomicMax on the bit pattern: non-negative floats order like ints).
+// by atomicMax on the bit pattern: non-negative floats order like ints).  The
+// smallest depths of levels 1-4 are kept as their bit pattern's distance from
+// kNoDepth's, so that they too grow from 0 and one memset starts both, and the
+// counter of the surviving bricks behind them.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) depth_max_kernel(const float *__restrict__ depth, int W, int H,
                                                         DepthMaxPyramid pyr) {
@@ -64,7 +73,7 @@ __global__ void __launch_bounds__(256) depth_max_kernel(const float *__restrict_
         for (int l = 1; l < kDepthMaxLevels; ++l) {
             const int i = (ty >> l) * pyr.tiles_x[l] + (tx >> l);
             atomicMax(reinterpret_cast<int *>(&pyr.level[l][i]), __float_as_int(m));
-            atomicMin(reinterpret_cast<int *>(&pyr.level_min[l][i]), __float_as_int(mn));
+            atomicMax(reinterpret_cast<int *>(&pyr.level_min[l][i]), __float_as_int(kNoDepth) - __float_as_int(mn));
         }
     }
 }
@@ -93,7 +102,10 @@ __device__ __forceinline__ float rect_min_depth(const DepthMaxPyramid &pyr, int 
     const int s = 4 + l;
     float m = kNoDepth;
     for (int ty = v0 >> s; ty <= (v1 >> s); ++ty)
-        for (int tx = u0 >> s; tx <= (u1 >> s); ++tx) m = fminf(m, pyr.level_min[l][ty * pyr.tiles_x[l] + tx]);
+        for (int tx = u0 >> s; tx <= (u1 >> s); ++tx) {
+            const float t = pyr.level_min[l][ty * pyr.tiles_x[l] + tx];
+            m = fminf(m, l == 0 ? t : __int_as_float(__float_as_int(kNoDepth) - __float_as_int(t)));
+        }
     return m;
 }
 
@@ -174,10 +186,11 @@ __device__ __forceinline__ bool brick_culled(const IntegrateParams &P, const Pos
 template <bool COLOR = false>
 __global__ void __launch_bounds__(256) cull_bricks_kernel(const IntegrateParams P,
                                                           const __grid_constant__ DepthMaxPyramid pyr,
-                                                          int *__restrict__ list, int *__restrict__ count,
-                                                          const uint8_t *__restrict__ sat) {
+                                                          int *list, int *count, const uint8_t *sat) {
     __shared__ Pose q;
     const int tid = threadIdx.x, lane = tid & 31;
+    allow_next_kernel();
+    wait_previous_kernel();
     if (tid < 12) {
         float v;
         if (P.dpose) v = tid < 9 ? P.dpose->R_inv[tid] : P.dpose->t[tid - 9];
@@ -217,14 +230,15 @@ __device__ __forceinline__ void mark_negative(uint8_t *neg_flags, unsigned long 
 // list so the work spreads over every SM whatever the scene's layout.
 template <int FMT>
 __global__ void __launch_bounds__(256, kIntBlocksPerSM) integrate_bricks_kernel(const float *__restrict__ depth, void *__restrict__ vol,
-                                                               const IntegrateParams P, const int *__restrict__ list,
-                                                               const int *__restrict__ count,
+                                                               const IntegrateParams P, const int *list, const int *count,
                                                                uint8_t *__restrict__ neg_flags,
                                                                unsigned long long *__restrict__ stats,
                                                                uint8_t *__restrict__ sat,
                                                                unsigned long long *neg_masks) {
     __shared__ Pose q;
     const int tid = threadIdx.x, lane = tid & 31;
+    allow_next_kernel();
+    wait_previous_kernel();
     if (tid < 12) {
         float v;
         if (P.dpose) v = tid < 9 ? P.dpose->R_inv[tid] : P.dpose->t[tid - 9];
@@ -525,28 +539,34 @@ size_t depth_max_floats(int W, int H) {
     return n;
 }
 
-// The max pyramid, then the min pyramid (same layout).
+// Level 0's largest and smallest depths, then levels 1-4's largest, then their
+// smallest.
 DepthMaxPyramid depth_max_layout(float *base, int W, int H) {
     DepthMaxPyramid p;
-    const size_t n = depth_max_floats(W, H);
-    size_t off = 0;
+    const size_t l0 = (size_t)div_up(W, 16) * div_up(H, 16), upper = depth_max_floats(W, H) - l0;
+    size_t off = 2 * l0;
     for (int l = 0; l < kDepthMaxLevels; ++l) {
         const int t = 16 << l;
         p.tiles_x[l] = (W + t - 1) / t;
-        p.level[l] = base + off;
-        p.level_min[l] = base + n + off;
-        off += (size_t)p.tiles_x[l] * ((H + t - 1) / t);
+        p.level[l] = l ? base + off : base;
+        p.level_min[l] = l ? base + off + upper : base + l0;
+        if (l) off += (size_t)p.tiles_x[l] * ((H + t - 1) / t);
     }
     return p;
 }
 
+// Scratch of an integration: the depth pyramids, then (256-byte aligned) the
+// counter of the surviving bricks, and their list.
+static size_t brick_counter_offset(int W, int H) {
+    return ((2 * depth_max_floats(W, H) * sizeof(float)) + 255) & ~size_t(255);
+}
+
 int launch_depth_max(const float *depth_scaled, int W, int H, float *scratch, cudaStream_t stream) {
     DepthMaxPyramid pyr = depth_max_layout(scratch, W, H);
-    // levels >= 1 are atomicMax / atomicMin targets: start them at +0 / kNoDepth
-    const size_t l0 = (size_t)pyr.tiles_x[0] * ((H + 15) / 16), n = depth_max_floats(W, H);
-    cudaError_t e = cudaMemsetAsync(scratch + l0, 0, (n - l0) * sizeof(float), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(scratch + n + l0, 0x7f, (n - l0) * sizeof(float), stream);
-    if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "depth_max: %s", cudaGetErrorString(e));
+    // levels >= 1 are targets of atomicMax, and the bricks are counted from 0
+    char *const from = reinterpret_cast<char *>(pyr.level[1]);
+    char *const to = reinterpret_cast<char *>(scratch) + brick_counter_offset(W, H) + sizeof(int);
+    TDE_CUDA(cudaMemsetAsync(from, 0, (size_t)(to - from), stream), "depth_max");
     dim3 grid(div_up(W, 16), div_up(H, 16));
     depth_max_kernel<<<grid, 256, 0, stream>>>(depth_scaled, W, H, pyr);
     return check_launch("depth_max");
@@ -570,26 +590,21 @@ int launch_brick_masks(const uint8_t *neg_flags, const tde_round_buffer &rb, uns
 }
 
 size_t integrate_scratch_bytes(int W, int H, const tde_round_buffer &rb) {
-    // depth max and min pyramids, then (aligned) the brick counter and the brick list
-    const size_t dm = ((2 * depth_max_floats(W, H) * sizeof(float)) + 255) & ~size_t(255);
-    return dm + 256 + brick_count(rb) * sizeof(int);
+    return brick_counter_offset(W, H) + 256 + brick_count(rb) * sizeof(int);
 }
 
 int launch_integrate(const float *depth_scaled, void *volume, int format, const IntegrateParams &P, void *scratch,
                      uint8_t *neg_flags, unsigned long long *stats, cudaStream_t stream, uint8_t *sat_flags,
-                     unsigned long long *neg_masks) {
+                     unsigned long long *neg_masks, bool chained) {
     const int W = P.intr.cols, H = P.intr.rows;
     float *dmax = static_cast<float *>(scratch);
-    const size_t dm = ((2 * depth_max_floats(W, H) * sizeof(float)) + 255) & ~size_t(255);
+    const size_t dm = brick_counter_offset(W, H);
     int *count = reinterpret_cast<int *>(static_cast<char *>(scratch) + dm);
     int *list = reinterpret_cast<int *>(static_cast<char *>(scratch) + dm + 256);
     const DepthMaxPyramid pyr = depth_max_layout(dmax, W, H);
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), stream);
-    if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "integrate: %s", cudaGetErrorString(e));
     const unsigned nb = (unsigned)brick_count(P.rb);
-    cull_bricks_kernel<<<div_up(nb, 256u), 256, 0, stream>>>(P, pyr, list, count, sat_flags);
-    int st = check_launch("integrate/cull");
-    if (st) return st;
+    TDE_TRY(launch_chained("integrate/cull", chained, cull_bricks_kernel<false>, div_up(nb, 256u), 256, stream, P, pyr, list,
+                           count, sat_flags));
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -597,9 +612,8 @@ int launch_integrate(const float *depth_scaled, void *volume, int format, const 
     // 0.0655 ms, 6: 0.0696, 8: 0.0658, 12: 0.0658)
     const unsigned blocks = std::min(div_up(nb, 8u), (unsigned)(sms * kIntBlocksPerSM));
     return dispatch_format(format, [&](auto F) {
-        integrate_bricks_kernel<decltype(F)::value><<<blocks, 256, 0, stream>>>(depth_scaled, volume, P, list, count,
-                                                                               neg_flags, stats, sat_flags, neg_masks);
-        return check_launch("integrate_tsdf");
+        return launch_chained("integrate_tsdf", chained, integrate_bricks_kernel<decltype(F)::value>, blocks, 256, stream,
+                              depth_scaled, volume, P, list, count, neg_flags, stats, sat_flags, neg_masks);
     });
 }
 
@@ -616,12 +630,10 @@ int launch_integrate_colors(tde_color *col, const uint8_t *rgb, const float *vma
     int st = check_launch("integrate_colors/model distances");
     if (st) return st;
     if ((st = launch_depth_max(dist, W, H, reinterpret_cast<float *>(iscratch), stream))) return st;
-    const size_t dm = ((2 * depth_max_floats(W, H) * sizeof(float)) + 255) & ~size_t(255);
+    const size_t dm = brick_counter_offset(W, H);
     int *count = reinterpret_cast<int *>(iscratch + dm);
     int *list = reinterpret_cast<int *>(iscratch + dm + 256);
     const DepthMaxPyramid pyr = depth_max_layout(reinterpret_cast<float *>(iscratch), W, H);
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), stream);
-    if (e != cudaSuccess) return set_error(TDE_ERR_CUDA, "integrate_colors: %s", cudaGetErrorString(e));
     const unsigned nb = (unsigned)brick_count(P.rb);
     cull_bricks_kernel<true><<<div_up(nb, 256u), 256, 0, stream>>>(P, pyr, list, count, nullptr);
     if ((st = check_launch("integrate_colors/cull"))) return st;

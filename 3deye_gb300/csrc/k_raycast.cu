@@ -258,6 +258,8 @@ __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__rest
                                                      float *__restrict__ nmap, const __grid_constant__ RayParams p) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
+    allow_next_kernel();
+    wait_previous_kernel();
     const int x = blockIdx.x * kRayBlockCols + warp * 8 + (lane & 7);
     const int y = blockIdx.y * kRayBlockRows + (lane >> 3);
     const int W = p.intr.cols, H = p.intr.rows;
@@ -446,10 +448,12 @@ __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__rest
 // resize_vertex_map / resize_normal_map (absent from the reference; named at
 // common/inc/constants.h:175-176): 2x2 block mean, all four valid.
 template <bool NORMAL>
-__global__ void resize_map_kernel(const float *__restrict__ src, float *__restrict__ dst, int sc, int sr) {
+__global__ void resize_map_kernel(const float *src, float *dst, int sc, int sr) {
     const int dc = sc >> 1, dr = sr >> 1;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
+    allow_next_kernel();
+    wait_previous_kernel();
     if (x >= dc || y >= dr) return;
     const float qnan = __int_as_float(0x7fffffff);
     float sx = 0.f, sy = 0.f, sz = 0.f;
@@ -578,8 +582,8 @@ __global__ void transform_maps_kernel(const float *__restrict__ vs, const float 
 
 int launch_raycast(const void *volume, int format, float *vmap, float *nmap, const tde_point3f &t,
                    const tde_matrix3f &R, float trunc, const tde_intrinsics &intr, const tde_round_buffer &rb,
-                   const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags, const unsigned long long *neg_masks,
-                   cudaStream_t stream, unsigned *touched) {
+                   const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags,
+                   const unsigned long long *neg_masks, cudaStream_t stream, bool chained, unsigned *touched) {
     RayParams p;
     p.dpose = dpose;
     p.neg_flags = neg_flags;
@@ -603,18 +607,16 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
             return neg_masks ? raycast_kernel<FM, FLAG_MASKS, ST>
                              : neg_flags ? raycast_kernel<FM, FLAG_BYTES, ST> : raycast_kernel<FM, FLAG_NONE, ST>;
         };
-        const auto k = touched ? kernel(std::true_type{}) : kernel(std::false_type{});
-        k<<<grid, block, 0, stream>>>(volume, vmap, nmap, p);
-        return check_launch("raycast");
+        return launch_chained("raycast", chained, touched ? kernel(std::true_type{}) : kernel(std::false_type{}), grid,
+                              block, stream, volume, vmap, nmap, p);
     });
 }
 
 int launch_resize_map(const float *src, float *dst, int sc, int sr, bool normal, cudaStream_t stream) {
     dim3 block(32, 8);
     dim3 grid(div_up(sc >> 1, 32), div_up(sr >> 1, 8));
-    if (normal) resize_map_kernel<true><<<grid, block, 0, stream>>>(src, dst, sc, sr);
-    else resize_map_kernel<false><<<grid, block, 0, stream>>>(src, dst, sc, sr);
-    return check_launch("resize_map");
+    return launch_chained("resize_map", true, normal ? resize_map_kernel<true> : resize_map_kernel<false>, grid, block,
+                          stream, src, dst, sc, sr);
 }
 
 int launch_resize_model_maps(const float *v0, const float *n0, float *v1, float *n1, float *v2, float *n2, int c0,

@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stddef.h>
 #include <type_traits>
+#include <utility>
 
 #include "../../include/tde_capi.h"
 
@@ -50,6 +51,34 @@ inline int cuda_fail(cudaError_t e, const char *what) {
         int s_ = (call);             \
         if (s_ != TDE_OK) return s_; \
     } while (0)
+
+// ---------------------------------------------------------------------------
+// Chained launches (programmatic stream serialisation): a kernel's blocks come up
+// while the kernel before it on the stream finishes, and wait_previous_kernel
+// returns once that one has completed and its writes are visible.  Every block
+// of a chained kernel waits, so its own completion implies its predecessor's;
+// what precedes the wait touches no memory, and buffers that the predecessor
+// writes are not read through the read-only path (whose loads the compiler may
+// move over the wait).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+int launch_chained(const char *what, bool chained, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream,
+                   Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    TDE_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...), what);
+    return check_launch(what);
+}
 
 // ---------------------------------------------------------------------------
 // OpenCL min/max for floats: max(x, y) = x < y ? y : x.

@@ -28,7 +28,8 @@ struct IntegrateParams {
 // Max observed depth per screen tile: level l has (16 << l)-pixel tiles.
 constexpr int kDepthMaxLevels = 5;
 // Per screen tile: the largest scaled depth (level) and the smallest
-// non-zero one (level_min, kNoDepth where the tile has none).
+// non-zero one (level_min, kNoDepth where the tile has none; from level 1 as the
+// distance of its bits below kNoDepth's).
 struct DepthMaxPyramid {
     float *level[kDepthMaxLevels];
     float *level_min[kDepthMaxLevels];
@@ -64,8 +65,9 @@ int launch_depth_max(const float *depth_scaled, int W, int H, float *scratch, cu
 // neg_flags (may be null): per physical brick, set to 1 when a write leaves a
 // negative value there; a 0 therefore guarantees the brick holds no negative
 // TSDF value.
-// Scratch of one integration: the depth max / min pyramids (filled by
-// launch_depth_max at its start) followed by the surviving-brick list.
+// Scratch of one integration: the depth max / min pyramids followed by the
+// surviving-brick counter and list.  launch_depth_max fills the pyramids and
+// clears the counter: one call of it before each integration.
 size_t integrate_scratch_bytes(int W, int H, const tde_round_buffer &rb);
 // sat_flags (may be null): per logical brick (brick_count bytes, zero when a
 // pipeline starts or the round buffer moves), 1 when the last integration
@@ -75,10 +77,11 @@ size_t integrate_scratch_bytes(int W, int H, const tde_round_buffer &rb);
 // so it is not swept.
 // neg_masks (may be null; neg_flags is set too then): per physical super-brick
 // (superbrick_count words) the flags of its bricks, bit x + 4 y + 16 z of the
-// brick's place in it.
+// brick's place in it.  chained: launch_chained (the pipeline does not: blocks
+// that wait hold the slots of the next frame's preprocessing beside them).
 int launch_integrate(const float *depth_scaled, void *volume, int format, const IntegrateParams &P, void *scratch,
                      uint8_t *neg_flags, unsigned long long *stats, cudaStream_t stream, uint8_t *sat_flags = nullptr,
-                     unsigned long long *neg_masks = nullptr);
+                     unsigned long long *neg_masks = nullptr, bool chained = true);
 // neg_masks from neg_flags.
 int launch_brick_masks(const uint8_t *neg_flags, const tde_round_buffer &rb, unsigned long long *neg_masks,
                        cudaStream_t stream);

@@ -170,3 +170,52 @@ def test_empty_bricks_are_skipped_exactly(cuda, tde, orc, voxels, fmt):
     check(q)
     q.process(depths[6])
     check(q)
+
+
+@pytest.mark.parametrize("cols,rows,voxels", [(1, 1, 16), (16, 17, 20), (33, 300, 64), (611, 457, 48)])
+def test_integrate_takes_undefined_scratch_on_any_stream(cuda, tde, orc, cols, rows, voxels):
+    """tde_integrate_tsdf_ex from scratch of zeros and of ones, enqueued on a
+    stream of the caller's right behind the frame's scaling and followed by the
+    raycast: the oracle's volume and maps, bit for bit."""
+    import torch
+    syn = importlib.import_module("3deye_gb300.synth")
+    cfg = syn.small_config("c1", frames=2, cols=cols, rows=rows, voxels=voxels, fmt=1)
+    scene, traj = syn.make_scene(cfg, 1000), syn.make_trajectory(cfg, 2000)
+    oi = orc.Intr(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cols, rows)
+    it = tde.Intrinsics(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cols, rows)
+    depth = orc.apply_noise(orc.render_depth(scene, traj[0], oi), 3000, 0)
+    R, t = traj[0][:9].reshape(3, 3).astype(np.float32), traj[0][9:].astype(np.float32)
+    ob = orc.make_rb((voxels,) * 3, (cfg.volume_m,) * 3, (3, 9, 14))
+    rb = tde.round_buffer((voxels,) * 3, (cfg.volume_m,) * 3, (3, 9, 14))
+    cell = np.full(3, cfg.cell, np.float32)
+    ref = np.zeros(orc.volume_bytes(1, ob), np.uint8)
+    for _ in range(2):
+        orc.integrate(orc.scale_depth(depth, oi), ref, 1, cfg.trunc_m, np.ascontiguousarray(R.T), t, oi, cell, ob)
+    vmo, nmo = orc.raycast(ref, 1, ob, oi, R, t, cfg.trunc_m, cell)
+    L, V, I, F = tde.lib, C.c_void_p, C.c_int, C.c_float
+    pM, pV, pI, pRB = (C.POINTER(k) for k in (tde.Matrix3f, tde.Point3f, tde.Intrinsics, tde.RoundBuffer))
+    L.tde_integrate_tsdf_scratch_bytes.restype = C.c_size_t
+    L.tde_integrate_tsdf_scratch_bytes.argtypes = [I, I, pRB]
+    L.tde_integrate_tsdf_ex.argtypes = [V, V, I, F, pM, pV, pI, pV, pRB, I, V, C.c_size_t, V, V]
+    sb = L.tde_integrate_tsdf_scratch_bytes(cols, rows, C.byref(rb))
+    d = torch.from_numpy(depth.view(np.int16)).cuda()
+    Ri, Rm, tt, cs = tde.mat3(R.T.copy()), tde.mat3(R), tde.vec3(t), tde.vec3(cell)
+    for fill in (0, 255):
+        s = torch.cuda.Stream()
+        scratch = torch.full((sb,), fill, dtype=torch.uint8, device="cuda")
+        vol = torch.zeros(ref.size, dtype=torch.uint8, device="cuda")
+        sd = torch.empty((rows, cols), device="cuda")
+        maps = torch.empty((2, rows, cols, 3), device="cuda")
+        s.wait_stream(torch.cuda.current_stream())
+        for _ in range(2):
+            tde.check(tde.lib.tde_scale_depth(d.data_ptr(), sd.data_ptr(), C.byref(it), s.cuda_stream))
+            tde.check(tde.lib.tde_integrate_tsdf_ex(sd.data_ptr(), vol.data_ptr(), 1, cfg.trunc_m, C.byref(Ri),
+                                                    C.byref(tt), C.byref(it), C.byref(cs), C.byref(rb), 128,
+                                                    scratch.data_ptr(), sb, None, s.cuda_stream))
+        tde.check(tde.lib.tde_raycast(vol.data_ptr(), 1, maps[0].data_ptr(), maps[1].data_ptr(), C.byref(tt),
+                                      C.byref(Rm), cfg.trunc_m, C.byref(it), C.byref(rb), C.byref(cs), s.cuda_stream))
+        s.synchronize()
+        assert np.array_equal(vol.cpu().numpy(), ref)
+        got = maps.cpu().numpy()
+        for a, b in zip(got, (vmo, nmo)):
+            assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.nan_to_num(a), np.nan_to_num(b))
