@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(THREADS) icp_step_kernel(const IcpArgs a, IcpS
     __shared__ IcpPose P;
     __shared__ float red[THREADS / 32][32];
     __shared__ ffl Rs[9], ts[3];  // this launch's pose (float-float)
+    __shared__ SolveTerms sh;
     __shared__ unsigned ticket;
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(THREADS) icp_step_kernel(const IcpArgs a, IcpS
         if (iter > 0) {
             inliers = __shfl_sync(0xffffffffu, (int)whole, 27);
             ffl o, xl;
-            ok = warp_solve_step(term, Rs, ts, lane, o, xl) && inliers >= kIcpMinInliers;
+            ok = warp_solve_step(term, Rs, ts, lane, sh, o, xl) && inliers >= kIcpMinInliers;
             if (ok) pv = o;
             __syncwarp();
             if (lane < 9) Rs[lane] = pv;
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(THREADS) icp_step_kernel(const IcpArgs a, IcpS
     if (warp != 0) return;
     const int inliers = __shfl_sync(0xffffffffu, (int)whole, 27);
     ffl o, xl;
-    const bool ok = warp_solve_step(term, Rs, ts, lane, o, xl) && inliers >= kIcpMinInliers;
+    const bool ok = warp_solve_step(term, Rs, ts, lane, sh, o, xl) && inliers >= kIcpMinInliers;
     // accept the estimate (in FP64), or keep the start pose when any solve failed
     const bool lost = !ok || (*(volatile int *)&st->status & kIcpStatusSolveFailed);
     double nv = 0.0;
@@ -442,6 +443,7 @@ __global__ void __launch_bounds__(THREADS) icp_step_kernel(const IcpArgs a, IcpS
 __global__ void icp_solve_kernel(const double *__restrict__ sums, int n, double *__restrict__ pose,
                                  double *__restrict__ x, int *__restrict__ okv) {
     __shared__ ffl Rs[4][9], ts[4][3];
+    __shared__ SolveTerms sh[4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * 4 + warp;
     if (i >= n) return;  // whole warps leave together
@@ -451,7 +453,7 @@ __global__ void icp_solve_kernel(const double *__restrict__ sums, int n, double 
     else if (lane < 12) ts[warp][lane - 9] = ffl_from_double(pv);
     __syncwarp();
     ffl o, xl;
-    const bool ok = warp_solve_step(term, Rs[warp], ts[warp], lane, o, xl);
+    const bool ok = warp_solve_step(term, Rs[warp], ts[warp], lane, sh[warp], o, xl);
     if (lane < 12) pose[(size_t)12 * i + lane] = ok ? ffl_to_double(o) : pv;
     if (ok && lane < 6) x[(size_t)6 * i + lane] = ffl_to_double(xl);
     if (lane == 0) okv[i] = ok;

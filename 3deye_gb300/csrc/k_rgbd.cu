@@ -18,6 +18,7 @@
 // Built with -fmad=false: the pair tests and row values are the same IEEE
 // operations as the CPU oracle (oracle/oracle_rgbd.c), explicit fused
 // multiply-adds written out on both sides.
+#include <atomic>
 #include <cmath>
 #include <utility>
 
@@ -174,11 +175,18 @@ struct Level {
 };
 
 // One piece of R' = K R K^-1, t' = K t (FP64, explicit fused operations,
-// then float) and of the float pose M: row t of R' for t < 3, t' for t = 3;
-// threads 4..15 convert pose entry t - 4.  Threads 0..15 of a block run it
-// side by side (the FP64 pipe is narrow: one thread doing everything
-// serialises several microseconds of dependent FP64 work).
-__device__ __forceinline__ void projective_part(int t, const double *pose, const Level &L, float *proj, float *M) {
+// then float) and of the float pose M: row t of R' for t < 3, t' for t = 3,
+// M for t = 4 (by lanes).  Five warps of a block run it side by
+// side: the FP64 pipe's latency makes each piece some 600 cycles, and as lanes of one
+// warp, which takes its branches in turn, they took 3000.
+__device__ __forceinline__ void projective_part(int t, int lane, const double *pose, const Level &L, float *proj,
+                                                float *M) {
+    if (t < 0 || t > 4) return;
+    if (t == 4) {
+        if (lane < 12) M[lane] = (float)pose[lane];
+        return;
+    }
+    if (lane != 0) return;
     const double fx = L.fx, fy = L.fy, cx = L.cx, cy = L.cy;
     const double *R = pose, *tv = pose + 9;
     if (t < 3) {
@@ -205,8 +213,6 @@ __device__ __forceinline__ void projective_part(int t, const double *pose, const
         proj[9] = (float)__fma_rn(fx, tv[0], __dmul_rn(cx, tv[2]));
         proj[10] = (float)__fma_rn(fy, tv[1], __dmul_rn(cy, tv[2]));
         proj[11] = (float)tv[2];
-    } else if (t < 16) {
-        M[t - 4] = (float)pose[t - 4];
     }
 }
 
@@ -235,31 +241,43 @@ __device__ __forceinline__ bool find_pair(const Level &L, const float *P, int u,
     return true;
 }
 
-// The previous frame's depth at K pixels (raster indices i[k]; entries at or
-// past W*H are not pixels): independent of the pose, so the step kernels
-// issue these loads before waiting for the previous step.
+// K pixels of the previous frame (raster indices i[k]; entries at or past W*H
+// are not pixels) with their columns, rows and depths: independent of the pose,
+// so the step kernels form and load these before waiting for the previous step.
 template <int K>
-__device__ __forceinline__ void load_depths(const Level &L, const int (&i)[K], float (&z)[K]) {
+struct Pixels {
+    int i[K];
+    float u[K], v[K], z[K];
+};
+template <int K>
+__device__ __forceinline__ void load_pixels(const Level &L, Pixels<K> &q) {
     const int npix = L.W * L.H;
 #pragma unroll
-    for (int k = 0; k < K; ++k) z[k] = i[k] < npix ? __ldg(L.Dp + i[k]) : 0.f;
+    for (int k = 0; k < K; ++k) {
+        const int row = q.i[k] / L.W;
+        q.z[k] = q.i[k] < npix ? __ldg(L.Dp + q.i[k]) : 0.f;
+        q.u[k] = (float)(q.i[k] - row * L.W);
+        q.v[k] = (float)row;
+    }
 }
 
-// find_pair for the K pixels of load_depths (depths z[k]): the projections,
+// find_pair for the K pixels of load_pixels: the projections,
 // then the gathers of every candidate issued together, then the tests -- the
 // same operations and results as find_pair, with K load chains in flight
 // instead of one.  Bit k of the result is set for a kept pair; j[k], r[k] and
 // the current frame's derivatives gx[k], gy[k] at j[k] are valid for those.
 template <int K>
-__device__ __forceinline__ unsigned find_pairs(const Level &L, const float *P, const int (&i)[K], int (&j)[K],
-                                               float (&r)[K], const float (&z)[K], float (&gx)[K], float (&gy)[K]) {
+__device__ __forceinline__ unsigned find_pairs(const Level &L, const float *P, const Pixels<K> &q, int (&j)[K],
+                                               float (&r)[K], float (&gx)[K], float (&gy)[K]) {
+    const int (&i)[K] = q.i;
+    const float (&z)[K] = q.z;
     float pz[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         j[k] = -1;
         pz[k] = 0.f;
         if (!depth_ok(z[k], L.maxd)) continue;
-        const float fu = (float)(i[k] % L.W), fv = (float)(i[k] / L.W);
+        const float fu = q.u[k], fv = q.v[k];
         const float px = __fmaf_rn(z[k], __fmaf_rn(P[1], fv, __fmaf_rn(P[0], fu, P[2])), P[9]);
         const float py = __fmaf_rn(z[k], __fmaf_rn(P[4], fv, __fmaf_rn(P[3], fu, P[5])), P[10]);
         pz[k] = __fmaf_rn(z[k], __fmaf_rn(P[7], fv, __fmaf_rn(P[6], fu, P[8])), P[11]);
@@ -294,9 +312,9 @@ __device__ __forceinline__ unsigned find_pairs(const Level &L, const float *P, c
 }
 
 // The 7-vector (C0..C5, -w r) of a kept pair; M = R row-major, t (float).
-__device__ __forceinline__ void pair_row(const Level &L, const float *M, int u, int v, float z, float gx, float gy,
+__device__ __forceinline__ void pair_row(const Level &L, const float *M, float u, float v, float z, float gx, float gy,
                                          float r, float sigma, float ifx, float ify, float row[7]) {
-    const float xn = __fmul_rn((float)u - L.cx, ifx), yn = __fmul_rn((float)v - L.cy, ify);
+    const float xn = __fmul_rn(u - L.cx, ifx), yn = __fmul_rn(v - L.cy, ify);
     const float X = __fmul_rn(z, xn), Y = __fmul_rn(z, yn);
     const float Px = __fmaf_rn(M[2], z, __fmaf_rn(M[1], Y, __fmul_rn(M[0], X))) + M[9];
     const float Py = __fmaf_rn(M[5], z, __fmaf_rn(M[4], Y, __fmul_rn(M[3], X))) + M[10];
@@ -317,6 +335,77 @@ __device__ __forceinline__ void pair_row(const Level &L, const float *M, int u, 
     row[6] = -__fmul_rn(w, r);
 }
 
+// Kept count and sum of squared differences (integers: exact; 128 squares of
+// at most 255 stay below 2^23) of a warp's K pixels a lane.
+template <int K>
+__device__ __forceinline__ void count_pairs(unsigned kept, const float (&r)[K], unsigned &n, unsigned &r2) {
+    static_assert(K * 32 * 65025ull < (1ull << 32), "a warp's sum of squares");
+    n = __popc(kept);
+    r2 = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if ((kept >> k) & 1u) {
+            const int ri = (int)r[k];
+            r2 += (unsigned)(ri * ri);
+        }
+    n = __reduce_add_sync(0xffffffffu, n);
+    r2 = __reduce_add_sync(0xffffffffu, r2);
+}
+
+__device__ __forceinline__ float sigma_of(unsigned long long n, unsigned long long s) {
+    return n ? __fsqrt_rn((float)((double)s / (double)n)) : 0.f;
+}
+
+// The 27 terms and the count of a thread's kept pairs, in its pixels' order.
+template <int K>
+__device__ __forceinline__ void pair_sums(const Level &L, const float *M, unsigned kept, const Pixels<K> &q,
+                                          const float (&gx)[K], const float (&gy)[K], const float (&r)[K], float sigma,
+                                          float (&acc)[32]) {
+    const float ifx = __frcp_rn(L.fx), ify = __frcp_rn(L.fy);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) acc[k] = 0.f;  // 4 unused
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        if (!((kept >> k) & 1u)) continue;
+        float row[7];
+        pair_row(L, M, q.u[k], q.v[k], q.z[k], gx[k], gy[k], r[k], sigma, ifx, ify, row);
+        int t = 0;
+#pragma unroll
+        for (int a = 0; a < 6; ++a)
+#pragma unroll
+            for (int b = a; b < 7; ++b) {
+                acc[t] = __fmaf_rn(row[a], row[b], acc[t]);
+                ++t;
+            }
+        acc[27] += 1.f;
+    }
+}
+
+// The pose as the solve reads it, by the lanes of one warp (FP64 conversions,
+// 1000 cycles one after the other: early, where the chain does not wait for them).
+__device__ __forceinline__ void pose_to_ff(const double *pose, ffl *Rs, ffl *ts, int lane) {
+    if (lane < 9) Rs[lane] = ffl_from_double(pose[lane]);
+    else if (lane < 12) ts[lane - 9] = ffl_from_double(pose[lane]);
+}
+
+// Warp 0: the 28 totals of the warps' sums (in order; `warps` of them have a
+// block, the others' zeros change nothing), the solve from pose_to_ff's pose, and
+// the pose moved in place.  Returns the status bit.
+__device__ __forceinline__ int solve_totals(const ffl (*redf)[28], int warps, double *pose, const ffl *Rs,
+                                            const ffl *ts, int lane) {
+    __shared__ SolveTerms sh;
+    ffl term{0.f, 0.f};
+    if (lane < 28) {
+        term = redf[0][lane];
+        for (int w = 1; w < warps; ++w) term = ffl_add(term, redf[w][lane]);
+    }
+    const float count = __shfl_sync(0xffffffffu, term.hi, 27);  // an integer below 2^24: exact
+    ffl o, xl;
+    const bool ok = count >= (float)kIcpMinInliers && warp_solve_step(term, Rs, ts, lane, sh, o, xl);
+    if (ok && lane < 12) pose[lane] = ffl_to_double(o);
+    return ok ? 2 : 1;
+}
+
 // Pass 1: kept count and sum of squared differences per block.
 __global__ void __launch_bounds__(kOdoThreads) residual_kernel(const Level L, const double *__restrict__ pose,
                                                             unsigned long long *__restrict__ partials) {
@@ -326,39 +415,29 @@ __global__ void __launch_bounds__(kOdoThreads) residual_kernel(const Level L, co
     // the second pass (launched with programmatic serialisation) may start its
     // pose-independent loads now
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    int idx[kPix], j[kPix];
-    float r[kPix], z[kPix], gx[kPix], gy[kPix];
+    Pixels<kPix> q;
+    int j[kPix];
+    float r[kPix], gx[kPix], gy[kPix];
 #pragma unroll
-    for (int k = 0; k < kPix; ++k) idx[k] = blockIdx.x * kOdoThreads * kPix + k * kOdoThreads + threadIdx.x;
-    load_depths<kPix>(L, idx, z);
+    for (int k = 0; k < kPix; ++k) q.i[k] = blockIdx.x * kOdoThreads * kPix + k * kOdoThreads + threadIdx.x;
+    load_pixels<kPix>(L, q);
     // launched with programmatic serialisation after the previous step's
     // second pass: its pose update and this pass's writes of the partials
     // that pass read come after this wait (0.507 against 0.514 ms per frame
     // with graphs, 0.551 against 0.595 eager, than a plain launch)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (threadIdx.x < 16) projective_part(threadIdx.x, pose, L, P, M);
+    projective_part(threadIdx.x >> 5, threadIdx.x & 31, pose, L, P, M);
     if (threadIdx.x == 0) {
         s_n = 0;
         s_r2 = 0ull;
     }
     __syncthreads();
-    unsigned n = 0;
-    unsigned long long r2 = 0;  // squared integer differences: exact
-    const unsigned kept = find_pairs<kPix>(L, P, idx, j, r, z, gx, gy);
-#pragma unroll
-    for (int k = 0; k < kPix; ++k)
-        if ((kept >> k) & 1u) {
-            ++n;
-            const int ri = (int)r[k];
-            r2 += (unsigned long long)(ri * ri);
-        }
-    for (int o = 16; o > 0; o >>= 1) {
-        n += __shfl_down_sync(0xffffffffu, n, o);
-        r2 += __shfl_down_sync(0xffffffffu, r2, o);
-    }
+    unsigned n, r2;
+    const unsigned kept = find_pairs<kPix>(L, P, q, j, r, gx, gy);
+    count_pairs<kPix>(kept, r, n, r2);
     if ((threadIdx.x & 31) == 0) {
         atomicAdd(&s_n, n);
-        atomicAdd(&s_r2, r2);
+        atomicAdd(&s_r2, (unsigned long long)r2);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -386,54 +465,51 @@ __global__ void __launch_bounds__(kOdoThreads) lsm_kernel(const Level L, double 
     __shared__ float P[12], M[12];
     __shared__ float s_sigma;
     __shared__ float red[NW][32];
+    __shared__ ffl Rs[9], ts[3];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    int idx[kPix], j[kPix];
-    float r[kPix], z[kPix], gx[kPix], gy[kPix];
+    Pixels<kPix> q;
+    int j[kPix];
+    float r[kPix], gx[kPix], gy[kPix];
 #pragma unroll
-    for (int k = 0; k < kPix; ++k) idx[k] = blockIdx.x * kOdoThreads * kPix + k * kOdoThreads + tid;
-    load_depths<kPix>(L, idx, z);
+    for (int k = 0; k < kPix; ++k) q.i[k] = blockIdx.x * kOdoThreads * kPix + k * kOdoThreads + tid;
+    load_pixels<kPix>(L, q);
     // the first pass's partials and the pose are complete past this point
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == 0) {
         unsigned long long n = 0, s = 0;
-        for (int b = lane; b < nres; b += 32) {
-            n += res_partials[2 * b];
-            s += res_partials[2 * b + 1];
+        constexpr int kAhead = 5;  // loads in flight: 160 blocks, as 640x480 has
+        for (int b0 = lane; b0 < nres; b0 += 32 * kAhead) {
+            unsigned long long bn[kAhead], bs[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                const bool in = b0 + 32 * k < nres;
+                bn[k] = in ? res_partials[2 * (b0 + 32 * k)] : 0;
+                bs[k] = in ? res_partials[2 * (b0 + 32 * k) + 1] : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                n += bn[k];
+                s += bs[k];
+            }
         }
         for (int o = 16; o > 0; o >>= 1) {
             n += __shfl_xor_sync(0xffffffffu, n, o);
             s += __shfl_xor_sync(0xffffffffu, s, o);
         }
         if (lane == 0) {
-            s_sigma = n ? __fsqrt_rn((float)((double)s / (double)n)) : 0.f;
+            s_sigma = sigma_of(n, s);
             if (sigma_out && blockIdx.x == 0) *sigma_out = s_sigma;
         }
-    } else if (warp == 1 && lane < 16) {
-        projective_part(lane, pose, L, P, M);
+    } else if (SOLVE && warp == 6) {
+        pose_to_ff(pose, Rs, ts, lane);
+    } else {
+        projective_part(warp - 1, lane, pose, L, P, M);
     }
     __syncthreads();
-    const float sigma = s_sigma;
-    const float ifx = __frcp_rn(L.fx), ify = __frcp_rn(L.fy);
-    float acc[32];  // 27 terms and the count; 4 unused
-#pragma unroll
-    for (int k = 0; k < 32; ++k) acc[k] = 0.f;
-    const unsigned kept = find_pairs<kPix>(L, P, idx, j, r, z, gx, gy);
-#pragma unroll
-    for (int k = 0; k < kPix; ++k) {
-        if (!((kept >> k) & 1u)) continue;
-        float row[7];
-        pair_row(L, M, idx[k] % L.W, idx[k] / L.W, z[k], gx[k], gy[k], r[k], sigma, ifx, ify, row);
-        int t = 0;
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-            for (int b = a; b < 7; ++b) {
-                acc[t] = __fmaf_rn(row[a], row[b], acc[t]);
-                ++t;
-            }
-        acc[27] += 1.f;
-    }
+    float acc[32];
+    const unsigned kept = find_pairs<kPix>(L, P, q, j, r, gx, gy);
+    pair_sums<kPix>(L, M, kept, q, gx, gy, r, s_sigma, acc);
     // warp totals (transpose butterfly: lane l holds term l), then the warps
     // in order: float sums in a fixed order
     red[warp][lane] = warp_transpose_reduce(acc, lane);
@@ -457,27 +533,146 @@ __global__ void __launch_bounds__(kOdoThreads) lsm_kernel(const Level L, double 
     __shared__ ffl redf[NW][28];
     if (lane < 28) {
         ffl v{0.f, 0.f};
-        for (int b = warp; b < (int)gridDim.x; b += NW) v = ffl_add_f(v, __ldcg(partials + (size_t)b * 28 + lane));
+        constexpr int kAhead = 10;  // loads in flight; a block past the end adds nothing
+        for (int b0 = warp; b0 < (int)gridDim.x; b0 += NW * kAhead) {
+            float p[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+                p[k] = b0 + NW * k < (int)gridDim.x ? __ldcg(partials + (size_t)(b0 + NW * k) * 28 + lane) : 0.f;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+                if (b0 + NW * k < (int)gridDim.x) v = ffl_add_f(v, p[k]);
+        }
         redf[warp][lane] = v;
     }
     __syncthreads();
     if (warp != 0) return;
     if (lane == 0) *counter = 0u;
-    __shared__ ffl Rs[9], ts[3];
-    ffl term{0.f, 0.f};
-    if (lane < 28) {
-        term = redf[0][lane];
-        for (int w = 1; w < NW; ++w) term = ffl_add(term, redf[w][lane]);
+    const int bit = solve_totals(redf, min(NW, (int)gridDim.x), pose, Rs, ts, lane);
+    if (lane == 0) *status |= bit;
+}
+
+// ---- the coarse levels in one cluster ----
+// Each step of a small level is a chain of latencies (two launches, the pose's
+// FP64 arithmetic twice, two gathers, a ticket, the solve: 15 us at 80x60 as at
+// 320x240), so one cluster runs all steps of the levels that it has the warps
+// for: a level's blocks of kOdoThreads x kPix pixels are dealt out by warps, as
+// evenly over the cluster's SMs as they go (a block's 16 warps on one SM wait for
+// each other's issue slots); the counts, then the warps' sums travel through
+// distributed shared memory, with a cluster barrier each, and every block of
+// the cluster adds up and solves for itself -- the same operations on the same
+// bits as the launches, so the same pose.  A step takes 7.8 us.  Levels
+// of more blocks (38 at 320x240) take the launches, 17 us a step: with a level's blocks
+// three to a cluster block they gained nothing here.  640x480, 17 of its 31 steps
+// in the cluster: 500 -> 352 us.
+constexpr int kOdoCluster = 16;  // blocks of the cluster, and most blocks of a level
+
+struct OdoLevels {
+    Level L[TDE_RGBD_MAX_LEVELS];
+    int blocks[TDE_RGBD_MAX_LEVELS], iters[TDE_RGBD_MAX_LEVELS];
+    int n;
+};
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of this block's shared variable in block `rank` of the cluster.
+__device__ __forceinline__ unsigned remote(const void *p, unsigned rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+
+__global__ void __launch_bounds__(kOdoThreads) odo_cluster_kernel(const __grid_constant__ OdoLevels A,
+                                                                  double *__restrict__ pose_out,
+                                                                  int *__restrict__ status_out) {
+    constexpr int NW = kOdoThreads / 32;
+    static_assert(NW == kOdoCluster, "a level's warps dealt evenly: as many a cluster block as the level has blocks");
+    __shared__ float P[12], M[12], s_sigma;
+    __shared__ uint2 counts[kOdoCluster * NW];        // (pairs, sum of squares) by level block and warp
+    __shared__ float sums[kOdoCluster * NW][28];      // by level block and warp
+    __shared__ ffl redf[NW][28], Rs[9], ts[3];
+    __shared__ double pose[12];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned rank = cluster_rank();
+    int status = 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid < 12) pose[tid] = pose_out[tid];
+    cluster_sync();  // every block has started: its shared memory can be written
+    for (int l = 0; l < A.n; ++l) {
+        const Level L = A.L[l];
+        const int nb = A.blocks[l];
+        const bool work = warp < nb;
+        const int g = (int)rank * nb + warp;  // this warp's place among the level's nb * NW
+        Pixels<kPix> q;
+        int j[kPix];
+        float r[kPix], gx[kPix], gy[kPix];
+#pragma unroll
+        for (int k = 0; k < kPix; ++k)
+            q.i[k] = (g / NW) * kOdoThreads * kPix + k * kOdoThreads + (g % NW) * 32 + lane;
+        load_pixels<kPix>(L, q);
+        for (int it = 0; it < A.iters[l]; ++it) {
+            __syncthreads();  // the pose
+            if (warp == 5) pose_to_ff(pose, Rs, ts, lane);
+            else projective_part(warp, lane, pose, L, P, M);
+            __syncthreads();
+            unsigned kept = 0;
+            if (work) {
+                unsigned n, r2;
+                kept = find_pairs<kPix>(L, P, q, j, r, gx, gy);
+                count_pairs<kPix>(kept, r, n, r2);
+                if (lane < kOdoCluster)
+                    asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(remote(&counts[g], lane)),
+                                 "r"(n), "r"(r2)
+                                 : "memory");
+            }
+            cluster_sync();
+            if (warp == 0) {
+                // at most 2^15 pixels here: their squares sum below 2^31
+                unsigned n = 0, s = 0;
+                for (int c = lane; c < kOdoCluster * nb; c += 32) {
+                    n += counts[c].x;
+                    s += counts[c].y;
+                }
+                n = __reduce_add_sync(0xffffffffu, n);
+                s = __reduce_add_sync(0xffffffffu, s);
+                if (lane == 0) s_sigma = sigma_of(n, s);
+            }
+            __syncthreads();
+            if (work) {
+                float acc[32];
+                pair_sums<kPix>(L, M, kept, q, gx, gy, r, s_sigma, acc);
+                const float v = warp_transpose_reduce(acc, lane);
+                if (lane < 28) {
+#pragma unroll
+                    for (int c = 0; c < kOdoCluster; ++c)
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote(&sums[g][lane], c)), "f"(v)
+                                     : "memory");
+                }
+            }
+            cluster_sync();
+            // lsm_kernel's order: a block's warps in turn, then the blocks
+            if (work && lane < 28) {
+                float s = sums[warp * NW][lane];
+#pragma unroll
+                for (int w = 1; w < NW; ++w) s = __fadd_rn(s, sums[warp * NW + w][lane]);
+                redf[warp][lane] = ffl_add_f(ffl{0.f, 0.f}, s);
+            }
+            __syncthreads();
+            if (warp == 0) status |= solve_totals(redf, nb, pose, Rs, ts, lane);
+        }
     }
-    const double pv = lane < 12 ? pose[lane] : 0.0;
-    if (lane < 9) Rs[lane] = ffl_from_double(pv);
-    else if (lane < 12) ts[lane - 9] = ffl_from_double(pv);
-    __syncwarp();
-    const float count = __shfl_sync(0xffffffffu, term.hi, 27);  // an integer below 2^24: exact
-    ffl o, xl;
-    const bool ok = count >= (float)kIcpMinInliers && warp_solve_step(term, Rs, ts, lane, o, xl);
-    if (lane < 12) pose[lane] = ok ? ffl_to_double(o) : pv;
-    if (lane == 0) *status |= ok ? 2 : 1;
+    __syncthreads();
+    if (rank == 0) {
+        if (tid < 12) pose_out[tid] = pose[tid];
+        if (tid == 0) *status_out |= status;
+    }
+    cluster_sync();  // no block leaves while another may still write to it
 }
 
 // The 28 sums of `nb` float partials in FP64: warp w takes blocks w, w + 8,
@@ -556,6 +751,25 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, cudaStream_t s, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// Whether this device takes the cluster (a property of device and kernel).
+bool cluster_fits(cudaLaunchConfig_t cfg) {
+    static std::atomic<int> known[64];  // 0 not asked, 1 no, 2 yes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (k == 0) {
+        int n = 0;
+        const bool ok =
+            cudaFuncSetAttribute(odo_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&n, odo_cluster_kernel, &cfg) == cudaSuccess && n >= 1;
+        if (!ok) (void)cudaGetLastError();
+        k = ok ? 2 : 1;
+        known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k == 2;
 }
 
 Level make_level(const uint8_t *ip, const float *dp, const uint8_t *ic, const float *dc, const int16_t *dx,
@@ -749,14 +963,49 @@ int tde_rgbd_odometry(const tde_rgbd_frame *prev, const tde_rgbd_frame *curr, co
     set_pose_kernel<<<1, 32, 0, s>>>(P, pose12_device, status_device, ticket);
     int st = check_launch("rgbd_odometry");
     if (st) return st;
-    for (int l = levels - 1; l >= 0; --l) {
+    const auto level = [&](int l) {
         const float div = (float)(1 << l);
         const tde_intrinsics in = {intr0->fx / div, intr0->fy / div, intr0->cx / div, intr0->cy / div,
                                    intr0->cols >> l, intr0->rows >> l};
-        const Level L = make_level(prev->intensity[l], prev->depth[l], curr->intensity[l], curr->depth[l], curr->dx[l],
-                                   curr->dy[l], in, params->max_depth_diff, params->max_depth,
-                                   params->min_gradient[l]);
-        const unsigned nb = odo_blocks(in.cols, in.rows);
+        return make_level(prev->intensity[l], prev->depth[l], curr->intensity[l], curr->depth[l], curr->dx[l],
+                          curr->dy[l], in, params->max_depth_diff, params->max_depth, params->min_gradient[l]);
+    };
+    // the coarse levels in one cluster
+    int l = levels - 1;
+    OdoLevels A;
+    A.n = 0;
+    for (; l >= 0; --l) {
+        const Level L = level(l);
+        const unsigned nb = odo_blocks(L.W, L.H);
+        if (nb > (unsigned)kOdoCluster) break;
+        if (params->iters[l] == 0) continue;
+        A.L[A.n] = L;
+        A.blocks[A.n] = (int)nb;
+        A.iters[A.n++] = params->iters[l];
+    }
+    if (A.n > 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kOdoCluster);
+        cfg.blockDim = dim3(kOdoThreads);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kOdoCluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cluster_fits(cfg)) {
+            cfg.numAttrs = 2;
+            TDE_CUDA(cudaLaunchKernelEx(&cfg, odo_cluster_kernel, A, pose12_device, status_device), "rgbd_odometry");
+        } else {
+            l = levels - 1;
+        }
+    }
+    for (; l >= 0; --l) {
+        const Level L = level(l);
+        const unsigned nb = odo_blocks(L.W, L.H);
         for (int it = 0; it < params->iters[l]; ++it) {
             TDE_CUDA(launch_pdl(residual_kernel, nb, s, L, (const double *)pose12_device, res), "rgbd_odometry");
             TDE_CUDA(launch_pdl(lsm_kernel<true>, nb, s, L, pose12_device, (const unsigned long long *)res, (int)nb,

@@ -189,10 +189,16 @@ __device__ __forceinline__ float warp_transpose_reduce(const float (&s)[32], int
 // 0.1404 ms per frame).
 constexpr int kSolveRefinements = 1;
 
-// One Gauss-Newton step, executed by all 32 lanes of a warp: lanes share every
-// instruction (one matrix or vector entry each, operands chosen by lane) and
-// exchange values by shuffles.  Lane l < 27 holds term l of [A | b] (term 27,
-// the inlier count, is not used).  [A | b] is first scaled by powers of two
+// The terms of a solve as its warp shares them (shared memory, one per warp).
+struct SolveTerms {
+    float4 hi[7];    // high parts of the scaled terms 0..26
+    float lo[28];    // their low parts
+    float scale[8];  // of the six unknowns
+};
+
+// One Gauss-Newton step, executed by all 32 lanes of a warp.  Lane l < 27 holds
+// term l of [A | b] (term 27, the inlier count, is not used).  [A | b] is first
+// scaled by powers of two
 // (D A D y = D b, x = D y; D = diag(2^k) with every diagonal entry of D A D in
 // [1, 4): exact, and the adjugate products below stay far inside the float
 // range).  The scaled system is factored and solved in FP32 -- with
@@ -213,70 +219,105 @@ constexpr int kSolveRefinements = 1;
 // the old entry) when A is not positive definite: a leading minor of the
 // scaled P or S at or below 2^-100 of its reference (integer tests on the
 // exponent bits), or a determinant product outside the normal float range.
-__device__ bool warp_solve_step(ffl term, const ffl *R_old, const ffl *t_old, int lane, ffl &out, ffl &xl) {
+//
+// Latency is all that counts here.  Every lane computes the whole FP32 solution
+// from the terms read back as 16-byte broadcasts: some 170 independent enough
+// operations, where one entry a lane needs a shuffle (25 cycles and an
+// instruction) per operand.  Only the float-float residual is spread, a row a
+// lane.  With an entry a lane throughout, the 19 steps of a 640x480 frame took
+// 122 us, now 117 (four-pixel blocks of 256 threads: 106 and 102 at 160x120, 135 and 125 beside
+// the refiner).  Lane constants formed ahead of the wait, or the solve out of line
+// (125 us), were slower: instructions that a launch meets for the first time.
+__device__ __forceinline__ bool warp_solve_step(ffl term, const ffl *R_old, const ffl *t_old, int lane, SolveTerms &sh,
+                                                ffl &out, ffl &xl) {
     const unsigned full = 0xffffffffu;
     const bool vec = lane >= 9;                       // lanes 9..11: vector entries
     const int vi = (lane >= 9 && lane < 12) ? lane - 9 : 0;
     const int l9 = lane < 9 ? lane : 0;
-    const int r = l9 / 3, c = l9 % 3;
-    const int r1 = (r + 1) % 3, r2 = (r + 2) % 3, c1 = (c + 1) % 3, c2 = (c + 2) % 3;
+    const int row = vec ? vi : l9 / 3, c = l9 % 3;
     // ---- the scaling: lane l < 27 holds entry (i, j), i <= j (j = 6: b_i) ----
-    float sx1, sx2;  // the scales of unknowns vi and 3 + vi (lanes 9..11)
     {
         const int i = (lane >= 7) + (lane >= 13) + (lane >= 18) + (lane >= 22) + (lane >= 25);
         const int j = lane - term_index(i, i) + i;
         const int jd = j < 6 ? j : 0;
         const float si = diag_scale(__shfl_sync(full, term.hi, term_index(i, i)));
         const float sj = diag_scale(__shfl_sync(full, term.hi, term_index(jd, jd)));
-        sx1 = diag_scale(__shfl_sync(full, term.hi, term_index(vi, vi)));
-        sx2 = diag_scale(__shfl_sync(full, term.hi, term_index(3 + vi, 3 + vi)));
-        if (lane < 27) term = ffl_scale(ffl_scale(term, si), j < 6 ? sj : 1.f);
+        if (lane < 27) {
+            term = ffl_scale(ffl_scale(term, si), j < 6 ? sj : 1.f);
+            reinterpret_cast<float *>(sh.hi)[lane] = term.hi;
+            sh.lo[lane] = term.lo;
+            if (j == 6) sh.scale[i] = si;
+        }
     }
-    const float th = term.hi;
-    auto T = [&](int src) { return __shfl_sync(full, th, src); };
+    __syncwarp();
+    float h[28];
+    #pragma unroll
+    for (int q = 0; q < 7; ++q) {
+        const float4 v = sh.hi[q];
+        h[4 * q] = v.x; h[4 * q + 1] = v.y; h[4 * q + 2] = v.z; h[4 * q + 3] = v.w;
+    }
+    // the residual's row of this lane (i < 6), ahead of its use
+    const int ri = lane < 6 ? lane : 0;
+    ffl Arow[6];
+    #pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const int k = term_index(ri, j);
+        Arow[j] = ffl{-reinterpret_cast<const float *>(sh.hi)[k], -sh.lo[k]};
+    }
+    const ffl brow{reinterpret_cast<const float *>(sh.hi)[term_index(ri, 6)], sh.lo[term_index(ri, 6)]};
+    float scale[6];
+    #pragma unroll
+    for (int k = 0; k < 6; ++k) scale[k] = sh.scale[k];
+    const ffl k0 = vec ? t_old[0] : R_old[c], k1 = vec ? t_old[1] : R_old[3 + c], k2 = vec ? t_old[2] : R_old[6 + c];
+    auto T = [&](int r, int q) { return h[term_index(r, q)]; };
     // ---- FP32 factors and first solution ----
-    // adj(P): cofactors (lane r, c), det(P) through the first row
-    const float CP = __fmaf_rn(T(term_index(r1, c1)), T(term_index(r2, c2)),
-                               -__fmul_rn(T(term_index(r1, c2)), T(term_index(r2, c1))));
-    auto CPs = [&](int src) { return __shfl_sync(full, CP, src); };
-    const float P0 = T(0);
-    const float detP = __fmaf_rn(P0, CPs(0), __fmaf_rn(T(1), CPs(1), __fmul_rn(T(2), CPs(2))));
-    const float CP8 = CPs(8);  // P00 P11 - P01^2
+    // adj(P): cofactors (symmetric), det(P) through the first row
+    float CP[3][3];
+    #pragma unroll
+    for (int i = 0; i < 3; ++i)
+        #pragma unroll
+        for (int j = i; j < 3; ++j) {
+            const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+            CP[i][j] = CP[j][i] = __fmaf_rn(T(i1, j1), T(i2, j2), -__fmul_rn(T(i1, j2), T(i2, j1)));
+        }
+    const float P0 = T(0, 0);
+    const float detP = __fmaf_rn(P0, CP[0][0], __fmaf_rn(T(0, 1), CP[0][1], __fmul_rn(T(0, 2), CP[0][2])));
+    const float CP8 = CP[2][2];  // P00 P11 - P01^2
     bool ok = clearly_pos_f(P0, 127) && clearly_pos_f(CP8, fexp(P0)) && clearly_pos_f(detP, fexp(CP8));
-    // the factors' entries a vector lane (9 + vi) needs for a right-hand side
-    float cpv[3], twr[3], csr[3], twc[3];
+    // T' = Q^T adj(P); v = adj(P) b1
+    float TW[3][3], v1[3];
     #pragma unroll
-    for (int k = 0; k < 3; ++k) cpv[k] = CPs(3 * k + vi);
-    // T' = Q^T adj(P) (lane r, c); v = adj(P) b1 (lane 9 + i)
-    float TW;
-    {
-        const int col = vec ? vi : c;
-        const float a0 = T(vec ? term_index(0, 6) : term_index(0, 3 + r));
-        const float a1 = T(vec ? term_index(1, 6) : term_index(1, 3 + r));
-        const float a2 = T(vec ? term_index(2, 6) : term_index(2, 3 + r));
-        TW = __fmaf_rn(a0, CPs(col), __fmaf_rn(a1, CPs(3 + col), __fmul_rn(a2, CPs(6 + col))));
+    for (int j = 0; j < 3; ++j) {
+        #pragma unroll
+        for (int i = 0; i < 3; ++i)
+            TW[i][j] =
+                __fmaf_rn(T(0, 3 + i), CP[0][j], __fmaf_rn(T(1, 3 + i), CP[1][j], __fmul_rn(T(2, 3 + i), CP[2][j])));
+        v1[j] = __fmaf_rn(T(0, 6), CP[0][j], __fmaf_rn(T(1, 6), CP[1][j], __fmul_rn(T(2, 6), CP[2][j])));
     }
-    auto TWs = [&](int src) { return __shfl_sync(full, TW, src); };
+    // S' = det(P) R - T' Q; u' = det(P) b2 - T' b1
+    float SU[3][3], u1[3];
     #pragma unroll
-    for (int k = 0; k < 3; ++k) { twr[k] = TWs(3 * vi + k); twc[k] = TWs(3 * k + vi); }
-    // S' = det(P) R - T' Q (lane r, c); u' = det(P) b2 - T' b1 (lane 9 + i)
-    float SU;
-    {
-        const int row = vec ? vi : r;
-        const float base = __fmul_rn(detP, T(vec ? term_index(3 + vi, 6) : term_index(3 + r, 3 + c)));
-        SU = __fmaf_rn(-TWs(3 * row), T(vec ? term_index(0, 6) : term_index(0, 3 + c)),
-                       __fmaf_rn(-TWs(3 * row + 1), T(vec ? term_index(1, 6) : term_index(1, 3 + c)),
-                                 __fmaf_rn(-TWs(3 * row + 2), T(vec ? term_index(2, 6) : term_index(2, 3 + c)), base)));
+    for (int i = 0; i < 3; ++i) {
+        auto minus_tw = [&](int col, float base) {
+            return __fmaf_rn(-TW[i][0], T(0, col),
+                             __fmaf_rn(-TW[i][1], T(1, col), __fmaf_rn(-TW[i][2], T(2, col), base)));
+        };
+        #pragma unroll
+        for (int j = 0; j < 3; ++j) SU[i][j] = minus_tw(3 + j, __fmul_rn(detP, T(3 + i, 3 + j)));
+        u1[i] = minus_tw(6, __fmul_rn(detP, T(3 + i, 6)));
     }
-    auto SUs = [&](int src) { return __shfl_sync(full, SU, src); };
-    // adj(S'), det(S'); U = adj(S') u' (lane 9 + i); the tests of S = S' / det(P)
-    const float CS = __fmaf_rn(SUs(3 * r1 + c1), SUs(3 * r2 + c2), -__fmul_rn(SUs(3 * r1 + c2), SUs(3 * r2 + c1)));
-    auto CSs = [&](int src) { return __shfl_sync(full, CS, src); };
+    // adj(S'), det(S'); the tests of S = S' / det(P)
+    float CS[3][3];
     #pragma unroll
-    for (int k = 0; k < 3; ++k) csr[k] = CSs(3 * vi + k);
-    const float S0 = SUs(0);
-    const float detS = __fmaf_rn(S0, CSs(0), __fmaf_rn(SUs(1), CSs(1), __fmul_rn(SUs(2), CSs(2))));
-    const float CS8 = CSs(8);
+    for (int i = 0; i < 3; ++i)
+        #pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+            CS[i][j] = __fmaf_rn(SU[i1][j1], SU[i2][j2], -__fmul_rn(SU[i1][j2], SU[i2][j1]));
+        }
+    const float S0 = SU[0][0];
+    const float detS = __fmaf_rn(S0, CS[0][0], __fmaf_rn(SU[0][1], CS[0][1], __fmul_rn(SU[0][2], CS[0][2])));
+    const float CS8 = CS[2][2];
     const int eP = fexp(detP) - 127;
     ok = ok && clearly_pos_f(S0, 127 + eP) && clearly_pos_f(CS8, fexp(S0) + eP) && clearly_pos_f(detS, fexp(CS8) + eP);
     // both inverses from one reciprocal (of a normal product), one Newton step
@@ -286,50 +327,50 @@ __device__ bool warp_solve_step(ffl term, const ffl *R_old, const ffl *t_old, in
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rPS) : "f"(dPS));
     rPS = __fmaf_rn(rPS, __fmaf_rn(-dPS, rPS, 1.f), rPS);
     const float rS = __fmul_rn(detP, rPS), rP = __fmul_rn(detS, rPS), rSP = __fmul_rn(rS, rP);
-    // y for a right-hand side: v = adj(P) h1 and u' (lane 9 + i) in, y1 and
-    // y2 (lane 9 + i) out
-    auto back = [&](float v, float u, float &y1, float &y2) {
-        const float u0 = __shfl_sync(full, u, 9), u1 = __shfl_sync(full, u, 10), u2 = __shfl_sync(full, u, 11);
-        const float U = __fmaf_rn(csr[0], u0, __fmaf_rn(csr[1], u1, __fmul_rn(csr[2], u2)));
-        const float U0 = __shfl_sync(full, U, 9), U1 = __shfl_sync(full, U, 10), U2 = __shfl_sync(full, U, 11);
-        const float W = __fmaf_rn(twc[0], U0, __fmaf_rn(twc[1], U1, __fmul_rn(twc[2], U2)));
-        y2 = __fmul_rn(U, rS);
-        y1 = __fmaf_rn(-W, rSP, __fmul_rn(v, rP));
+    // y for a right-hand side: v = adj(P) h1 and u' in, y1 and y2 out
+    auto back = [&](const float (&v)[3], const float (&u)[3], float (&y1)[3], float (&y2)[3]) {
+        float U[3];
+        #pragma unroll
+        for (int i = 0; i < 3; ++i)
+            U[i] = __fmaf_rn(CS[i][0], u[0], __fmaf_rn(CS[i][1], u[1], __fmul_rn(CS[i][2], u[2])));
+        #pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float W = __fmaf_rn(TW[0][i], U[0], __fmaf_rn(TW[1][i], U[1], __fmul_rn(TW[2][i], U[2])));
+            y2[i] = __fmul_rn(U[i], rS);
+            y1[i] = __fmaf_rn(-W, rSP, __fmul_rn(v[i], rP));
+        }
     };
-    float y1f, y2f;
-    back(TW, SU, y1f, y2f);
-    ffl y1{y1f, 0.f}, y2{y2f, 0.f};
+    ffl y[6];
+    {
+        float y1[3], y2[3];
+        back(v1, u1, y1, y2);
+        #pragma unroll
+        for (int i = 0; i < 3; ++i) { y[i] = ffl{y1[i], 0.f}; y[3 + i] = ffl{y2[i], 0.f}; }
+    }
     // ---- refinement: residual b - A y in float-float (lane i < 6 takes row
     // i), correction from the FP32 factors ----
-    {
-        const int ri = lane < 6 ? lane : 0;
-        ffl Arow[6];
+    #pragma unroll
+    for (int step = 0; step < kSolveRefinements; ++step) {
+        const float res = ffl_dot<6, true>(Arow, y, brow).hi;
+        float g[6], v[3], u[3], d1[3], d2[3];
         #pragma unroll
-        for (int j = 0; j < 6; ++j) Arow[j] = ffl_neg(shfl(term, term_index(ri, j)));
-        const ffl brow = shfl(term, term_index(ri, 6));
+        for (int k = 0; k < 6; ++k) g[k] = __shfl_sync(full, res, k);
         #pragma unroll
-        for (int step = 0; step < kSolveRefinements; ++step) {
-            const ffl yv[6] = {shfl(y1, 9), shfl(y1, 10), shfl(y1, 11), shfl(y2, 9), shfl(y2, 10), shfl(y2, 11)};
-            const float res = ffl_dot<6, true>(Arow, yv, brow).hi;
-            const float h0 = __shfl_sync(full, res, 0), h1 = __shfl_sync(full, res, 1), h2 = __shfl_sync(full, res, 2);
-            const float hb = __shfl_sync(full, res, 3 + vi);
-            const float v = __fmaf_rn(cpv[0], h0, __fmaf_rn(cpv[1], h1, __fmul_rn(cpv[2], h2)));
-            const float u = __fmaf_rn(-twr[0], h0, __fmaf_rn(-twr[1], h1, __fmaf_rn(-twr[2], h2, __fmul_rn(detP, hb))));
-            float d1, d2;
-            back(v, u, d1, d2);
-            y1 = ffl_add_f(y1, d1);
-            y2 = ffl_add_f(y2, d2);
+        for (int i = 0; i < 3; ++i) {
+            v[i] = __fmaf_rn(CP[0][i], g[0], __fmaf_rn(CP[1][i], g[1], __fmul_rn(CP[2][i], g[2])));
+            u[i] = __fmaf_rn(-TW[i][0], g[0],
+                             __fmaf_rn(-TW[i][1], g[1], __fmaf_rn(-TW[i][2], g[2], __fmul_rn(detP, g[3 + i]))));
         }
+        back(v, u, d1, d2);
+        #pragma unroll
+        for (int i = 0; i < 3; ++i) { y[i] = ffl_add_f(y[i], d1[i]); y[3 + i] = ffl_add_f(y[3 + i], d2[i]); }
     }
-    // x = D y (lane 9 + i)
-    const ffl X1 = ffl_scale(y1, sx1), X2 = ffl_scale(y2, sx2);
-    const ffl wx = shfl(X1, 9), wy = shfl(X1, 10), wz = shfl(X1, 11);
-    const ffl x20 = shfl(X2, 9), x21 = shfl(X2, 10), x22 = shfl(X2, 11);
+    // x = D y
+    const ffl wx = ffl_scale(y[0], scale[0]), wy = ffl_scale(y[1], scale[1]), wz = ffl_scale(y[2], scale[2]);
+    const ffl x20 = ffl_scale(y[3], scale[3]), x21 = ffl_scale(y[4], scale[4]), x22 = ffl_scale(y[5], scale[5]);
     xl = lane < 3 ? pick3(lane, wx, wy, wz) : pick3(lane - 3, x20, x21, x22);
     // the pose update: this lane's column (of R, or t) and row
-    const int row = vec ? vi : r;
     const ffl th2 = ffl_dot<3, false>({wx, wy, wz}, {wx, wy, wz}, ffl{});
-    const ffl k0 = vec ? t_old[0] : R_old[c], k1 = vec ? t_old[1] : R_old[3 + c], k2 = vec ? t_old[2] : R_old[6 + c];
     // (w x k)[row] = w[row+1] k[row+2] - w[row+2] k[row+1]
     const int ra = row == 2 ? 0 : row + 1, rb = row == 0 ? 2 : row - 1;
     const ffl cr = ffl_dot<2, false>({pick3(ra, wx, wy, wz), ffl_neg(pick3(rb, wx, wy, wz))},

@@ -598,7 +598,10 @@ def rgbd_pass(tde, syn, torch, cfg, dev, ws, rank, with_cpu, pairs=48, warm=4):
         et.append(np.linalg.norm(est[i][9:] - gt))
         er.append(np.degrees(np.arccos(np.clip((np.trace(Re) - 1) / 2, -1, 1))))
     levels = 4
-    launches = (1 + (levels - 1) + levels) + (1 + 2 * sum(int(x) for x in od.params.iters[:levels]))
+    # the pose, one launch for the steps of the levels of up to 16 blocks of 2048 pixels, two for each other step
+    large = [l for l in range(levels) if (cfg.cols >> l) * (cfg.rows >> l) > 16 * 2048]
+    launches = ((1 + (levels - 1) + levels) + 1 + int(len(large) < levels) +
+                2 * sum(int(od.params.iters[l]) for l in large))
     out = {"value": round(ws * pairs / (ms * 1e-3), 2), "unit": "frames/s", "ms_per_step": round(ms / pairs, 5),
            "ms_per_step_without_graphs": round(ms_eager / pairs, 5), "gpu_launches": launches * pairs,
            "graph_poses_equal_eager": bool(np.array_equal(est, est_eager)),

@@ -219,3 +219,46 @@ def test_integrate_takes_undefined_scratch_on_any_stream(cuda, tde, orc, cols, r
         got = maps.cpu().numpy()
         for a, b in zip(got, (vmo, nmo)):
             assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.nan_to_num(a), np.nan_to_num(b))
+
+
+@pytest.mark.parametrize("cols,rows,levels", [(64, 32, 1), (256, 128, 1), (257, 128, 1), (330, 200, 2), (320, 240, 3)])
+def test_odometry_steps_in_a_cluster_and_in_launches(cuda, tde, orc, cols, rows, levels):
+    """Levels of 1, 16 (the most that one cluster takes) and 17 blocks, and a
+    frame of both kinds: the first step is the oracle's, and all steps of a call
+    end where the same steps one call at a time do, bit for bit."""
+    import torch
+    syn = importlib.import_module("3deye_gb300.synth")
+    rg = importlib.import_module("3deye_gb300.rgbd")
+    cfg = syn.small_config("c2", frames=2, cols=cols, rows=rows)
+    scene, traj = syn.make_scene(cfg, 5), syn.make_trajectory(cfg, 5, 4)
+    oi = orc.Intr(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cols, rows)
+    it = tde.Intrinsics(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cols, rows)
+    host, dev = [], []
+    for k in (0, 1):
+        mm = np.rint(orc.render_depth(scene, traj[k], oi) * 1000).astype(np.uint16)
+        rgb = orc.render_rgb(scene, traj[k], oi)
+        host.append(orc.rgbd_levels(mm, rgb, levels))
+        dev.append(rg.RgbdFrame(cols, rows, levels, cuda).load(torch.from_numpy(mm.view(np.int16)).to(cuda),
+                                                               torch.from_numpy(rgb).to(cuda)))
+
+    def run(iters, init):
+        p = rg.default_params(levels)
+        for l in range(levels):
+            p.iters[l] = iters[l]
+        return rg.RgbdOdometry(it, p).estimate(dev[0], dev[1], init)
+
+    start = np.array([1, 0, 0, 0, 1, 0, 0, 0, 1, 0.002, -0.001, 0.003], np.float64)
+    one = [0] * (levels - 1) + [1]
+    pose, status = run(one, start)
+    ref, failed = orc.rgbd_odometry(host[0], host[1], oi, one, [10.0] * levels, init_pose12=start)
+    assert status == rg.STATUS_SOLVED and failed == 0
+    np.testing.assert_allclose(pose, ref, rtol=0, atol=1e-7)  # the bound of the one-step test at 640x480
+    steps = [3] * levels
+    whole, status = run(steps, start)
+    single = start
+    for l in range(levels - 1, -1, -1):
+        for _ in range(steps[l]):
+            single, st = run([int(k == l) for k in range(levels)], single)
+            assert st == rg.STATUS_SOLVED
+    assert status == rg.STATUS_SOLVED and np.array_equal(whole, single)
+    assert not np.array_equal(whole, pose)
