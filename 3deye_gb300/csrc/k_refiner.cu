@@ -334,10 +334,25 @@ struct AccAt {
 __host__ __device__ constexpr size_t conv_stage_bytes(int cout, bool pool) {
     return (size_t)32 * cout * 2 * (pool ? 2 : 1);
 }
+// The first plane's channels where the output may be two planes (48 channels: the
+// input gradient of the full-resolution layer with two sources), else 0.  A constant:
+// with the split as a factor of the addresses that convolution took 180 us of 131;
+// the layers of 80 and 112 channels, short of registers, lost with it what their
+// planes gained.
+__host__ __device__ constexpr int conv_split(int cout) { return cout == 48 ? 32 : 0; }
+// Channel c of pixel p of a run of pixels that begins at `first` in the first plane
+// and at `second` in the second.
+template <int COUT>
+__device__ __forceinline__ bf16 *split_at(bf16 *first, bf16 *second, int p, int c) {
+    constexpr int K = conv_split(COUT);
+    return c < K ? first + p * K + c : second + p * (COUT - K) + (c - K);
+}
 template <int COUT, bool POOL, int SETS>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs &A, ConvPipe &pp, const float *s_bias, const float *s_head,
                                            unsigned char *stage, int rows_per_item, int items, int NA, int warp, int lane) {
     constexpr int ROWS = POOL ? 2 : 1;
+    constexpr int KS = POOL ? 0 : conv_split(COUT);
+    bf16 *const plane2 = A.out + (size_t)A.n * A.h * A.w * KS;
     const bool staged = stage != nullptr;
     constexpr int UNITS = 4 * COUT / 8;  // 16-byte units of one run
     const uint32_t sbase = tc::smem_u32(stage) + (uint32_t)((warp - kConvMmaWarp - 1) * ROWS * 32 * COUT * 2);
@@ -409,8 +424,11 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs &A, ConvPipe &pp, c
                                      "r"(q0[r].y), "r"(q0[r].z), "r"(q0[r].w) : "memory");
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + (((u + 1) ^ run) * 16)),
                                      "r"(q1[r].x), "r"(q1[r].y), "r"(q1[r].z), "r"(q1[r].w) : "memory");
-                    } else {
-                        if (valid) store16(A.out + (pix + (size_t)r * A.w) * COUT + j, q0[r], q1[r]);
+                    } else if (valid) {
+                        const size_t at = pix + (size_t)r * A.w;
+                        bf16 *o = A.out + at * COUT + j;
+                        if (KS && A.split) o = split_at<COUT>(A.out + at * KS, plane2 + at * (COUT - KS), 0, j);
+                        store16(o, q0[r], q1[r]);
                     }
                 }
                 if constexpr (POOL) {
@@ -440,18 +458,44 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs &A, ConvPipe &pp, c
             if (staged) {
                 __syncwarp();
                 // pixel 4 * quarter + 16 * k of the tile begins run k
-                bf16 *dst = A.out + (((size_t)st.img * A.h + y) * A.w + st.x0 + 4 * (int)quarter) * COUT;
+                const size_t first = ((size_t)st.img * A.h + y) * A.w + st.x0 + 4 * (int)quarter;
+                const int left = A.w - st.x0 - 4 * (int)quarter;  // pixels of the row from there on
+                auto unit = [&](int r, int k, int u) {
+                    const uint32_t at = sbase + (uint32_t)((r * 8 + k) * UNITS * 16);
+                    uint4 q;
+                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "r"(at + ((u ^ k) * 16)) : "memory");
+                    return q;
+                };
+                if (KS && A.split) {
+                    // the units of the first plane, then those of the second
+                    constexpr int U1 = KS ? 4 * KS / 8 : 4, U2 = UNITS - U1;
+                    bf16 *d1 = A.out + first * KS, *d2 = plane2 + first * (COUT - KS);
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) {
+                    for (int t = 0; t < U1 / 4; ++t) {
+                        const int i = t * 32 + lane, k = i / U1, u = i - k * U1, p = u / (U1 / 4);
+                        if (16 * k + p < left)
+                            *reinterpret_cast<uint4 *>(d1 + 16 * k * KS + u * 8) =
+                                unit(0, k, p * (COUT / 8) + u - p * (U1 / 4));
+                    }
 #pragma unroll
-                    for (int t = 0; t < UNITS / 4; ++t) {
-                        const int i = t * 32 + lane, k = i / UNITS, u = i - k * UNITS;
-                        const uint32_t at = sbase + (uint32_t)((r * 8 + k) * UNITS * 16);
-                        uint4 q;
-                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                                     : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "r"(at + ((u ^ k) * 16)) : "memory");
-                        if (st.x0 + 4 * (int)quarter + 16 * k + u / (COUT / 8) < A.w)
-                            *reinterpret_cast<uint4 *>(dst + ((size_t)r * A.w + 16 * k) * COUT + u * 8) = q;
+                    for (int t = 0; t < U2 / 4; ++t) {
+                        const int i = t * 32 + lane, k = i / U2, u = i - k * U2, p = u / (U2 / 4);
+                        if (16 * k + p < left)
+                            *reinterpret_cast<uint4 *>(d2 + 16 * k * (COUT - KS) + u * 8) =
+                                unit(0, k, p * (COUT / 8) + KS / 8 + u - p * (U2 / 4));
+                    }
+                } else {
+                    bf16 *dst = A.out + first * COUT;
+#pragma unroll
+                    for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+                        for (int t = 0; t < UNITS / 4; ++t) {
+                            const int i = t * 32 + lane, k = i / UNITS, u = i - k * UNITS;
+                            const uint4 q = unit(r, k, u);
+                            if (16 * k + u / (COUT / 8) < left)
+                                *reinterpret_cast<uint4 *>(dst + ((size_t)r * A.w + 16 * k) * COUT + u * 8) = q;
+                        }
                     }
                 }
                 __syncwarp();
@@ -1466,14 +1510,37 @@ __global__ void loss_reduce_kernel(const float *__restrict__ partial, int blocks
 // ---------------------------------------------------------------------------
 // Gradient routing through upsampling, pooling and skips
 // ---------------------------------------------------------------------------
-__global__ void up_back_kernel(const bf16 *__restrict__ g, int cu, int ca, const bf16 *__restrict__ y_low,
-                               bf16 *__restrict__ dz, int n, int h, int w) {
-    const int hl = h >> 1, wl = w >> 1, cch = ca >> 3;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n * hl * wl * cch) return;
-    const int c = (int)(i % cch);
-    const size_t q = i / cch;
-    const int xl = (int)(q % wl), yl = (int)((q / wl) % hl), img = (int)(q / ((size_t)wl * hl));
+// A block takes kRouteThreads of the (pixel, 8 channels) items of one low-resolution
+// row, a thread one of them with its four full-resolution pixels.  Memory bounds
+// these kernels.  Of an interleaved gradient of two sources each kernel wants some
+// 32-byte sectors of each pixel, and DRAM moves 64 bytes, so the largest lies in two
+// planes.  Batch 16 of 640x480, that level: up_back 101 -> 73 us (470 MB),
+// pool_back_add 121 -> 69 us (510 MB).
+constexpr int kRouteThreads = 128;
+struct LowPixel {
+    int c, x, y, img;  // channel group, column, row, image
+    size_t q;          // raster index over the images
+};
+__device__ __forceinline__ bool low_pixel(int hl, int wl, int cch, LowPixel &t) {
+    const unsigned items = (unsigned)wl * (unsigned)cch, per_row = (items + kRouteThreads - 1) / kRouteThreads;
+    const unsigned row = blockIdx.x / per_row, i = (blockIdx.x - row * per_row) * kRouteThreads + threadIdx.x;
+    if (i >= items) return false;
+    t.x = (int)(i / (unsigned)cch);
+    t.c = (int)(i - (unsigned)t.x * (unsigned)cch);
+    t.img = (int)(row / (unsigned)hl);
+    t.y = (int)(row - (unsigned)t.img * (unsigned)hl);
+    t.q = (size_t)row * wl + t.x;
+    return true;
+}
+
+__global__ void __launch_bounds__(kRouteThreads) up_back_kernel(const bf16 *__restrict__ g, int cu, int ca,
+                                                                const bf16 *__restrict__ y_low, bf16 *__restrict__ dz,
+                                                                int h, int w) {
+    const int hl = h >> 1, wl = w >> 1;
+    LowPixel t;
+    if (!low_pixel(hl, wl, ca >> 3, t)) return;
+    const int c = t.c, xl = t.x, yl = t.y, img = t.img;
+    const size_t q = t.q;
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -1490,21 +1557,23 @@ __global__ void up_back_kernel(const bf16 *__restrict__ g, int cu, int ca, const
     *reinterpret_cast<uint4 *>(dz + q * ca + 8 * c) = pack8(s);
 }
 
-__global__ void pool_back_add_kernel(const bf16 *__restrict__ e, const bf16 *__restrict__ gp,
-                                     const bf16 *__restrict__ skip, int cu, int off, int ch, bf16 *__restrict__ dz,
-                                     int n, int h, int w) {
-    const int hl = h >> 1, wl = w >> 1, cch = ch >> 3;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n * hl * wl * cch) return;
-    const int c = (int)(i % cch);
-    const size_t q = i / cch;
-    const int xl = (int)(q % wl), yl = (int)((q / wl) % hl), img = (int)(q / ((size_t)wl * hl));
+__global__ void __launch_bounds__(kRouteThreads) pool_back_add_kernel(const bf16 *__restrict__ e,
+                                                                      const bf16 *__restrict__ gp,
+                                                                      const bf16 *__restrict__ skip, int cu, int ch,
+                                                                      bf16 *__restrict__ dz, int h, int w) {
+    const int hl = h >> 1, wl = w >> 1;
+    LowPixel t;
+    if (!low_pixel(hl, wl, ch >> 3, t)) return;
+    const int c = t.c, xl = t.x, yl = t.y, img = t.img;
+    const size_t q = t.q;
     float ev[4][8], mx[8];
     size_t pix[4];
+    uint4 sk[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         pix[k] = ((size_t)img * h + 2 * yl + (k >> 1)) * w + 2 * xl + (k & 1);
         unpack8(ldg16(e + pix[k] * ch + 8 * c), ev[k]);
+        sk[k] = ldg16(skip + pix[k] * cu + 8 * c);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) mx[j] = fmaxf(fmaxf(ev[0][j], ev[1][j]), fmaxf(ev[2][j], ev[3][j]));
@@ -1516,7 +1585,7 @@ __global__ void pool_back_add_kernel(const bf16 *__restrict__ e, const bf16 *__r
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         float s[8];
-        unpack8(ldg16(skip + pix[k] * cu + off + 8 * c), s);
+        unpack8(sk[k], s);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float v = s[j] + (first[j] == k ? gv[j] : 0.f);
@@ -1646,6 +1715,8 @@ static bool epilogue_for(int mode, int cca, int ccb, int cout, bool pool) {
 
 int launch_conv(const ConvArgs &a, const ConvPlan &plan, int num_sms, cudaStream_t s) {
     const int cin = a.ca + a.cb;
+    if (a.split && a.split != conv_split(a.cout))
+        return set_error(TDE_ERR_INVALID_ARG, "refiner conv: %d channels in planes of %d", a.cout, a.split);
     if (cin % 16 || a.ca % 8 || a.cout % 16 || a.cout < 16 || a.cout > 128 || cin > 128 || a.w <= 0 || a.h <= 0 ||
         a.n <= 0 || (a.head_w && a.cout != 16) || (a.mode_a == SRC_UP && (a.h % 2 || a.w % 2)) ||
         (a.pool_out && (a.h % 2 || a.w % 2 || a.mask)) ||
@@ -1764,16 +1835,20 @@ int launch_loss(const float *out_m, const float *depth_m, const uint16_t *target
     return check_launch("refiner loss reduce");
 }
 
+int conv_planes(int cout) { return conv_split(cout); }
+
+static unsigned route_blocks(int n, int hl, int wl, int cch) {
+    return (unsigned)(n * hl) * div_up(wl * cch, kRouteThreads);
+}
+
 int launch_up_back(const bf16 *g, int cu, int ca, const bf16 *y_low, bf16 *dz, int n, int h, int w, cudaStream_t s) {
-    const size_t items = (size_t)n * (h / 2) * (w / 2) * (ca / 8);
-    up_back_kernel<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(g, cu, ca, y_low, dz, n, h, w);
+    up_back_kernel<<<route_blocks(n, h / 2, w / 2, ca / 8), kRouteThreads, 0, s>>>(g, cu, ca, y_low, dz, h, w);
     return check_launch("refiner up_back");
 }
 
-int launch_pool_back_add(const bf16 *e, const bf16 *gp, const bf16 *skip, int cu, int off, int c, bf16 *dz, int n,
-                         int h, int w, cudaStream_t s) {
-    const size_t items = (size_t)n * (h / 2) * (w / 2) * (c / 8);
-    pool_back_add_kernel<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(e, gp, skip, cu, off, c, dz, n, h, w);
+int launch_pool_back_add(const bf16 *e, const bf16 *gp, const bf16 *skip, int cu, int c, bf16 *dz, int n, int h, int w,
+                         cudaStream_t s) {
+    pool_back_add_kernel<<<route_blocks(n, h / 2, w / 2, c / 8), kRouteThreads, 0, s>>>(e, gp, skip, cu, c, dz, h, w);
     return check_launch("refiner pool_back_add");
 }
 

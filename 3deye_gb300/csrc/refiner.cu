@@ -55,18 +55,18 @@ inline int conv_mode(const Conv &c) { return c.pool_in >= 0 ? (int)SRC_DIRECT : 
 // gradient goes to (masked by `mask` when the input is a ReLU output read
 // directly), and how that becomes the next output gradient.
 enum Post { POST_NONE, POST_UP, POST_POOL };
-struct Back { int dz, gx, mask, post, post_out, skip, skip_cu, skip_off; };
+struct Back { int dz, gx, mask, post, post_out, skip, skip_after; };
 const Back kBack[kConvs] = {
-    {G_DZ2, G_DZ1, E0A, POST_NONE, -1, -1, 0, 0},       // c2
-    {G_DZ3, G_P1, -1, POST_POOL, G_DZ2, G_U0, 48, 32},  // c3: e0 also feeds c11 (channels 32..47)
-    {G_DZ4, G_DZ3, E1A, POST_NONE, -1, -1, 0, 0},       // c4
-    {G_DZ5, G_P2, -1, POST_POOL, G_DZ4, G_U1, 80, 48},  // c5: e1 also feeds c10 (48..79)
-    {G_DZ6, G_DZ5, E2A, POST_NONE, -1, -1, 0, 0},       // c6
-    {G_DZ7, G_P3, -1, POST_POOL, G_DZ6, G_U2, 112, 64}, // c7: e2 also feeds c9 (64..111)
-    {G_DZ8, G_DZ7, B3A, POST_NONE, -1, -1, 0, 0},       // c8
-    {G_DZ9, G_U2, -1, POST_UP, G_DZ8, -1, 0, 0},        // c9
-    {G_DZ10, G_U1, -1, POST_UP, G_DZ9, -1, 0, 0},       // c10
-    {G_DZ11, G_U0, -1, POST_UP, G_DZ10, -1, 0, 0},      // c11
+    {G_DZ2, G_DZ1, E0A, POST_NONE, -1, -1, 0},       // c2
+    {G_DZ3, G_P1, -1, POST_POOL, G_DZ2, G_U0, 32},  // c3: e0 also feeds c11 (after 32 channels of its input)
+    {G_DZ4, G_DZ3, E1A, POST_NONE, -1, -1, 0},       // c4
+    {G_DZ5, G_P2, -1, POST_POOL, G_DZ4, G_U1, 48},  // c5: e1 also feeds c10
+    {G_DZ6, G_DZ5, E2A, POST_NONE, -1, -1, 0},       // c6
+    {G_DZ7, G_P3, -1, POST_POOL, G_DZ6, G_U2, 64},  // c7: e2 also feeds c9
+    {G_DZ8, G_DZ7, B3A, POST_NONE, -1, -1, 0},       // c8
+    {G_DZ9, G_U2, -1, POST_UP, G_DZ8, -1, 0},        // c9
+    {G_DZ10, G_U1, -1, POST_UP, G_DZ9, -1, 0},       // c10
+    {G_DZ11, G_U0, -1, POST_UP, G_DZ10, -1, 0},      // c11
 };
 
 constexpr int kC1W = 16 * 9 * 3, kC1B = 16;
@@ -226,15 +226,21 @@ int loss_grad(tde_refiner *r, const uint16_t *raw, const uint16_t *target, int n
         a.a = r->gr[k.dz]; a.ca = c.cout; a.mode_a = SRC_DIRECT;
         a.wgt = r->wt + kL.wq[i];
         a.out = r->gr[k.gx]; a.cout = cin; a.relu = 0;
+        a.split = k.post == POST_UP ? conv_planes(cin) : 0;  // the upsampled source's channels, then the skip's
         a.mask = k.mask >= 0 ? r->act[k.mask] : nullptr;
         a.n = n; a.h = h; a.w = w;
         a.err = r->err;
         TDE_TRY(launch_conv(a, r->bwd_plan[i], r->num_sms, s));
-        if (k.post == POST_UP)
-            TDE_TRY(launch_up_back(r->gr[k.gx], cin, c.ca, r->act[c.a], r->gr[k.post_out], n, h, w, s));
-        else if (k.post == POST_POOL)
-            TDE_TRY(launch_pool_back_add(r->act[c.a], r->gr[k.gx], r->gr[k.skip], k.skip_cu, k.skip_off, c.ca,
-                                         r->gr[k.post_out], n, h * 2, w * 2, s));
+        if (k.post == POST_UP) {
+            TDE_TRY(launch_up_back(r->gr[k.gx], a.split ? c.ca : cin, c.ca, r->act[c.a], r->gr[k.post_out], n, h, w,
+                                   s));
+        } else if (k.post == POST_POOL) {
+            const int cu = k.skip_after + c.ca;  // the skip's channels are the last c.ca of its layer's input
+            const bool planes = conv_planes(cu) != 0;
+            const bf16 *skip = r->gr[k.skip] + (planes ? (size_t)n * (h * 2) * (w * 2) : 1) * k.skip_after;
+            TDE_TRY(launch_pool_back_add(r->act[c.a], r->gr[k.gx], skip, planes ? c.ca : cu, c.ca, r->gr[k.post_out], n,
+                                         h * 2, w * 2, s));
+        }
     }
     TDE_TRY(launch_conv_in_wgrad(r->depth_m, r->gr[G_DZ1], n, H, W, r->in_partial, conv_in_wgrad_blocks(n, H, W),
                                  r->grad + kL.c1w, r->grad + kL.c1b, s));
@@ -436,6 +442,18 @@ int tde_refiner_get_tensor(tde_refiner *r, int id, void *host, size_t bytes) {
                       : id == ACT_COUNT ? (const void *)r->out_m
                                         : (const void *)r->gr[id - ACT_COUNT - 1];
     TDE_CUDA(cudaDeviceSynchronize(), "refiner_get_tensor");
+    for (int i = 0; i < kConvs; ++i) {
+        if (kBack[i].post != POST_UP || id != ACT_COUNT + 1 + kBack[i].gx || !conv_planes(kConv[i].ca + kConv[i].cb))
+            continue;
+        // two planes on the device (ConvArgs::split), one interleaved tensor here
+        const size_t ca = kConv[i].ca, cb = kConv[i].cb, np = need / (2 * (ca + cb));
+        char *h = static_cast<char *>(host);
+        TDE_CUDA(cudaMemcpy2D(h, 2 * (ca + cb), src, 2 * ca, 2 * ca, np, cudaMemcpyDeviceToHost), "refiner_get_tensor");
+        TDE_CUDA(cudaMemcpy2D(h + 2 * ca, 2 * (ca + cb), static_cast<const bf16 *>(src) + np * ca, 2 * cb, 2 * cb, np,
+                              cudaMemcpyDeviceToHost),
+                 "refiner_get_tensor");
+        return TDE_OK;
+    }
     TDE_CUDA(cudaMemcpy(host, src, bytes, cudaMemcpyDeviceToHost), "refiner_get_tensor");
     return TDE_OK;
 }

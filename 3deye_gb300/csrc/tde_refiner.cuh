@@ -27,8 +27,9 @@ struct ConvArgs {
     int cb;
     const bf16 *wgt;  // [cout][9][ca + cb]
     const float *bias;  // [cout] or null
-    bf16 *out;          // [n][h][w][cout]
+    bf16 *out;          // [n][h][w][cout]; split: [n][h][w][split], then [n][h][w][cout - split]
     int cout, relu;
+    int split;          // 0, or the channels of the first of two planes: conv_planes(cout)
     const bf16 *mask;  // null, or [n][h][w][cout]: out = 0 where mask <= 0
     // fused 1x1 head (cout == 16): depth_out = depth_in > 0 ? depth_in + 0.01 (w.out + b) : 0
     const float *head_w, *head_b, *depth_in;
@@ -101,11 +102,14 @@ int launch_loss(const float *out_m, const float *depth_m, const uint16_t *target
                 double *loss2, cudaStream_t s);
 int loss_blocks(int n, int h, int w);
 
-// dz[n,h/2,w/2,c] = bf16(sum_2x2 g[n,y,x,c] * (y_low > 0)), c < ca; g has cu channels.
+// The first plane's channels of an input gradient of `cout` channels (ConvArgs::split); 0: not in planes.
+int conv_planes(int cout);
+// dz[n,h/2,w/2,c] = bf16(sum_2x2 g[n,y,x,c] * (y_low > 0)), c < ca; g's pixels lie cu channels apart.
 int launch_up_back(const bf16 *g, int cu, int ca, const bf16 *y_low, bf16 *dz, int n, int h, int w, cudaStream_t s);
-// dz[n,y,x,c] = bf16((skip[n,y,x,off+c] + first-argmax(e) ? gp[n,y/2,x/2,c] : 0) * (e > 0)), skip with cu channels.
-int launch_pool_back_add(const bf16 *e, const bf16 *gp, const bf16 *skip, int cu, int off, int c, bf16 *dz, int n,
-                         int h, int w, cudaStream_t s);
+// dz[n,y,x,c] = bf16((skip[n,y,x,c] + first-argmax(e) ? gp[n,y/2,x/2,c] : 0) * (e > 0)), c channels; skip's pixels
+// lie cu channels apart.
+int launch_pool_back_add(const bf16 *e, const bf16 *gp, const bf16 *skip, int cu, int c, bf16 *dz, int n, int h, int w,
+                         cudaStream_t s);
 
 // AdamW on the flat parameter vector (decay applied where decay_mask != 0).
 int launch_adamw(float *theta, const float *grad, float *m, float *v, const uint8_t *decay_mask, size_t count,

@@ -61,3 +61,47 @@ def test_each_layer_at_tile_edges(cuda, n, h, w):
         Sw, Sb = U.conv3x3_wgrad(np.abs(x), np.abs(T[dz]))
         assert np.all(np.abs(g[name + ".w"] - dw) <= 1500 * 2.0 ** -23 * Sw + 1e-30), name + " weight gradient"
         assert np.all(np.abs(g[name + ".b"] - db) <= 1500 * 2.0 ** -23 * Sb + 1e-30), name + " bias gradient"
+
+
+@pytest.mark.parametrize("n,h,w", SIZES)
+def test_gradient_routing_at_row_ends(cuda, n, h, w):
+    """The gradients routed through upsampling, pooling and skips equal the same
+    FP32 operations on the stored tensors, rounded to bf16: rows of fewer items than
+    a block, of whole blocks and of one item more, whole and split gradients."""
+    import torch
+    rf = importlib.import_module("3deye_gb300.refiner")
+    rng = np.random.default_rng(n + h + w)
+    raw = rng.integers(500, 3000, (n, h, w)).astype(np.uint16)
+    tgt = np.clip(raw.astype(np.int64) + rng.integers(-6, 7, raw.shape), 0, 32767).astype(np.uint16)
+    R = rf.Refiner(n, h, w, seed=9)
+    theta = R.get_params()
+    theta[-17:-1] = rng.normal(0, 0.1, 16)  # the head
+    theta[:-17][theta[:-17] == 0] = 0.05    # biases
+    R.set_params(theta)
+    R.loss_grad(raw, tgt)
+    assert R.status() == 0
+    T = {k: R.tensor(k).astype(np.float32) for k in rf.ACTIVATIONS + rf.GRADIENTS}
+    R.close()
+
+    def bf16(x):
+        return torch.from_numpy(np.ascontiguousarray(x)).bfloat16().float().numpy()
+
+    def quad(x):  # the four pixels over each low-resolution one
+        return [x[:, k >> 1::2, k & 1::2] for k in range(4)]
+
+    for g, ca, y, dz in (("gu0", 32, "d1", "dz10"), ("gu1", 48, "d2", "dz9"), ("gu2", 64, "b3", "dz8")):
+        s = np.float32(0)
+        for q in quad(T[g][..., :ca]):
+            s = s + q
+        assert np.array_equal(T[dz], bf16(np.where(T[y] > 0, s, np.float32(0)))), dz
+        assert np.any(T[dz])
+    for g, ca, e, gp, dz in (("gu0", 32, "e0", "gp1", "dz2"), ("gu1", 48, "e1", "gp2", "dz4"),
+                             ("gu2", 64, "e2", "gp3", "dz6")):
+        ev, skip, got = quad(T[e]), quad(T[g][..., ca:]), quad(T[dz])
+        top, taken = np.maximum(np.maximum(ev[0], ev[1]), np.maximum(ev[2], ev[3])), np.zeros(ev[0].shape, bool)
+        for k in range(4):
+            mine = (ev[k] == top) & ~taken
+            taken |= mine
+            v = skip[k] + np.where(mine, T[gp], np.float32(0))
+            assert np.array_equal(got[k], bf16(np.where(ev[k] > 0, v, np.float32(0)))), (dz, k)
+        assert np.any(T[dz])
