@@ -117,54 +117,61 @@ __device__ __forceinline__ bool axis_z(const RayParams &p, float pt, float q, Ax
                     (unsigned)p.rb.voxels_size.x * (unsigned)p.rb.voxels_size.y, ax);
 }
 
-template <int FMT, bool STATS>
-__device__ __forceinline__ float trilinear(const void *vol, const RayParams &p, f3 pt) {
-    Axis X, Y, Z;
-    if (!axis_x(p, pt.x, pt.x / p.cell.x, X) || !axis_y(p, pt.y, pt.y / p.cell.y, Y) ||
-        !axis_z(p, pt.z, pt.z / p.cell.z, Z))
-        return __int_as_float(0x7fffffff);
-    return tri_corners<FMT, STATS>(vol, p, X, Y, Z);
-}
-
 // Zero crossing between time_curr and time_curr + step: secant refinement of
 // the hit and central-difference normal (raycast.cl:280-401).  Kept out of
 // line: it runs once per ray, and inlining it would bloat the march loop past
-// the instruction cache.
+// the instruction cache.  The samples' places are settled before their values
+// are read, so the reads of the two march samples, and then of the six normal
+// samples, are in flight together; a sample on the volume's border makes the
+// point, or the normal, NaN as a whole.
 template <int FMT, bool STATS>
 __device__ __noinline__ void refine_surface(const void *vol, const RayParams &p, f3 org, f3 dir, float time_curr,
                                             float &vx_out, float &vy_out, float &vz_out, float &nx_out,
                                             float &ny_out, float &nz_out) {
     const tde_point3i N = p.rb.voxels_size;
     const float step = p.time_step;
-    float ct = time_curr + step;
-    float Ftdt = trilinear<FMT, STATS>(vol, p, along(org, dir, ct));
-    if (isnan(Ftdt)) return;
-    float Ft = trilinear<FMT, STATS>(vol, p, along(org, dir, time_curr));
-    if (isnan(Ft)) return;
+    const f3 pa = along(org, dir, time_curr + step), pb = along(org, dir, time_curr);
+    const f3 qb{pb.x / p.cell.x, pb.y / p.cell.y, pb.z / p.cell.z};
+    Axis X, Y, Z, X2, Y2, Z2;
+    if (!axis_x(p, pa.x, pa.x / p.cell.x, X) || !axis_y(p, pa.y, pa.y / p.cell.y, Y) ||
+        !axis_z(p, pa.z, pa.z / p.cell.z, Z))
+        return;
+    // (a measurement reads as the reference does: one after the other)
+    if (STATS && isnan(tri_corners<FMT, STATS>(vol, p, X, Y, Z))) return;
+    if (!axis_x(p, pb.x, qb.x, X2) || !axis_y(p, pb.y, qb.y, Y2) || !axis_z(p, pb.z, qb.z, Z2)) return;
+    const float Ftdt = tri_corners<FMT, STATS>(vol, p, X, Y, Z);
+    const float Ft = tri_corners<FMT, STATS>(vol, p, X2, Y2, Z2);
+    if (isnan(Ftdt) || isnan(Ft)) return;
     float Ts = time_curr - step * Ft / (Ftdt - Ft);
     f3 vf = along(org, dir, Ts);
     vx_out = vf.x; vy_out = vf.y; vz_out = vf.z;
-    f3 p3 = along(org, dir, time_curr);
-    int hx = floor_sat(p3.x / p.cell.x), hy = floor_sat(p3.y / p.cell.y), hz = floor_sat(p3.z / p.cell.z);
+    int hx = floor_sat(qb.x), hy = floor_sat(qb.y), hz = floor_sat(qb.z);
     if (hx > 1 && hy > 1 && hz > 1 && hx < N.x - 2 && hy < N.y - 2 && hz < N.z - 2) {
         // vf +- cell on one axis: the other two axes are vf's
-        const float qnan = __int_as_float(0x7fffffff);
-        Axis X, Y, Z, A1, A2;
+        Axis P1, P2, Q1, Q2, R1, R2;
         const bool okx = axis_x(p, vf.x, vf.x / p.cell.x, X);
         const bool oky = axis_y(p, vf.y, vf.y / p.cell.y, Y);
         const bool okz = axis_z(p, vf.z, vf.z / p.cell.z, Z);
         float t1 = vf.x + p.cell.x, t2 = vf.x - p.cell.x;
-        const bool x1 = axis_x(p, t1, t1 / p.cell.x, A1), x2 = axis_x(p, t2, t2 / p.cell.x, A2);
-        const float Fx1 = (x1 && oky && okz) ? tri_corners<FMT, STATS>(vol, p, A1, Y, Z) : qnan;
-        const float Fx2 = (x2 && oky && okz) ? tri_corners<FMT, STATS>(vol, p, A2, Y, Z) : qnan;
+        const bool x1 = axis_x(p, t1, t1 / p.cell.x, P1), x2 = axis_x(p, t2, t2 / p.cell.x, P2);
         t1 = vf.y + p.cell.y; t2 = vf.y - p.cell.y;
-        const bool y1 = axis_y(p, t1, t1 / p.cell.y, A1), y2 = axis_y(p, t2, t2 / p.cell.y, A2);
-        const float Fy1 = (okx && y1 && okz) ? tri_corners<FMT, STATS>(vol, p, X, A1, Z) : qnan;
-        const float Fy2 = (okx && y2 && okz) ? tri_corners<FMT, STATS>(vol, p, X, A2, Z) : qnan;
+        const bool y1 = axis_y(p, t1, t1 / p.cell.y, Q1), y2 = axis_y(p, t2, t2 / p.cell.y, Q2);
         t1 = vf.z + p.cell.z; t2 = vf.z - p.cell.z;
-        const bool z1 = axis_z(p, t1, t1 / p.cell.z, A1), z2 = axis_z(p, t2, t2 / p.cell.z, A2);
-        const float Fz1 = (okx && oky && z1) ? tri_corners<FMT, STATS>(vol, p, X, Y, A1) : qnan;
-        const float Fz2 = (okx && oky && z2) ? tri_corners<FMT, STATS>(vol, p, X, Y, A2) : qnan;
+        const bool z1 = axis_z(p, t1, t1 / p.cell.z, R1), z2 = axis_z(p, t2, t2 / p.cell.z, R2);
+        if (!(okx && oky && okz && x1 && x2 && y1 && y2 && z1 && z2)) {
+            if (STATS) {
+                if (x1 && oky && okz) tri_corners<FMT, STATS>(vol, p, P1, Y, Z);
+                if (x2 && oky && okz) tri_corners<FMT, STATS>(vol, p, P2, Y, Z);
+                if (okx && y1 && okz) tri_corners<FMT, STATS>(vol, p, X, Q1, Z);
+                if (okx && y2 && okz) tri_corners<FMT, STATS>(vol, p, X, Q2, Z);
+                if (okx && oky && z1) tri_corners<FMT, STATS>(vol, p, X, Y, R1);
+                if (okx && oky && z2) tri_corners<FMT, STATS>(vol, p, X, Y, R2);
+            }
+            return;
+        }
+        const float Fx1 = tri_corners<FMT, STATS>(vol, p, P1, Y, Z), Fx2 = tri_corners<FMT, STATS>(vol, p, P2, Y, Z);
+        const float Fy1 = tri_corners<FMT, STATS>(vol, p, X, Q1, Z), Fy2 = tri_corners<FMT, STATS>(vol, p, X, Q2, Z);
+        const float Fz1 = tri_corners<FMT, STATS>(vol, p, X, Y, R1), Fz2 = tri_corners<FMT, STATS>(vol, p, X, Y, R2);
         f3 n = normalized(f3{Fx1 - Fx2, Fy1 - Fy2, Fz1 - Fz2});
         nx_out = n.x; ny_out = n.y; nz_out = n.z;
     }
@@ -238,11 +245,12 @@ __device__ __forceinline__ float advance(float tn, float step, float lim, float 
 // A block is a row of kRayWarps warps, a warp an 8 x 4 tile of pixels, so its rays
 // start close together and sample neighbouring voxels.  What bounds the kernel
 // at 640x480 / 512^3: its instructions (4000 a warp, 1600 of them the refinement's;
-// 66 % of the issue slots while an SM is busy) and the longest rays' chain of
+// two thirds of the issue slots while an SM is busy) and the longest rays' chain of
 // loads (an SM is busy for 100 to 140 thousand cycles; blocks of 1 to 8 warps end
 // within 5 % of each other).  The pipeline's cast: 97 us with byte flags read
-// sample by sample, 67 us with a word of flags a super-brick, rarer exact places
-// and four additions a round of `advance`.
+// sample by sample; 67 us with a word of flags a super-brick, rarer exact places
+// and four additions a round of `advance`; 63 us with strides across eight empty
+// bricks; 61 us with the refinement's reads together.
 constexpr int kRayWarps = 4;
 constexpr int kRayThreads = 32 * kRayWarps;
 constexpr int kRayBlockCols = 8 * kRayWarps, kRayBlockRows = 4;
@@ -252,10 +260,15 @@ constexpr int kRayBlockCols = 8 * kRayWarps, kRayBlockRows = 4;
 // a ray enters the super-brick in place of two dependent ones and one for each of
 // its bricks.
 enum FlagKind { FLAG_NONE, FLAG_BYTES, FLAG_MASKS };
+// Blocks an SM holds: without flags the march waits for records and wants warps
+// (86 us with 9, 93 with 7), with them the refinement's reads want registers (61 us
+// with 7, 64 with 9).
+constexpr int ray_blocks(FlagKind flags) { return flags == FLAG_NONE ? 9 : 7; }
 
 template <int FMT, FlagKind FLAGS, bool STATS>
-__global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__restrict__ vol, float *__restrict__ vmap,
-                                                     float *__restrict__ nmap, const __grid_constant__ RayParams p) {
+__global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
+    raycast_kernel(const void *__restrict__ vol, float *__restrict__ vmap, float *__restrict__ nmap,
+                   const __grid_constant__ RayParams p) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     allow_next_kernel();
@@ -387,20 +400,23 @@ __global__ void __launch_bounds__(kRayThreads) raycast_kernel(const void *__rest
             int py = sy + p.rb.origin_GRID.y; py -= py >= N.y ? N.y : 0;
             int pz = sz + p.rb.origin_GRID.z; pz -= pz >= N.z ? N.z : 0;
             const int sid = (px >> 5) + nsx * ((py >> 5) + nsy * (pz >> 5));
-            bool have;
+            bool have, empty_eight = false;
             if (FLAGS == FLAG_MASKS) {
                 if (sid != last_super) {
                     mask = __ldg(p.neg_masks + sid);
                     empty_super = mask == 0 && p.super_flags;
                 }
                 have = (mask >> (((px >> 3) & 3) | ((py >> 1) & 12) | ((pz << 1) & 48))) & 1;
+                // the eight bricks of the 16^3 corner of the super-brick that the sample is in
+                const int corner = ((px >> 3) & 2) | ((py >> 1) & 8) | ((pz << 1) & 32);
+                empty_eight = ((mask >> corner) & 0x330033ull) == 0 && p.super_flags;
             } else {
                 if (sid != last_super) empty_super = p.super_flags && !__ldg(p.super_flags + sid);
                 have = !empty_super && __ldg(p.neg_flags + ((px >> 3) + nbx * ((py >> 3) + nby * (pz >> 3)))) != 0;
             }
             last_super = sid;
             if (!have && !(known && tsdf < 0.f)) {
-                const int edge = empty_super ? 31 : 7;
+                const int edge = empty_super ? 31 : empty_eight ? 15 : 7;
                 const float lim = box_exit(rf, (float)(sx - (px & edge)), (float)(sy - (py & edge)),
                                            (float)(sz - (pz & edge)), (float)(edge + 1));
                 time_curr = advance(ct, step, lim, p.max_time);
