@@ -112,7 +112,8 @@ int tde_pipeline_stage_timings(tde_pipeline *p, float *ms, int capacity);
 /* Voxels read, voxels written and 8^3 bricks swept by integration since the
  * last reset, three counters (needs integrate_stats; synchronises). */
 int tde_pipeline_integrate_stats(tde_pipeline *p, uint64_t *read_written2, int reset);
-/* Number of kernel launches one tracked frame performs. */
+/* Number of kernel launches one tracked frame performs (without the one that
+ * writes pose_out12 and *status_out). */
 int tde_pipeline_launches_per_frame(tde_pipeline *p);
 
 /* Replace the volume origin bookkeeping after a cyclic shift (the caller has

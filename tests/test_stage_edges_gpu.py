@@ -262,3 +262,35 @@ def test_odometry_steps_in_a_cluster_and_in_launches(cuda, tde, orc, cols, rows,
             assert st == rg.STATUS_SOLVED
     assert status == rg.STATUS_SOLVED and np.array_equal(whole, single)
     assert not np.array_equal(whole, pose)
+
+
+def test_pose_reaches_any_host_memory(cuda, orc):
+    """The pose and status of enqueued frames in pinned memory, in pinned memory
+    off its alignment, and in memory that is not pinned: those of the blocking call."""
+    import torch
+    syn = importlib.import_module("3deye_gb300.synth")
+    pl = importlib.import_module("3deye_gb300.pipeline")
+    cfg = syn.small_config("c1", frames=5, cols=97, rows=61, voxels=64, fmt=2)
+    scene, traj = syn.make_scene(cfg, 1000), syn.make_trajectory(cfg, 2000)
+    intr = orc.Intr(cfg.fx, cfg.fy, cfg.cx, cfg.cy, cfg.cols, cfg.rows)
+    depths = [orc.apply_noise(orc.render_depth(scene, traj[i], intr), 3000, i) for i in range(cfg.frames)]
+    p = pl.Pipeline(cfg, traj[0])
+    ref = [p.process(d) for d in depths]
+    p.close()
+    host = torch.from_numpy(np.stack(depths).view(np.int16)).pin_memory()
+    pinned = torch.full((4096,), 77, dtype=torch.uint8).pin_memory()
+    plain = np.full(4096, 77, np.uint8)
+    for base, off in ((pinned.data_ptr(), 0), (pinned.data_ptr(), 3), (plain.ctypes.data, 8), (plain.ctypes.data, 1)):
+        p = pl.Pipeline(cfg, traj[0])
+        for i in range(cfg.frames):
+            p.enqueue(host[i].data_ptr(), False, base + off + 96 * i, base + 2048 + off + 4 * i)
+        p.sync()
+        got = (pinned.numpy() if base == pinned.data_ptr() else plain).copy()
+        pose = got[off:off + 96 * cfg.frames].view(np.float64).reshape(-1, 12)
+        status = got[2048 + off:2048 + off + 4 * cfg.frames].view(np.int32)
+        for i, (rp, rs) in enumerate(ref):
+            assert np.array_equal(pose[i], rp) and status[i] == rs
+        assert (got[off + 96 * cfg.frames:2048 + off] == 77).all() and (got[2048 + off + 4 * cfg.frames:] == 77).all()
+        p.close()
+        pinned.fill_(77)
+        plain[:] = 77
