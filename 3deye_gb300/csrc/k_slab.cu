@@ -435,10 +435,11 @@ __device__ __forceinline__ unsigned group_bits(const SlabParams &p, const RowGeo
 // its threads take a listed group each, with the +y and +z neighbour groups'
 // loads, so that all lanes of a warp work on such groups (evaluated where they
 // were loaded, a warp spent eight turns on a few lanes each: 204 us on a 512^3
-// volume holding a noisy band about the surfaces of one view, 134 us this way; its
-// records alone take 79 us).
+// volume holding a noisy band about the surfaces of one view, 124 us this way; its
+// records alone take 79 us).  Five blocks an SM: while some wait for their records
+// others evaluate (3: 139 us, 4: 134, 6, in 40 registers: 124).
 template <int FMT, bool ZONE, bool COLOR>
-__global__ void __launch_bounds__(kSlabThreads, 4) row_count_kernel(const SlabParams p, const RowGeom rg,
+__global__ void __launch_bounds__(kSlabThreads, 5) row_count_kernel(const SlabParams p, const RowGeom rg,
                                                                     uint32_t *__restrict__ counts) {
     __shared__ unsigned s_cnt[4];
     __shared__ unsigned s_n;
@@ -539,9 +540,11 @@ __device__ __forceinline__ int field(unsigned long long v, int q) { return (int)
 // shared memory; then the block writes the list, a point a thread: coalesced, the
 // weight and colour gathers of 32 points in flight together.  (Each thread writing
 // its own points one after the other, and every tile's bits read: 200 us on a 512^3
-// volume holding a noisy band about the surfaces of one view; 106 us now.)
+// volume holding a noisy band about the surfaces of one view; 78 us now.)  Eight
+// blocks an SM, short of registers as they are: a block's scan, ranks and gathers
+// are a chain that only other blocks cover (4: 103 us, 5: 91, 6: 85).
 template <int FMT, bool ZONE, bool COLOR>
-__global__ void __launch_bounds__(kSlabThreads, 4) row_scatter_kernel(const SlabParams p, const RowGeom rg,
+__global__ void __launch_bounds__(kSlabThreads, 8) row_scatter_kernel(const SlabParams p, const RowGeom rg,
                                                                   const Offsets offs, tde_xyzi *__restrict__ pts,
                                                                   tde_color *__restrict__ cols,
                                                                   float *__restrict__ wts, uint32_t capacity) {
