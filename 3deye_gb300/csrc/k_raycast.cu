@@ -271,8 +271,7 @@ __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
                    const __grid_constant__ RayParams p) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    allow_next_kernel();
-    wait_previous_kernel();
+    allow_next_kernel();  // (the resizes of its maps)
     const int x = blockIdx.x * kRayBlockCols + warp * 8 + (lane & 7);
     const int y = blockIdx.y * kRayBlockRows + (lane >> 3);
     const int W = p.intr.cols, H = p.intr.rows;
@@ -599,7 +598,7 @@ __global__ void transform_maps_kernel(const float *__restrict__ vs, const float 
 int launch_raycast(const void *volume, int format, float *vmap, float *nmap, const tde_point3f &t,
                    const tde_matrix3f &R, float trunc, const tde_intrinsics &intr, const tde_round_buffer &rb,
                    const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags,
-                   const unsigned long long *neg_masks, cudaStream_t stream, bool chained, unsigned *touched) {
+                   const unsigned long long *neg_masks, cudaStream_t stream, unsigned *touched) {
     RayParams p;
     p.dpose = dpose;
     p.neg_flags = neg_flags;
@@ -623,7 +622,9 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
             return neg_masks ? raycast_kernel<FM, FLAG_MASKS, ST>
                              : neg_flags ? raycast_kernel<FM, FLAG_BYTES, ST> : raycast_kernel<FM, FLAG_NONE, ST>;
         };
-        return launch_chained("raycast", chained, touched ? kernel(std::true_type{}) : kernel(std::false_type{}), grid,
+        // Not chained: it reads the volume and the flags through the read-only
+        // path, and a sweep, which lets its successor start, writes both.
+        return launch_chained("raycast", false, touched ? kernel(std::true_type{}) : kernel(std::false_type{}), grid,
                               block, stream, volume, vmap, nmap, p);
     });
 }

@@ -58,8 +58,10 @@ inline int cuda_fail(cudaError_t e, const char *what) {
 // returns once that one has completed and its writes are visible.  Every block
 // of a chained kernel waits, so its own completion implies its predecessor's;
 // what precedes the wait touches no memory, and buffers that the predecessor
-// writes are not read through the read-only path (whose loads the compiler may
-// move over the wait).
+// writes are not read through the read-only path (it is for memory that nothing
+// writes while the kernel runs, and the kernel runs from before the wait).  A kernel
+// that wants that path for such a buffer, as the raycast does for the volume, is
+// launched plainly; it may still let its own successor start.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
