@@ -830,8 +830,10 @@ const void *conv_kernel_fn(int mode, int cca, int ccb, bool pool) {
 //   warps 0-3 (producers): unit j goes to warp j & 3, two in flight each;
 //   warp 4 (MMA issuer): at unit u >= 2 the MMAs of output row u - 2, committed to
 //     the dZ slot and to the slot of the X row no later step reads;
-//   warps 5-8: sum dZ for the bias; at the end drain the accumulators, which
-//     stay in tensor memory across all the block's steps, into its partial.
+//   warps 5-8: sum dZ for the bias, waiting for dZ rows alone: a slot of X is
+//     released without them, so its phases could pass them by, where a dZ slot is
+//     filled again only after they have read it; at the end drain the accumulators,
+//     which stay in tensor memory across all the block's steps, into its partial.
 // Bounded waits as in the convolution.
 // ---------------------------------------------------------------------------
 constexpr int kWgProdWarps = 4, kWgMmaWarp = 4, kWgBiasWarps = 4;
@@ -860,7 +862,7 @@ __host__ __device__ constexpr int wg_mtiles(int cout) { return (3 * cout + 127) 
 __host__ __device__ constexpr int wg_partial(int cin, int cout) { return 9 * cin * cout + cout; }
 
 struct WgPipe {
-    uint64_t full[kWgMaxFlight + 3], empty[kWgMaxFlight + 3], zempty[kWgMaxFlight + 1], drain;
+    uint64_t full[kWgMaxFlight + 3], empty[kWgMaxFlight + 3], zfull[kWgMaxFlight + 1], zempty[kWgMaxFlight + 1], drain;
     uint32_t tmem;
     int abort;
 };
@@ -934,7 +936,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const WgradArgs
             tc::mbar_init(&pp.full[s], 1);
             tc::mbar_init(&pp.empty[s], 1);
         }
-        for (int s = 0; s < kDzSlots; ++s) tc::mbar_init(&pp.zempty[s], 1 + kWgBiasWarps);
+        for (int s = 0; s < kDzSlots; ++s) {
+            tc::mbar_init(&pp.zfull[s], 1);
+            tc::mbar_init(&pp.zempty[s], 1 + kWgBiasWarps);
+        }
         tc::mbar_init(&pp.drain, 1);
         pp.abort = 0;
     }
@@ -948,7 +953,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const WgradArgs
     if (warp < kWgProdWarps) {
         // ---- producers ----
         uint32_t j = 0, jz = 0;  // units and dZ rows of this block so far
-        int pending = -1;
+        int pending = -1, zpending = -1;  // slots of the unit issued before the current one
         bool ok = true;
         auto publish = [&](int wait_groups) {
             if (pending < 0) return;
@@ -956,8 +961,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const WgradArgs
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
             tc::fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&pp.full[pending]);
-            pending = -1;
+            if (lane == 0) {
+                mbar_arrive(&pp.full[pending]);
+                if (zpending >= 0) mbar_arrive(&pp.zfull[zpending]);
+            }
+            pending = zpending = -1;
         };
         auto wait_empty = [&](uint64_t *bar, uint32_t k) {
             if (k == 0 || tc::mbar_test_wait(bar, (k - 1) & 1u)) return true;
@@ -999,6 +1007,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const WgradArgs
                 asm volatile("cp.async.commit_group;" ::: "memory");
                 publish(1);
                 pending = (int)s;
+                zpending = has_z ? (int)sz : -1;
                 jz += has_z;
             }
             step += n;
@@ -1070,32 +1079,23 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const WgradArgs
         for (int c = 0; c < CT; ++c)
 #pragma unroll
             for (int e = 0; e < 8; ++e) sum[c][e] = 0.f;
-        uint32_t slot = 0, sphase = 0, zslot = 0;
-        bool ok = true;
-        for (int step = s0; step < s1 && ok;) {
-            const WgRun run = wg_run<KP>(A, step, s1);
-            const int n = run.y1 - run.y0;
-            for (int u = 0; u < n + 2; ++u) {
-                if (!(ok = pipe_wait(&pp.full[slot], sphase, abort, A.err))) break;
-                if (u >= 2) {
-                    const unsigned char *z = zring + zslot * zbytes + CZ * kPlane + px * 16;  // copy dx = 1
+        uint32_t zslot = 0, zphase = 0;
+        for (int step = s0; step < s1; ++step) {
+            if (!pipe_wait(&pp.zfull[zslot], zphase, abort, A.err)) break;
+            const unsigned char *z = zring + zslot * zbytes + CZ * kPlane + px * 16;  // copy dx = 1
 #pragma unroll
-                    for (int c = 0; c < CT; ++c) {
-                        float f[8];
-                        unpack8(*reinterpret_cast<const uint4 *>(z + (c0 + GR * c) * kPlane), f);
+            for (int c = 0; c < CT; ++c) {
+                float f[8];
+                unpack8(*reinterpret_cast<const uint4 *>(z + (c0 + GR * c) * kPlane), f);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) sum[c][e] += f[e];
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&pp.zempty[zslot]);
-                    if (++zslot == (uint32_t)kDzSlots) zslot = 0;
-                }
-                if (++slot == (uint32_t)kRowSlots) {
-                    slot = 0;
-                    sphase ^= 1u;
-                }
+                for (int e = 0; e < 8; ++e) sum[c][e] += f[e];
             }
-            step += n;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&pp.zempty[zslot]);
+            if (++zslot == (uint32_t)kDzSlots) {
+                zslot = 0;
+                zphase ^= 1u;
+            }
         }
         // over the warp's 32 pixels (the warps of a chunk are added below)
         const int wb = warp - kWgMmaWarp - 1;
