@@ -23,7 +23,7 @@ struct RayParams {
     size_t n;               // voxel count (F32 plane offset)
     const CamPose *dpose;   // when set, t and R are read from here
     const uint8_t *neg_flags;  // per physical 8^3 brick: 0 = holds no negative value
-    const uint8_t *super_flags;  // per physical 32^3 super-brick (null: no sample skipping)
+    const uint8_t *super_flags;  // per physical 32^3 super-brick (whole ones only)
     const unsigned long long *neg_masks;  // the brick flags as one word per super-brick (FLAG_MASKS)
     float inv_cell[3];
     unsigned *touched;      // measurement runs: one bit per voxel record read
@@ -194,14 +194,15 @@ struct RayFast {
     float margin;      // voxels
 };
 
-// Time at which the ray (fast coordinates) leaves the box [lo, lo + size)^3
+// Time at which the ray (fast coordinates) leaves the box [lo, lo + size)
 // shrunk by kSkipMargin voxels on every side: the last time a sample may take
 // and still lie inside the box (the fast coordinates' error is far below the
 // margin).
-__device__ __forceinline__ float box_exit(const RayFast &rf, float lox, float loy, float loz, float size) {
-    const float ex = ((rf.d[0] > 0.f ? lox + (size - kSkipMargin) : lox + kSkipMargin) - rf.o[0]) * rf.inv_d[0];
-    const float ey = ((rf.d[1] > 0.f ? loy + (size - kSkipMargin) : loy + kSkipMargin) - rf.o[1]) * rf.inv_d[1];
-    const float ez = ((rf.d[2] > 0.f ? loz + (size - kSkipMargin) : loz + kSkipMargin) - rf.o[2]) * rf.inv_d[2];
+__device__ __forceinline__ float box_exit(const RayFast &rf, float lox, float loy, float loz, float sx, float sy,
+                                         float sz) {
+    const float ex = ((rf.d[0] > 0.f ? lox + (sx - kSkipMargin) : lox + kSkipMargin) - rf.o[0]) * rf.inv_d[0];
+    const float ey = ((rf.d[1] > 0.f ? loy + (sy - kSkipMargin) : loy + kSkipMargin) - rf.o[1]) * rf.inv_d[1];
+    const float ez = ((rf.d[2] > 0.f ? loz + (sz - kSkipMargin) : loz + kSkipMargin) - rf.o[2]) * rf.inv_d[2];
     return fminf(fminf(ex, ey), ez);
 }
 
@@ -265,7 +266,10 @@ enum FlagKind { FLAG_NONE, FLAG_BYTES, FLAG_MASKS };
 // with 7, 64 with 9).
 constexpr int ray_blocks(FlagKind flags) { return flags == FLAG_NONE ? 9 : 7; }
 
-template <int FMT, FlagKind FLAGS, bool STATS>
+// WHOLE: every axis is whole super-bricks, which strides across more than a brick
+// need.  (Asked of the parameters at each stride it cost a 640x480 frame of a 512^3
+// pipeline 1 us.)
+template <int FMT, FlagKind FLAGS, bool WHOLE, bool STATS>
 __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
     raycast_kernel(const void *__restrict__ vol, float *__restrict__ vmap, float *__restrict__ nmap,
                    const __grid_constant__ RayParams p) {
@@ -403,21 +407,29 @@ __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
             if (FLAGS == FLAG_MASKS) {
                 if (sid != last_super) {
                     mask = __ldg(p.neg_masks + sid);
-                    empty_super = mask == 0 && p.super_flags;
+                    empty_super = WHOLE && mask == 0;
                 }
                 have = (mask >> (((px >> 3) & 3) | ((py >> 1) & 12) | ((pz << 1) & 48))) & 1;
                 // the eight bricks of the 16^3 corner of the super-brick that the sample is in
                 const int corner = ((px >> 3) & 2) | ((py >> 1) & 8) | ((pz << 1) & 32);
-                empty_eight = ((mask >> corner) & 0x330033ull) == 0 && p.super_flags;
+                empty_eight = WHOLE && ((mask >> corner) & 0x330033ull) == 0;
             } else {
-                if (sid != last_super) empty_super = p.super_flags && !__ldg(p.super_flags + sid);
+                if (WHOLE && sid != last_super) empty_super = !__ldg(p.super_flags + sid);
                 have = !empty_super && __ldg(p.neg_flags + ((px >> 3) + nbx * ((py >> 3) + nby * (pz >> 3)))) != 0;
             }
             last_super = sid;
             if (!have && !(known && tsdf < 0.f)) {
                 const int edge = empty_super ? 31 : empty_eight ? 15 : 7;
+                float bx = (float)(edge + 1), by = bx, bz = bx;
+                if (!WHOLE) {
+                    // the last brick of an axis that is not whole bricks is shorter, and
+                    // across the origin another one's voxels follow it inside the volume
+                    bx = fminf(bx, (float)(N.x - (px & ~7)));
+                    by = fminf(by, (float)(N.y - (py & ~7)));
+                    bz = fminf(bz, (float)(N.z - (pz & ~7)));
+                }
                 const float lim = box_exit(rf, (float)(sx - (px & edge)), (float)(sy - (py & edge)),
-                                           (float)(sz - (pz & edge)), (float)(edge + 1));
+                                           (float)(sz - (pz & edge)), bx, by, bz);
                 time_curr = advance(ct, step, lim, p.max_time);
                 known = false;
                 prev_ct = time_curr;
@@ -607,9 +619,7 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
     p.max_time = 3.f * ((rb.volume_size.x + rb.volume_size.y) + rb.volume_size.z);
     p.intr = intr; p.rb = rb; p.cell = cell; p.n = voxel_count(rb);
     p.inv_cell[0] = 1.f / cell.x; p.inv_cell[1] = 1.f / cell.y; p.inv_cell[2] = 1.f / cell.z;
-    // super-brick sample skipping needs whole 32^3 super-bricks on every axis
     const bool whole = rb.voxels_size.x % 32 == 0 && rb.voxels_size.y % 32 == 0 && rb.voxels_size.z % 32 == 0;
-    // (with masks only asked whether it is null)
     p.super_flags = (neg_flags && whole) ? neg_flags + brick_count(rb) : nullptr;
     p.neg_masks = neg_masks;
     p.touched = touched;
@@ -619,8 +629,11 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
         constexpr int FM = decltype(F)::value;
         const auto kernel = [&](auto stats) {
             constexpr bool ST = decltype(stats)::value;
-            return neg_masks ? raycast_kernel<FM, FLAG_MASKS, ST>
-                             : neg_flags ? raycast_kernel<FM, FLAG_BYTES, ST> : raycast_kernel<FM, FLAG_NONE, ST>;
+            if (neg_masks)
+                return whole ? raycast_kernel<FM, FLAG_MASKS, true, ST> : raycast_kernel<FM, FLAG_MASKS, false, ST>;
+            if (neg_flags)
+                return whole ? raycast_kernel<FM, FLAG_BYTES, true, ST> : raycast_kernel<FM, FLAG_BYTES, false, ST>;
+            return raycast_kernel<FM, FLAG_NONE, false, ST>;
         };
         // Not chained: it reads the volume and the flags through the read-only
         // path, and a sweep, which lets its successor start, writes both.
