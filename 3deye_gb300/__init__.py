@@ -108,7 +108,7 @@ def estimate_combined(vcur, ncur, vprev, nprev, R_cur, t_cur, R_prev_inv, t_prev
                                     C.byref(Rp), C.byref(tp), C.byref(intr), dist_thresh, angle_thresh, ptr(g),
                                     ptr(m), stream_ptr(stream)))
     if stream is not None and stream != torch.cuda.current_stream():
-        stream.synchronize()  # the scratch and the result belong to the current stream
+        stream.synchronize()  # the scratch and the result belong to the current stream: not for a capture on another
     return m
 
 

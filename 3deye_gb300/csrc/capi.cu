@@ -192,7 +192,14 @@ int tde_estimate_combined(const float *vmap_cur, const float *nmap_cur, const fl
     a.W = intr->cols; a.H = intr->rows;
     a.fx = intr->fx; a.fy = intr->fy; a.cx = intr->cx; a.cy = intr->cy;
     icp_set_thresholds(a, dist_thresh, angle_thresh);
-    return launch_icp(a, pose, st, mbuf, s);
+    TDE_TRY(launch_icp(a, pose, st, mbuf, s));
+    // The sums are there, and the scratch is the caller's again, when this returns:
+    // callers read the one from other streams and free or reuse the other, and get
+    // the kernels' errors here.  (A captured call has nothing to wait for.)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TDE_CUDA(cudaStreamIsCapturing(s, &capture), "estimate_combined");
+    if (capture == cudaStreamCaptureStatusNone) TDE_CUDA(cudaStreamSynchronize(s), "estimate_combined");
+    return TDE_OK;
 }
 
 int tde_transform_estimation(const float *gbuf, float *out, int buf_length, int group_stride, void *stream) {

@@ -260,9 +260,9 @@ __device__ __forceinline__ void load_current(const IcpArgs &a, float3 (&nc)[PIX]
 }
 
 // One-shot sums (the Estimate_Combined drop-in) for a pose given by value: the
-// caller's scratch needs no upload and the call no wait (a 6 KB state copied from
-// pageable memory and the stream synchronised after it made the call 26 us at
-// 640x480, of which the kernel was 9).  The accumulators of the scratch start
+// caller's scratch needs no upload of a 6 KB state from pageable memory (27 us a
+// call with it at 640x480, 25 now: the kernel's 9, its launch and the call's wait
+// for it; 11 where calls did not wait).  The accumulators of the scratch start
 // undefined: clear_sums_kernel zeroes them while this grid, launched with
 // programmatic serialisation, loads its maps.  The last block writes the exact
 // totals to st->sums / mbuf.

@@ -155,8 +155,9 @@ size_t tde_estimate_combined_gbuf_floats(int cols, int rows);
  * metres or with sin(angle) >= angle_thresh.  Writes the 27 sums
  * [A00..A05 b0 A11..A15 b1 ... A55 b5] (the unpack order of
  * opencl_wrappers.cpp:426-437) to mbuf (device, 27 floats), using gbuf
- * (device, tde_estimate_combined_gbuf_floats floats) as scratch until the work
- * enqueued on the stream is done.
+ * (device, tde_estimate_combined_gbuf_floats floats) as scratch.  Waits for the
+ * stream: the sums are in mbuf and gbuf is free when it returns (while the stream
+ * is being captured it only records).
  * Sums are compensated FP32. */
 int tde_estimate_combined(const float *vmap_cur, const float *nmap_cur, const float *vmap_prev_g,
                           const float *nmap_prev_g, const tde_matrix3f *R_cur, const tde_point3f *t_cur,
