@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
     const int warp = tid >> 5, lane = tid & 31;
     allow_next_kernel();  // (the resizes of its maps)
     const int x = blockIdx.x * kRayBlockCols + warp * 8 + (lane & 7);
-    const int y = blockIdx.y * kRayBlockRows + (lane >> 3);
+    const int y = (int)(blockIdx.z * gridDim.y + blockIdx.y) * kRayBlockRows + (lane >> 3);
     const int W = p.intr.cols, H = p.intr.rows;
     // the pose: from the parameters, or read on the device
     tde_matrix3f R = p.R;
@@ -624,7 +624,9 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
     p.neg_masks = neg_masks;
     p.touched = touched;
     dim3 block(kRayThreads);
-    dim3 grid(div_up(intr.cols, kRayBlockCols), div_up(intr.rows, kRayBlockRows));
+    // a grid takes 65,535 blocks of rows; images of more come in layers
+    const unsigned row_blocks = div_up(intr.rows, kRayBlockRows), layers = div_up(row_blocks, 65535u);
+    dim3 grid(div_up(intr.cols, kRayBlockCols), div_up(row_blocks, layers), layers);
     return dispatch_format(format, [&](auto F) {
         constexpr int FM = decltype(F)::value;
         const auto kernel = [&](auto stats) {

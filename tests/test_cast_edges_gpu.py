@@ -180,3 +180,31 @@ def test_model_maps_behind_a_short_brick(cuda, tde, fmt, voxels):
                 assert np.isfinite(ref[0]).any()
                 assert np.array_equal(got.view(np.uint32), ref.view(np.uint32)), (axis, toward, at)
     p.close()
+
+
+@pytest.mark.parametrize("cols,rows", [(1, 262140), (1, 262141), (2, 300001)])
+def test_cast_of_a_very_tall_image(cuda, tde, cols, rows):
+    """Images of more rows than a grid has blocks for (65,535 of four rows): their
+    maps hold the rows of short images that look the same way."""
+    import torch
+    L = _declare(tde)
+    n, cell = 40, np.float32(0.0625)
+    vol, _ = _plane((n,) * 3, 2, 21.61, 1, 1)
+    dv = torch.from_numpy(vol.copy()).to(cuda)
+    rb = tde.round_buffer((n,) * 3, (float(n * cell),) * 3, (n // 2,) * 3)
+    R, t, cs = tde.mat3(np.eye(3)), tde.vec3([n * cell / 2, n * cell / 2, 1.5 * cell]), tde.vec3([cell] * 3)
+
+    def cast(first, count):
+        it = tde.Intrinsics(2.0 * rows, 2.0 * rows, 0.0, float(rows // 2 - first), cols, count)
+        m = torch.full((2, count, cols, 3), 7.0, device=cuda)
+        torch.cuda.synchronize()
+        tde.check(L.tde_raycast_ex(dv.data_ptr(), 1, m[0].data_ptr(), m[1].data_ptr(), C.byref(t), C.byref(R), 0.0625,
+                                   C.byref(it), C.byref(rb), C.byref(cs), None, None))
+        torch.cuda.synchronize()
+        return m.cpu().numpy()
+
+    tall = cast(0, rows)
+    assert np.isfinite(tall[0]).all()
+    for first in (0, rows // 2, 262140 - 37, rows - 64):
+        count = min(64, rows - first)
+        assert np.array_equal(tall[:, first:first + count].view(np.uint32), cast(first, count).view(np.uint32))
