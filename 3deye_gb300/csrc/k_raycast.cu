@@ -57,7 +57,7 @@ __device__ __forceinline__ int floor_sat(float v) { return __float2int_rd(v); } 
 template <int FMT, bool STATS>
 __device__ __forceinline__ float load_rec(const void *vol, const RayParams &p, size_t addr) {
     if (STATS) atomicOr(p.touched + (addr >> 5), 1u << (addr & 31));
-    return TsdfStore<FMT>::value_ro(vol, addr, p.n);
+    return TsdfStore<FMT>::value(vol, addr, p.n);
 }
 
 template <int FMT, bool STATS>
@@ -271,11 +271,11 @@ constexpr int ray_blocks(FlagKind flags) { return flags == FLAG_NONE ? 9 : 7; }
 // pipeline 1 us.)
 template <int FMT, FlagKind FLAGS, bool WHOLE, bool STATS>
 __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
-    raycast_kernel(const void *__restrict__ vol, float *__restrict__ vmap, float *__restrict__ nmap,
-                   const __grid_constant__ RayParams p) {
+    raycast_kernel(const void *vol, float *vmap, float *nmap, const __grid_constant__ RayParams p) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    allow_next_kernel();  // (the resizes of its maps)
+    allow_next_kernel();
+    wait_previous_kernel();
     const int x = blockIdx.x * kRayBlockCols + warp * 8 + (lane & 7);
     const int y = (int)(blockIdx.z * gridDim.y + blockIdx.y) * kRayBlockRows + (lane >> 3);
     const int W = p.intr.cols, H = p.intr.rows;
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
             bool have, empty_eight = false;
             if (FLAGS == FLAG_MASKS) {
                 if (sid != last_super) {
-                    mask = __ldg(p.neg_masks + sid);
+                    mask = p.neg_masks[sid];
                     empty_super = WHOLE && mask == 0;
                 }
                 have = (mask >> (((px >> 3) & 3) | ((py >> 1) & 12) | ((pz << 1) & 48))) & 1;
@@ -414,8 +414,8 @@ __global__ void __launch_bounds__(kRayThreads, ray_blocks(FLAGS))
                 const int corner = ((px >> 3) & 2) | ((py >> 1) & 8) | ((pz << 1) & 32);
                 empty_eight = WHOLE && ((mask >> corner) & 0x330033ull) == 0;
             } else {
-                if (WHOLE && sid != last_super) empty_super = !__ldg(p.super_flags + sid);
-                have = !empty_super && __ldg(p.neg_flags + ((px >> 3) + nbx * ((py >> 3) + nby * (pz >> 3)))) != 0;
+                if (WHOLE && sid != last_super) empty_super = !p.super_flags[sid];
+                have = !empty_super && p.neg_flags[(px >> 3) + nbx * ((py >> 3) + nby * (pz >> 3))] != 0;
             }
             last_super = sid;
             if (!have && !(known && tsdf < 0.f)) {
@@ -610,7 +610,7 @@ __global__ void transform_maps_kernel(const float *__restrict__ vs, const float 
 int launch_raycast(const void *volume, int format, float *vmap, float *nmap, const tde_point3f &t,
                    const tde_matrix3f &R, float trunc, const tde_intrinsics &intr, const tde_round_buffer &rb,
                    const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags,
-                   const unsigned long long *neg_masks, cudaStream_t stream, unsigned *touched) {
+                   const unsigned long long *neg_masks, cudaStream_t stream, bool chained, unsigned *touched) {
     RayParams p;
     p.dpose = dpose;
     p.neg_flags = neg_flags;
@@ -637,9 +637,7 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
                 return whole ? raycast_kernel<FM, FLAG_BYTES, true, ST> : raycast_kernel<FM, FLAG_BYTES, false, ST>;
             return raycast_kernel<FM, FLAG_NONE, false, ST>;
         };
-        // Not chained: it reads the volume and the flags through the read-only
-        // path, and a sweep, which lets its successor start, writes both.
-        return launch_chained("raycast", false, touched ? kernel(std::true_type{}) : kernel(std::false_type{}), grid,
+        return launch_chained("raycast", chained, touched ? kernel(std::true_type{}) : kernel(std::false_type{}), grid,
                               block, stream, volume, vmap, nmap, p);
     });
 }

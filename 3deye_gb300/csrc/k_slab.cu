@@ -49,7 +49,7 @@ __device__ __forceinline__ bool color_set(tde_color c) { return (c.r | c.g | c.b
 template <int FMT>
 __device__ __forceinline__ void fetch(const SlabParams &p, int x, int y, int z, float &f, int &w) {
     typedef TsdfStore<FMT> S;
-    S::decode(S::load_raw(p.vol, voxel_address(x, y, z, p.rb), p.n), f, w);
+    S::decode(S::load_raw_ro(p.vol, voxel_address(x, y, z, p.rb), p.n), f, w);
 }
 __device__ __forceinline__ bool crossing(float F, float Fn, int Wn) {
     return (Wn != 0 && Fn != 1.f) && ((F > 0 && Fn < 0) || (F < 0 && Fn > 0));
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kSlabThreads) slab_scatter_kernel(const SlabPa
             if (cols) cols[slot] = p.color ? p.color[a] : tde_color{0, 0, 0, 0};
             if (wts) {
                 float f; int w;
-                TsdfStore<FMT>::decode(TsdfStore<FMT>::load_raw(p.vol, a, p.n), f, w);
+                TsdfStore<FMT>::decode(TsdfStore<FMT>::load_raw_ro(p.vol, a, p.n), f, w);
                 wts[slot] = (float)w;
             }
         }
@@ -405,7 +405,7 @@ __device__ __forceinline__ unsigned group_bits(const SlabParams &p, const RowGeo
         int wx3 = 0;
         if (live[3] && x0 + 3 != rg.xlast) {
             const int xn = x0 + 4 == W ? 0 : x0 + 4;
-            TsdfStore<FMT>::decode(TsdfStore<FMT>::load_raw(p.vol, row + xn, p.n), fx3, wx3);
+            TsdfStore<FMT>::decode(TsdfStore<FMT>::load_raw_ro(p.vol, row + xn, p.n), fx3, wx3);
         }
         #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kSlabThreads, 8) row_scatter_kernel(const Slab
                 if (cols) cols[slot] = COLOR ? p.color[a] : tde_color{0, 0, 0, 0};
                 if (wts) {
                     float f; int w;
-                    TsdfStore<FMT>::decode(TsdfStore<FMT>::load_raw(p.vol, a, p.n), f, w);
+                    TsdfStore<FMT>::decode(TsdfStore<FMT>::load_raw_ro(p.vol, a, p.n), f, w);
                     wts[slot] = (float)w;
                 }
             }

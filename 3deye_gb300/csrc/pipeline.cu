@@ -174,7 +174,7 @@ int cast_model(tde_pipeline *p, cudaStream_t s) {
     tde_point3f t0{0, 0, 0};
     tde_matrix3f R0{};
     return launch_raycast(p->volume, c.tsdf_format, p->vmod[0], p->nmod[0], t0, R0, c.trunc, p->intr[0], p->rb, p->cell,
-                          p->cam, p->negflags, p->negmasks, s);
+                          p->cam, p->negflags, p->negmasks, s, false);
 }
 
 // Records one segment for input set `set` onto stream s.
@@ -911,7 +911,7 @@ int tde_pipeline_raycast_records(tde_pipeline *p, int skip_empty, uint64_t *reco
         tde_matrix3f R0{};
         st = launch_raycast(p->volume, p->cfg.tsdf_format, vm, nm, t0, R0, p->cfg.trunc, p->intr[0], p->rb, p->cell,
                             p->cam, skip_empty ? p->negflags : nullptr, skip_empty ? p->negmasks : nullptr, p->stream,
-                            bits);
+                            false, bits);
         if (st == TDE_OK) {
             popcount_kernel<<<1024, 256, 0, p->stream>>>(bits, words, cnt);
             unsigned long long h = 0;

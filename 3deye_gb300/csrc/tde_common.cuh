@@ -59,9 +59,7 @@ inline int cuda_fail(cudaError_t e, const char *what) {
 // of a chained kernel waits, so its own completion implies its predecessor's;
 // what precedes the wait touches no memory, and buffers that the predecessor
 // writes are not read through the read-only path (it is for memory that nothing
-// writes while the kernel runs, and the kernel runs from before the wait).  A kernel
-// that wants that path for such a buffer, as the raycast does for the volume, is
-// launched plainly; it may still let its own successor start.
+// writes while the kernel runs, and the kernel runs from before the wait).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -129,12 +127,11 @@ template <> struct TsdfStore<TDE_TSDF_I16> {
         int v = reinterpret_cast<const tde_tsdf_i16 *>(base)[i].value;
         return (float)v / (float)TDE_MAX_DEPTH_VALUE;
     }
-    // value() through the read-only path (the volume must not change during the kernel)
-    __device__ __forceinline__ static float value_ro(const void *base, size_t i, size_t) {
-        int v = __ldg(reinterpret_cast<const short *>(base) + 2 * i);
-        return (float)v / (float)TDE_MAX_DEPTH_VALUE;
-    }
     __device__ __forceinline__ static Raw load_raw(const void *base, size_t i, size_t) {
+        return reinterpret_cast<const uint32_t *>(base)[i];
+    }
+    // load_raw() through the read-only path: the volume must not change during the kernel
+    __device__ __forceinline__ static Raw load_raw_ro(const void *base, size_t i, size_t) {
         return __ldg(reinterpret_cast<const uint32_t *>(base) + i);
     }
     __device__ __forceinline__ static void decode(Raw raw, float &f, int &w) {
@@ -163,10 +160,11 @@ template <> struct TsdfStore<TDE_TSDF_F16> {
     __device__ __forceinline__ static float value(const void *base, size_t i, size_t) {
         return __half2float(reinterpret_cast<const __half *>(base)[2 * i]);
     }
-    __device__ __forceinline__ static float value_ro(const void *base, size_t i, size_t) {
-        return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(base) + 2 * i)));
-    }
     __device__ __forceinline__ static Raw load_raw(const void *base, size_t i, size_t) {
+        return reinterpret_cast<const uint32_t *>(base)[i];
+    }
+    // load_raw() through the read-only path: the volume must not change during the kernel
+    __device__ __forceinline__ static Raw load_raw_ro(const void *base, size_t i, size_t) {
         return __ldg(reinterpret_cast<const uint32_t *>(base) + i);
     }
     __device__ __forceinline__ static void decode(Raw raw, float &f, int &w) {
@@ -193,13 +191,13 @@ template <> struct TsdfStore<TDE_TSDF_F32> {
     __device__ __forceinline__ static float value(const void *base, size_t i, size_t) {
         return reinterpret_cast<const float *>(base)[i];
     }
-    __device__ __forceinline__ static float value_ro(const void *base, size_t i, size_t) {
-        return __ldg(reinterpret_cast<const float *>(base) + i);
-    }
     __device__ __forceinline__ static const unsigned short *wplane(const void *base, size_t n) {
         return reinterpret_cast<const unsigned short *>(reinterpret_cast<const float *>(base) + n);
     }
     __device__ __forceinline__ static Raw load_raw(const void *base, size_t i, size_t n) {
+        return Raw{reinterpret_cast<const float *>(base)[i], (int)wplane(base, n)[i]};
+    }
+    __device__ __forceinline__ static Raw load_raw_ro(const void *base, size_t i, size_t n) {
         return Raw{__ldg(reinterpret_cast<const float *>(base) + i), (int)__ldg(wplane(base, n) + i)};
     }
     __device__ __forceinline__ static void decode(Raw raw, float &f, int &w) { f = raw.f; w = raw.w; }

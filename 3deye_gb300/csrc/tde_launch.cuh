@@ -21,7 +21,7 @@ int launch_raycast(const void *volume, int format, float *vmap, float *nmap, con
                    const tde_matrix3f &R, float trunc, const tde_intrinsics &intr, const tde_round_buffer &rb,
                    const tde_point3f &cell, const CamPose *dpose, const uint8_t *neg_flags,
                    const unsigned long long *neg_masks,  // the flags' masks (read in their place), or null
-                   cudaStream_t stream,
+                   cudaStream_t stream, bool chained = true,
                    unsigned *touched = nullptr);  // touched: measurement bitmap of records read, or null
 int launch_resize_map(const float *src, float *dst, int sc, int sr, bool normal, cudaStream_t stream);
 // Vertex and normal maps of level 0 (c0 x r0) -> levels 1 and (v2, n2 not

@@ -37,7 +37,10 @@ def test_a_waiting_kernel_reads_its_predecessors_buffers_coherently():
             waiting.add(name)
             ro = {p.split()[-1].lstrip("*") for p in params.split(",")
                   if re.search(r"\bconst\b[^*]*\*\s*__restrict__", p)}
-            ro |= set(re.findall(r"__ldg\(\s*&?(\w+)", body))
+            ro |= set(re.findall(r"__ldg\(\s*&?([\w.]+)", body)) | set(re.findall(r"\w+_ro\b", body))
             assert ro <= UNCHANGED.get(name, set()), (name, ro)
     assert {"raycast_kernel", "integrate_bricks_kernel", "resize_map_kernel", "bilateral_kernel"} <= found
-    assert {"integrate_bricks_kernel", "cull_bricks_kernel", "resize_map_kernel", "normal_map_kernel"} <= waiting
+    assert {"integrate_bricks_kernel", "cull_bricks_kernel", "raycast_kernel", "resize_map_kernel"} <= waiting
+    # the records that a sweep writes and a cast behind it reads, inside the functions they call
+    for f in ("k_raycast.cu", "k_integrate.cu"):
+        assert not re.search(r"\w+_ro\s*\(", (CSRC / f).read_text()), f
