@@ -1327,8 +1327,8 @@ __global__ void __launch_bounds__(128) conv_in_kernel(const uint16_t *__restrict
 // pixel's features again: 413 us at batch 16 of 640x480; 212 us now.)
 // Row strides of 72 words put a warp's eight distinct reads into different banks.
 constexpr int kInPartial = 16 * (kInK + 1);
-constexpr int kInTile = 64, kInStride = 72, kInMaxBlocks = 608;  // four blocks for each of 152 SMs
-__global__ void __launch_bounds__(256, 4) conv_in_wgrad_kernel(const float *__restrict__ depth_m,
+constexpr int kInTile = 64, kInStride = 72, kInBlocksPerSM = 4;
+__global__ void __launch_bounds__(256, kInBlocksPerSM) conv_in_wgrad_kernel(const float *__restrict__ depth_m,
                                                             const bf16 *__restrict__ dz1, int n, int h, int w,
                                                             float *__restrict__ partial) {
     __shared__ __align__(16) float F[kInK + 1][kInStride], G[16][kInStride];
@@ -1805,9 +1805,9 @@ int launch_conv_in(const uint16_t *raw, float *depth_m, const float *w1, const f
     return check_launch("refiner conv_in");
 }
 
-int conv_in_wgrad_blocks(int n, int h, int w) {
-    const size_t tiles = (size_t)n * h * ((w + kInTile - 1) / kInTile);
-    return (int)(tiles < (size_t)kInMaxBlocks ? tiles : (size_t)kInMaxBlocks);
+int conv_in_wgrad_blocks(int num_sms, int n, int h, int w) {
+    const size_t tiles = (size_t)n * h * ((w + kInTile - 1) / kInTile), resident = (size_t)num_sms * kInBlocksPerSM;
+    return (int)(tiles < resident ? tiles : resident);
 }
 
 int launch_conv_in_wgrad(const float *depth_m, const bf16 *dz1, int n, int h, int w, float *partial, int blocks,

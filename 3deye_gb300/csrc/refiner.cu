@@ -242,7 +242,8 @@ int loss_grad(tde_refiner *r, const uint16_t *raw, const uint16_t *target, int n
                                          h * 2, w * 2, s));
         }
     }
-    TDE_TRY(launch_conv_in_wgrad(r->depth_m, r->gr[G_DZ1], n, H, W, r->in_partial, conv_in_wgrad_blocks(n, H, W),
+    TDE_TRY(launch_conv_in_wgrad(r->depth_m, r->gr[G_DZ1], n, H, W, r->in_partial,
+                                 conv_in_wgrad_blocks(r->num_sms, n, H, W),
                                  r->grad + kL.c1w, r->grad + kL.c1b, s));
     return TDE_OK;
 }
@@ -292,7 +293,7 @@ int tde_refiner_create(int max_batch, int rows, int cols, uint64_t seed, tde_ref
             (st = dalloc(r, &r->v, P)) || (st = dalloc(r, &r->decay, P)) || (st = dalloc(r, &r->wq, kL.wq_total)) ||
             (st = dalloc(r, &r->wt, kL.wq_total)) || (st = dalloc(r, &r->depth_m, pixels(r, max_batch, 0))) ||
             (st = dalloc(r, &r->out_m, pixels(r, max_batch, 0))) || (st = dalloc(r, &r->wpartial, wpart)) ||
-            (st = dalloc(r, &r->in_partial, (size_t)conv_in_wgrad_blocks(max_batch, rows, cols) * 448)) ||
+            (st = dalloc(r, &r->in_partial, (size_t)conv_in_wgrad_blocks(r->num_sms, max_batch, rows, cols) * 448)) ||
             (st = dalloc(r, &r->loss_partial, (size_t)loss_blocks(max_batch, rows, cols) * 19)) ||
             (st = dalloc(r, &r->loss2, 2)) || (st = dalloc(r, &r->err, 1)))
             break;

@@ -91,7 +91,7 @@ int launch_conv_in(const uint16_t *raw, float *depth_m, const float *w1, const f
 // Gradient of the first convolution: partial sums per block, then reduced.
 int launch_conv_in_wgrad(const float *depth_m, const bf16 *dz1, int n, int h, int w, float *partial, int blocks,
                          float *dw1, float *db1, cudaStream_t s);
-int conv_in_wgrad_blocks(int n, int h, int w);
+int conv_in_wgrad_blocks(int num_sms, int n, int h, int w);
 
 // Masked L1 loss against target depth (mm) on pixels valid in both, divided
 // by n*h*w; with dr its gradient with respect to the head output,
