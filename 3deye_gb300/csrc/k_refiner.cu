@@ -74,32 +74,6 @@ __device__ __forceinline__ uint4 pack8(const float *f) {
     return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
 }
 
-// Chunk c (channels 8c..8c+7) of the concatenated convolution input at
-// (img, y, x); zero outside the image.  ca and cb are multiples of 8.
-template <int MODE, typename Args>
-__device__ __forceinline__ uint4 load_input_chunk(const Args &A, int img, int y, int x, int c) {
-    if (y < 0 || y >= A.h || x < 0 || x >= A.w) return make_uint4(0u, 0u, 0u, 0u);
-    const int cca = A.ca >> 3;
-    if (c < cca) {
-        if (MODE == SRC_DIRECT) return ldg16(A.a + (((size_t)img * A.h + y) * A.w + x) * A.ca + 8 * c);
-        if (MODE == SRC_UP) {
-            const int hh = A.h >> 1, ww = A.w >> 1;
-            return ldg16(A.a + (((size_t)img * hh + (y >> 1)) * ww + (x >> 1)) * A.ca + 8 * c);
-        }
-        const int W2 = A.w * 2;
-        const bf16 *p = A.a + (((size_t)img * (A.h * 2) + 2 * y) * W2 + 2 * x) * A.ca + 8 * c;
-        const size_t row = (size_t)W2 * A.ca;
-        return bmax4(bmax4(ldg16(p), ldg16(p + A.ca)), bmax4(ldg16(p + row), ldg16(p + row + A.ca)));
-    }
-    return ldg16(A.b + (((size_t)img * A.h + y) * A.w + x) * A.cb + 8 * (c - cca));
-}
-template <typename Args>
-__device__ __forceinline__ uint4 load_input_chunk(const Args &A, int img, int y, int x, int c) {
-    if (A.mode_a == SRC_POOL) return load_input_chunk<SRC_POOL>(A, img, y, x, c);
-    if (A.mode_a == SRC_UP) return load_input_chunk<SRC_UP>(A, img, y, x, c);
-    return load_input_chunk<SRC_DIRECT>(A, img, y, x, c);
-}
-
 // ---------------------------------------------------------------------------
 // Forward / input-gradient convolution: a warp-specialised pipeline.
 //

@@ -313,9 +313,6 @@ template <> __device__ __forceinline__ void decode4<TDE_TSDF_F32>(const Raw4<TDE
     c.f[0] = r.f.x; c.f[1] = r.f.y; c.f[2] = r.f.z; c.f[3] = r.f.w;
     c.w[0] = r.w.x; c.w[1] = r.w.y; c.w[2] = r.w.z; c.w[3] = r.w.w;
 }
-template <int FMT> __device__ __forceinline__ void load4(const void *vol, uint32_t a, size_t n, Rec4 &c) {
-    decode4<FMT>(load_raw4<FMT>(vol, a, n), c);
-}
 
 // 4-bit mask of the group's voxels with w != 0 and f != 1, read from the
 // record bits: I16 f == 1 only for v == 32767 (v / 32767 is correctly

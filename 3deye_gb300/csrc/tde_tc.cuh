@@ -69,7 +69,8 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
         ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead));
 }
-// commit() by the lane with `lead` set; mbar: shared-memory address.
+// The mbarrier (shared-memory address) completes one phase when every MMA that the
+// lane with `lead` set issued so far has finished, and its shared-memory reads with it.
 __device__ __forceinline__ void commit_lead(uint32_t mbar, uint32_t lead) {
     asm volatile(
         "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
@@ -87,13 +88,6 @@ __device__ __forceinline__ bool elect_one() {
         "selp.b32 %0, 1, 0, p;\n\t}"
         : "=r"(e));
     return e != 0;
-}
-
-// The mbarrier completes one phase when every MMA this thread issued so far
-// has finished (and its shared-memory reads with it).
-__device__ __forceinline__ void commit(uint64_t *mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
-                 : "memory");
 }
 
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
